@@ -141,6 +141,13 @@ static int full_counts(Context *c, int64_t n, const float *basis, int isPBC, int
     Basis Bs = make_basis(B);
     const double pairs = 0.5 * (double)n * (double)(n - 1);
     FullTune tn = current_tune();
+    // a tile configuration set by the caller keeps the tiled kernel
+    if (tn == FullTune() && pairs >= kMinPairsCells && cell_hist_applies(n, bm, Bs, minD, maxD, bin, ne, hs)) {
+        TRY(c->buf[BUF_CELLS].ensure(cell_hist_scratch((int)n)));
+        return launch_cell_hist(c->sms, c->max_smem_optin, c->buf[BUF_COORDS].as<float>(), nullptr,
+                                c->buf[BUF_EL].as<int>(), c->buf[BUF_MOL].as<int>(), (int)n, bm, Bs, minD, maxD, bin,
+                                ne, hs, counts, counts + total, c->buf[BUF_CELLS].p, c->stream);
+    }
     if (pairs < tn.min_pairs_tiled) {
         return launch_rows_hist(c->buf[BUF_COORDS].as<float>(), c->buf[BUF_EL].as<int>(), c->buf[BUF_MOL].as<int>(),
                                 (int)n, nullptr, (int)n, 0, bm, Bs, minD, maxD, bin, ne, hs, counts, counts + total,

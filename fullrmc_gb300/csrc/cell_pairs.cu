@@ -1,0 +1,906 @@
+// All-pairs histograms over spatially sorted atoms (full_pairs_histograms_coords,
+// Extensions/pairs_histograms.pyx:289-335).
+//
+// k_full_tiles (hist_kernels.cu) evaluates every pair i < j, although at
+// r <= 20 A in a 103 A box only 3.5 % of them are in range.  Here the atoms
+// are sorted along a serpentine of columns first, so that 32 consecutive
+// atoms (a block) fill about a cube, and only pairs of blocks that can hold a
+// pair in range are evaluated:
+//
+//   k_cell_bounds   range of the atoms' real-space positions;
+//   k_cell_count    cell of every atom and its rank there;
+//   k_cell_scan     exclusive scan of the cell counts (one CTA);
+//   k_cell_scatter  atoms to their sorted places;
+//   k_cell_blocks   bounding boxes of each block, in box coordinates and in
+//                   real space (one warp per block);
+//   k_cell_hist     block pairs: a warp holds one atom of the row block per
+//                   lane, tests 32 column blocks at once (one per lane) and
+//                   evaluates the surviving ones.
+//
+// What makes it exact: the float32 difference a - b and the reference's
+// round() are monotone, so if round() of the smallest and of the largest
+// difference two blocks can have agree on every axis, it is that constant k
+// for every pair of the two blocks, and box = (a - b) - k needs no rounding
+// of its own (most blocks: k = 0 and no subtraction).  Then every real-space
+// vector of the two blocks lies within their bounding boxes' difference minus
+// k B, whose distance from the origin bounds the pairs' distances from below.
+// Where k is not constant, |real| >= |g| w with g the wrapped difference of
+// one axis and w the box's perpendicular width bounds them, and the pairs
+// that are left take the whole minimum image (pair_s).  A block pair is
+// skipped only beyond maxD plus a margin far above the float32 rounding of
+// positions and distances.  Distances are symmetric bit for bit, so a pair is
+// evaluated once, in either order, and counted at [el(i)][el(j)] for the
+// original indexes i < j.
+//
+// Bound: SM issue and the FMA pipe.  Two columns at a time go through
+// add/fma.rn.f32x2 (one issue slot for two IEEE float32 operations, at the
+// FMA pipe's scalar rate), the bin comes from an approximate quotient that is
+// checked against the distance to the next integer, and one lane in three of
+// an evaluated pair counts; per-lane queues of the counted pairs, as in
+// k_full_tiles, measured slower here (1.10 against 0.90 ms per call: the lanes
+// of a block have unequal numbers of neighbours).  Measured (whole host calls):
+// 100,000 atoms, 103 A box with gamma = 120, r 0-20 A: 6.92 -> 0.78 ms, the
+// kernel 6.81 -> 0.62 ms for 5.1e5 of 4.9e6 block pairs, 34 issue slots per
+// column of 32 rows; 11,303 atoms, r 0-12 A: 335 -> 158 us; a 100,000-atom
+// particle with every pair counted (shape function): 12.5 -> 5.2 ms.
+#include <algorithm>
+#include <cmath>
+#include <cstdint>
+
+#include "frmc_math.cuh"
+#include "frmc_ptx.cuh"
+#include "frmc_runtime.h"
+
+namespace frmc {
+
+constexpr int kCellBlock = 32;        // atoms of a block: one per lane
+constexpr int kCellCap = 1 << 16;     // cells at most (one CTA scans them)
+constexpr int kCellSub = 8;           // cells per block along a column
+constexpr int kCellThreads = 768;
+constexpr int kCellItems = 24;        // work items per warp
+
+// Range of the positions as ordered unsigned bits, the largest coordinate
+// magnitude and the work counter; zeroed (lo: inverted) by k_cell_bounds' memset.
+struct CellScalars {
+    unsigned nlo[3];   // ~ordered(lo): an atomicMax from zero
+    unsigned hi[3];
+    unsigned amax;     // bits of max |coordinate|
+    unsigned next;     // items claimed after each warp's first
+    int ncells;        // cells of the sort
+    unsigned bad;      // an element index is outside the histogram
+};
+
+struct CellSort {
+    const float *coords;     // (n, 3), or null: atoms4
+    const float4 *atoms4;    // (x, y, z, el bits)
+    const int *el, *mol;
+    int n, nb, ne, hs, pbc;
+    Basis B;
+    double volume;           // of the box (0: of the range of positions)
+    CellScalars *sc;
+    int *cells;              // counts, then starts
+    int2 *place;             // per atom: cell, rank
+    float *x, *y, *z;        // sorted, negated; NaN past the last atom
+    int4 *meta;              // el ne hs, el hs, molecule, original index
+    float4 *bounds;          // per block: 3 float4 (box lo, box hi, real lo, real hi)
+};
+
+struct CellHist {
+    int nb, nseg, segw;
+    const float *x, *y, *z;
+    const int4 *meta;
+    const float4 *bounds;
+    CellScalars *sc;
+    Basis B;
+    float w[3];              // perpendicular widths of the box
+    float reach0, reach1;    // reach = reach0 + reach1 * max |coordinate|
+    float s_lo, s_hi, minD, binw;
+    float inv, off, slack;   // 1 / bin, 1 - min / bin, see CellBins
+    unsigned total;
+    unsigned *intra, *inter;
+    int smem_hist;
+    float negzero;           // -0 (mul2)
+};
+
+__device__ __forceinline__ unsigned ordered_bits(float f)
+{
+    const unsigned u = __float_as_uint(f);
+    return u & 0x80000000u ? ~u : u | 0x80000000u;
+}
+
+__device__ __forceinline__ float from_ordered(unsigned u)
+{
+    return __uint_as_float(u & 0x80000000u ? u & 0x7fffffffu : ~u);
+}
+
+__device__ __forceinline__ float3 cell_atom(const CellSort &p, int i)
+{
+    if (p.atoms4) {
+        const float4 a = p.atoms4[i];
+        return make_float3(a.x, a.y, a.z);
+    }
+    return make_float3(p.coords[3ll * i], p.coords[3ll * i + 1], p.coords[3ll * i + 2]);
+}
+
+// Position in real space (sorting and bounds only; the margin covers its rounding).
+__device__ __forceinline__ float3 cell_real(const CellSort &p, float3 c)
+{
+    if (!p.pbc)
+        return c;
+    return make_float3(c.x * p.B.b[0] + c.y * p.B.b[3] + c.z * p.B.b[6],
+                       c.x * p.B.b[1] + c.y * p.B.b[4] + c.z * p.B.b[7],
+                       c.x * p.B.b[2] + c.y * p.B.b[5] + c.z * p.B.b[8]);
+}
+
+__global__ void __launch_bounds__(256) k_cell_bounds(CellSort p)
+{
+    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY}, am = 0.f;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < p.n; i += gridDim.x * blockDim.x) {
+        const float3 c = cell_atom(p, i);
+        const float3 r = cell_real(p, c);
+        am = fmaxf(am, fmaxf(fabsf(c.x), fmaxf(fabsf(c.y), fabsf(c.z))));
+        lo[0] = fminf(lo[0], r.x); lo[1] = fminf(lo[1], r.y); lo[2] = fminf(lo[2], r.z);
+        hi[0] = fmaxf(hi[0], r.x); hi[1] = fmaxf(hi[1], r.y); hi[2] = fmaxf(hi[2], r.z);
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const unsigned a = __reduce_max_sync(0xffffffffu, ~ordered_bits(lo[k]));
+        const unsigned b = __reduce_max_sync(0xffffffffu, ordered_bits(hi[k]));
+        if ((threadIdx.x & 31u) == 0) {
+            atomicMax(&p.sc->nlo[k], a);
+            atomicMax(&p.sc->hi[k], b);
+        }
+    }
+    const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(am));
+    if ((threadIdx.x & 31u) == 0)
+        atomicMax(&p.sc->amax, m);
+}
+
+struct CellGeom {
+    float lo[3], inv[3];
+    int n[3];
+};
+
+// Columns (x, y) about as wide as the cube that holds one block at the mean
+// density, cut into cells of an eighth of it along z.
+__device__ CellGeom cell_geom(const CellSort &p)
+{
+    CellGeom g;
+    float ext[3];
+    for (int k = 0; k < 3; ++k) {
+        g.lo[k] = from_ordered(~p.sc->nlo[k]);
+        ext[k] = from_ordered(p.sc->hi[k]) - g.lo[k];
+        if (!(ext[k] > 0.f && ext[k] < INFINITY))
+            ext[k] = 0.f;
+    }
+    const float vol = p.volume > 0.0 ? (float)p.volume : ext[0] * ext[1] * ext[2];
+    const float a = cbrtf(vol * (float)kCellBlock / (float)p.n);
+    for (int k = 0; k < 3; ++k) {
+        const float m = a > 0.f ? ext[k] / a * (k == 2 ? (float)kCellSub : 1.f) : 1.f;
+        g.n[k] = m < 1.f ? 1 : (m > 4096.f ? 4096 : (int)(m + 0.5f));
+    }
+    while ((long long)g.n[0] * g.n[1] > kCellCap) {
+        g.n[0] = (g.n[0] + 1) / 2;
+        g.n[1] = (g.n[1] + 1) / 2;
+    }
+    g.n[2] = min(g.n[2], max(1, kCellCap / (g.n[0] * g.n[1])));
+    for (int k = 0; k < 3; ++k) g.inv[k] = ext[k] > 0.f ? (float)g.n[k] / ext[k] : 0.f;
+    return g;
+}
+
+__device__ __forceinline__ int cell_axis(const CellGeom &g, int k, float v)
+{
+    const float t = (v - g.lo[k]) * g.inv[k];
+    return t > 0.f ? (t < (float)g.n[k] ? (int)t : g.n[k] - 1) : 0;  // NaN: 0
+}
+
+__global__ void __launch_bounds__(256) k_cell_count(CellSort p)
+{
+    __shared__ CellGeom g;
+    if (threadIdx.x == 0) {
+        g = cell_geom(p);
+        if (blockIdx.x == 0)
+            p.sc->ncells = g.n[0] * g.n[1] * g.n[2];
+    }
+    __syncthreads();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= p.n)
+        return;
+    const float3 r = cell_real(p, cell_atom(p, i));
+    const int ix = cell_axis(g, 0, r.x), iy = cell_axis(g, 1, r.y), iz = cell_axis(g, 2, r.z);
+    // serpentine: neighbouring columns join at the same end
+    const int col = ix * g.n[1] + (ix & 1 ? g.n[1] - 1 - iy : iy);
+    const int cell = col * g.n[2] + (col & 1 ? g.n[2] - 1 - iz : iz);
+    p.place[i] = make_int2(cell, atomicAdd(p.cells + cell, 1));
+}
+
+// Exclusive scan of the cell counts in place, 4,096 cells a turn.
+__global__ void __launch_bounds__(1024) k_cell_scan(int *cells, const CellScalars *sc)
+{
+    __shared__ int warp[2][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int turns = (sc->ncells + 4095) / 4096;
+    int carry = 0;
+    int4 *v = reinterpret_cast<int4 *>(cells) + threadIdx.x;
+    int4 c = *v;
+    for (int t = 0; t < turns; ++t, v += 1024) {
+        const int4 nxt = t + 1 < turns ? v[1024] : make_int4(0, 0, 0, 0);
+        const int mine = c.x + c.y + c.z + c.w;
+        int incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, incl, o);
+            incl += lane >= o ? u : 0;
+        }
+        if (lane == 31)
+            warp[t & 1][w] = incl;
+        __syncthreads();
+        // every warp scans the 32 warp totals itself
+        int all = warp[t & 1][lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, all, o);
+            all += lane >= o ? u : 0;
+        }
+        const int before = w ? __shfl_sync(0xffffffffu, all, w - 1) : 0;
+        const int at = carry + before + incl - mine;
+        *v = make_int4(at, at + c.x, at + c.x + c.y, at + c.x + c.y + c.z);
+        carry += __shfl_sync(0xffffffffu, all, 31);
+        c = nxt;
+    }
+}
+
+// el * f, or a value beyond every histogram (the caller's element indexes are
+// not checked).
+__device__ __forceinline__ int cell_offset(int el, long long f)
+{
+    const long long v = el * f;
+    return v > (1ll << 30) || v < -(1ll << 30) ? 1 << 30 : (int)v;
+}
+
+__global__ void __launch_bounds__(256) k_cell_scatter(CellSort p)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= p.nb * kCellBlock)
+        return;
+    if (i >= p.n) {
+        p.x[i] = p.y[i] = p.z[i] = __int_as_float(0x7fc00000);  // no pair in range
+        p.meta[i] = make_int4(0, 0, 0, 0);
+        return;
+    }
+    const int2 pl = p.place[i];
+    const int at = p.cells[pl.x] + pl.y;
+    const float3 c = cell_atom(p, i);
+    const int el = p.atoms4 ? __float_as_int(p.atoms4[i].w) : p.el[i];
+    p.x[at] = -c.x;
+    p.y[at] = -c.y;
+    p.z[at] = -c.z;
+    if ((unsigned)el >= (unsigned)p.ne)
+        p.sc->bad = 1u;
+    p.meta[at] = make_int4(cell_offset(el, (long long)p.ne * p.hs), cell_offset(el, p.hs), p.mol[i], i);
+}
+
+__device__ __forceinline__ float warp_min(float v)
+{
+#pragma unroll
+    for (int o = 16; o; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+
+__global__ void __launch_bounds__(256) k_cell_blocks(CellSort p)
+{
+    const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (b >= p.nb)
+        return;
+    const int lane = threadIdx.x & 31, i = b * kCellBlock + lane;
+    const float3 c = make_float3(-p.x[i], -p.y[i], -p.z[i]);
+    const float3 r = cell_real(p, c);
+    // NaN atoms are in no pair; fminf and fmaxf pass over them
+    const float v[6] = {c.x, c.y, c.z, r.x, r.y, r.z};
+    float lo[6], hi[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        lo[k] = warp_min(v[k]);
+        hi[k] = -warp_min(-v[k]);
+    }
+    if (lane == 0) {
+        p.bounds[3 * b] = make_float4(lo[0], lo[1], lo[2], hi[0]);
+        p.bounds[3 * b + 1] = make_float4(hi[1], hi[2], lo[3], lo[4]);
+        p.bounds[3 * b + 2] = make_float4(lo[5], hi[3], hi[4], hi[5]);
+    }
+}
+
+// ------------------------------------------------------------ block pairs
+typedef unsigned long long f2;  // two float32 in one 64-bit register
+
+__device__ __forceinline__ f2 dup2(float v)
+{
+    const unsigned u = __float_as_uint(v);
+    return (f2)u << 32 | u;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b)
+{
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// a b, rounded once.  ptxas contracts mul.rn.f32x2 and add.rn.f32x2 into one
+// fma.rn.f32x2 (unlike the scalar forms, whose .rn keeps them apart), which
+// would change the last bit of a distance.  So a product is an fma that adds
+// nz = -0, which is exact for every product (x + -0 = x, also for x = +-0),
+// and nz comes from the kernel's parameters, so it is no constant to fold.
+__device__ __forceinline__ f2 mul2(f2 a, f2 b, f2 nz)
+{
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(nz));
+    return r;
+}
+
+// The basis terms that pair_s<BM> keeps, duplicated for f32x2, and -0.
+template <int BM>
+struct Basis2 {
+    f2 b[BM == BM_IBC ? 1 : 9], nz;
+    __device__ Basis2(const Basis &B, float negzero)
+    {
+        if (BM != BM_IBC)
+#pragma unroll
+            for (int k = 0; k < 9; ++k) b[k] = dup2(B.b[k]);
+        nz = dup2(negzero);
+    }
+};
+
+// Squared distances of two pairs from their wrapped box differences, in the
+// operation order of pair_s<BM>.
+template <int BM>
+__device__ __forceinline__ f2 square2(f2 dx, f2 dy, f2 dz, const Basis2<BM> &B)
+{
+    f2 x = dx, y = dy, z = dz;
+    if (BM == BM_DIAG) {
+        x = mul2(dx, B.b[0], B.nz);
+        y = mul2(dy, B.b[4], B.nz);
+        z = mul2(dz, B.b[8], B.nz);
+    } else if (BM == BM_XYTRI) {
+        x = add2(mul2(dx, B.b[0], B.nz), mul2(dy, B.b[3], B.nz));
+        y = mul2(dy, B.b[4], B.nz);
+        z = mul2(dz, B.b[8], B.nz);
+    } else if (BM == BM_LOWER) {
+        x = add2(add2(mul2(dx, B.b[0], B.nz), mul2(dy, B.b[3], B.nz)), mul2(dz, B.b[6], B.nz));
+        y = add2(mul2(dy, B.b[4], B.nz), mul2(dz, B.b[7], B.nz));
+        z = mul2(dz, B.b[8], B.nz);
+    } else if (BM == BM_GENERAL) {
+        x = add2(add2(mul2(dx, B.b[0], B.nz), mul2(dy, B.b[3], B.nz)), mul2(dz, B.b[6], B.nz));
+        y = add2(add2(mul2(dx, B.b[1], B.nz), mul2(dy, B.b[4], B.nz)), mul2(dz, B.b[7], B.nz));
+        z = add2(add2(mul2(dx, B.b[2], B.nz), mul2(dy, B.b[5], B.nz)), mul2(dz, B.b[8], B.nz));
+    }
+    return add2(add2(mul2(x, x, B.nz), mul2(y, y, B.nz)), mul2(z, z, B.nz));
+}
+
+// round() of one difference as pair_s takes it.
+__device__ __forceinline__ float round_ref(float d)
+{
+    return truncf(__fadd_rn(d, copysignf(0.5f, d)));
+}
+
+__device__ __forceinline__ float rsqrt_approx(float s)
+{
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(s));
+    return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c)
+{
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f2 pack2(float a, float b)
+{
+    return (f2)__float_as_uint(b) << 32 | __float_as_uint(a);
+}
+__device__ __forceinline__ float lo2(f2 a) { return __uint_as_float((unsigned)a); }
+__device__ __forceinline__ float hi2(f2 a) { return __uint_as_float((unsigned)(a >> 32)); }
+
+// One warp's column block in shared memory: x, y, z negated, and the atoms'
+// histogram offsets, molecule and original index.
+struct __align__(16) CellStage {
+    float x[kCellBlock], y[kCellBlock], z[kCellBlock];
+    int4 meta[kCellBlock];
+};
+
+// A row atom: sorted index, position, histogram offsets, molecule and original index.
+struct CellRow {
+    int index;
+    float x, y, z;
+    int4 meta;
+};
+
+constexpr float kMagic = 8388608.0f;           // 2^23: t + 2^23 rounded down is 2^23 + floor(t), 0 <= t < 2^22
+constexpr unsigned kMagicBits = 0x4b000000u;
+
+__device__ __forceinline__ f2 add2_down(f2 a, f2 b)
+{
+    f2 r;
+    asm("add.rz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// What every pair needs, in registers: limits, the bin quotient's constants
+// and 2^23 for the packed minimum image.
+struct CellBins {
+    f2 inv, off, magic;
+    float s_lo, s_hi;
+    float slack;             // the fast bin holds where |fraction - 0.5| < slack
+    unsigned limit;          // bytes of a histogram in global memory, 0: in shared memory
+    unsigned spare;          // shared-memory address of the lane's spare counter
+    __device__ CellBins(const CellHist &p, unsigned shaddr) : inv(dup2(p.inv)), off(dup2(p.off)), magic(dup2(kMagic))
+    {
+        s_lo = p.s_lo;
+        s_hi = p.s_hi;
+        slack = p.sc->bad ? -1.0f : p.slack;
+        limit = p.smem_hist ? 0u : 4u * p.total;
+        spare = shaddr + 4u * (p.total + 1u + (threadIdx.x & 31u));
+    }
+};
+
+// The pairs that the fast path leaves: the IEEE root and quotient, counts of
+// atoms of one molecule and checked offsets.  j: the column's sorted index.
+__device__ __noinline__ void bin_exact(const CellHist &p, float s, int i, int j, unsigned *shist)
+{
+    const int4 row = p.meta[i], col = p.meta[j];
+    const unsigned flat =
+        (unsigned)(row.w < col.w ? row.x + col.y : col.x + row.y) + (unsigned)pair_bin(s, p.minD, p.binw);
+    if (flat < p.total) {
+        if (row.z == col.z)
+            atomicAdd(p.intra + flat, 1u);
+        else if (shist)
+            atomicAdd(shist + flat, 1u);
+        else
+            atomicAdd(p.inter + flat, 1u);
+    }
+}
+
+// Counts four columns' pairs (squared distances s, two and two) with one row
+// atom per lane.  A quotient from rsqrt.approx (2^-22.9) differs from the
+// reference's by less than a known bound, so where it is further than that
+// from an integer its floor is the bin; the others (0.2 % of the pairs at
+// 2,000 bins) and pairs of one molecule go through bin_exact.  Offsets in
+// `row` and `meta` are in bytes and count from `shaddr` and 2^23's bits.
+template <bool LO>
+__device__ __forceinline__ void bin_quad(const CellHist &p, const CellBins &k, f2 s01, f2 s23, const CellRow &row,
+                                         const int4 *meta, int j0, unsigned *shist, f2 nz)
+{
+    const float s[4] = {lo2(s01), hi2(s01), lo2(s23), hi2(s23)};
+    bool in[4];
+#pragma unroll
+    for (int h = 0; h < 4; ++h) in[h] = (!LO || s[h] >= k.s_lo) && s[h] < k.s_hi;  // s >= 0 or NaN
+    if (!__any_sync(0xffffffffu, in[0] || in[1] || in[2] || in[3]))
+        return;
+    bool fast[4], rare = false;
+    unsigned at[4];
+#pragma unroll
+    for (int h = 0; h < 4; h += 2) {
+        const f2 d = mul2(h ? s23 : s01, pack2(rsqrt_approx(s[h]), rsqrt_approx(s[h + 1])), nz);
+        const f2 t = fma2(d, k.inv, k.off);            // quotient + 1
+        const f2 r = add2_down(t, k.magic);            // 2^23 + floor
+        // fraction - 0.5: t - (floor + 0.5), every step exact
+        const f2 u = fma2(add2(r, dup2(0.5f - kMagic)), dup2(-1.0f), t);
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+            const int4 col = meta[h + g];
+            at[h + g] = (row.meta.w < col.w ? row.meta.x + col.y : col.x + row.meta.y) +
+                        4u * __float_as_uint(g ? hi2(r) : lo2(r));
+            fast[h + g] = in[h + g] && fabsf(g ? hi2(u) : lo2(u)) < k.slack && row.meta.z != col.z;
+            rare |= in[h + g] && !fast[h + g];
+        }
+    }
+    if (k.limit == 0u) {
+        // the other lanes add to a spare counter: a predicated shared-memory
+        // atomic compiles to a branch around it (three more issue slots)
+#pragma unroll
+        for (int h = 0; h < 4; ++h)
+            asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(fast[h] ? at[h] : k.spare) : "memory");
+    } else {
+#pragma unroll
+        for (int h = 0; h < 4; ++h)
+            if (fast[h] && at[h] < k.limit)
+                atomicAdd(p.inter + at[h] / 4u, 1u);
+    }
+    if (__any_sync(0xffffffffu, rare)) {
+        unsigned left = 0u;
+#pragma unroll
+        for (int h = 0; h < 4; ++h) left |= in[h] && !fast[h] ? 1u << h : 0u;
+        while (left) {
+            const int h = __ffs(left) - 1;
+            left &= left - 1;
+            bin_exact(p, h < 2 ? (h ? s[1] : s[0]) : (h == 2 ? s[2] : s[3]), row.index, j0 + h, shist);
+        }
+    }
+}
+
+// The minimum image of two differences: x - trunc(x + copysign(0.5, x)) with
+// the sign set aside and the truncation by adding 2^23 rounded down, exact
+// for |x| < 2^22 (FRND runs on the quarter-rate pipe).
+__device__ __forceinline__ f2 wrap2(f2 x, f2 magic)
+{
+    const f2 sign = 0x8000000080000000ull;
+    const f2 a = x & ~sign;
+    const f2 n = add2(add2_down(add2(a, dup2(0.5f)), magic), dup2(-kMagic));
+    return fma2(n, dup2(-1.0f), a) ^ (x & sign);
+}
+
+// What two blocks need for the pairs' minimum image.
+enum CellWrap : int {
+    CW_NONE = 0,   // every image shift is 0
+    CW_SHIFT = 1,  // one constant shift
+    CW_WRAP = 2,   // the whole minimum image
+    CW_FAR = 3,    // the same for coordinates beyond wrap2's range
+};
+
+// One lane's row atom against the 32 staged columns (sorted indexes from j0).
+// CW_WRAP and CW_FAR take only the columns past `after` (a block against
+// itself: past the lane's own).
+template <int BM, bool LO, int WRAP>
+__device__ __forceinline__ void block_pairs(const CellHist &p, const CellStage &c, const CellRow &row, const float *sh,
+                                            const Basis2<BM> &B2, const CellBins &bins, int j0, int after,
+                                            unsigned *shist)
+{
+    const f2 rx2 = dup2(row.x), ry2 = dup2(row.y), rz2 = dup2(row.z);
+    const f2 kx = dup2(-sh[0]), ky = dup2(-sh[1]), kz = dup2(-sh[2]);
+#pragma unroll 1
+    for (int g = 0; g < kCellBlock; g += 4) {
+        f2 s[2];
+        if (WRAP != CW_FAR) {
+            const ulonglong2 X = *reinterpret_cast<const ulonglong2 *>(c.x + g);
+            const ulonglong2 Y = *reinterpret_cast<const ulonglong2 *>(c.y + g);
+            const ulonglong2 Z = *reinterpret_cast<const ulonglong2 *>(c.z + g);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                f2 dx = add2(rx2, h ? X.y : X.x), dy = add2(ry2, h ? Y.y : Y.x), dz = add2(rz2, h ? Z.y : Z.x);
+                if (WRAP == CW_SHIFT) {
+                    dx = add2(dx, kx);
+                    dy = add2(dy, ky);
+                    dz = add2(dz, kz);
+                } else if (WRAP == CW_WRAP && BM != BM_IBC) {
+                    dx = wrap2(dx, bins.magic);
+                    dy = wrap2(dy, bins.magic);
+                    dz = wrap2(dz, bins.magic);
+                }
+                s[h] = square2<BM>(dx, dy, dz, B2);
+            }
+        } else {
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                s[h] = pack2(pair_s<BM>(row.x, row.y, row.z, -c.x[g + 2 * h], -c.y[g + 2 * h], -c.z[g + 2 * h], p.B),
+                             pair_s<BM>(row.x, row.y, row.z, -c.x[g + 2 * h + 1], -c.y[g + 2 * h + 1],
+                                        -c.z[g + 2 * h + 1], p.B));
+        }
+        if (WRAP >= CW_WRAP)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                s[h] = pack2(g + 2 * h > after ? lo2(s[h]) : INFINITY, g + 2 * h + 1 > after ? hi2(s[h]) : INFINITY);
+        bin_quad<LO>(p, bins, s[0], s[1], row, c.meta + g, j0 + g, shist, B2.nz);
+    }
+}
+
+struct BlockBox {
+    float lo[3], hi[3], rlo[3], rhi[3];
+};
+
+__device__ __forceinline__ BlockBox block_box(const float4 *bounds, int b)
+{
+    const float4 u = bounds[3 * b], v = bounds[3 * b + 1], w = bounds[3 * b + 2];
+    BlockBox r;
+    r.lo[0] = u.x; r.lo[1] = u.y; r.lo[2] = u.z; r.hi[0] = u.w;
+    r.hi[1] = v.x; r.hi[2] = v.y; r.rlo[0] = v.z; r.rlo[1] = v.w;
+    r.rlo[2] = w.x; r.rhi[0] = w.y; r.rhi[1] = w.z; r.rhi[2] = w.w;
+    return r;
+}
+
+// The CellWrap of two blocks (`pack`: the shift of CW_SHIFT as three int8), or
+// -1 where every pair is out of range.
+template <int BM>
+__device__ __forceinline__ int block_test(const CellHist &p, const BlockBox &a, const BlockBox &b, float reach,
+                                          unsigned &pack)
+{
+    pack = 0u;
+    float k[3] = {0.f, 0.f, 0.f};
+    bool same = true, near = true;
+    if (BM != BM_IBC) {
+        bool far = false;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const float lo = __fsub_rn(a.lo[d], b.hi[d]), hi = __fsub_rn(a.hi[d], b.lo[d]);
+            const float k0 = round_ref(lo), k1 = round_ref(hi);
+            same &= k0 == k1 && fabsf(k0) < 100.f;
+            near &= lo > -4e6f && hi < 4e6f;
+            k[d] = k0;
+            // smallest |g| over the interval: 0 where it holds an integer
+            const float n = floorf(hi);
+            const float m = n >= lo ? 0.f : fminf(lo - n, n + 1.f - hi);
+            far |= m * p.w[d] > reach;
+        }
+        if (far)
+            return -1;
+        if (!same)
+            return near ? CW_WRAP : CW_FAR;
+    }
+    float gap2 = 0.f;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const float t = BM == BM_IBC ? 0.f : k[0] * p.B.b[d] + k[1] * p.B.b[3 + d] + k[2] * p.B.b[6 + d];
+        const float gap = fmaxf(0.f, fmaxf(a.rlo[d] - b.rhi[d] - t, t - (a.rhi[d] - b.rlo[d])));
+        gap2 += gap * gap;
+    }
+    if (gap2 > reach * reach)
+        return -1;
+    if (BM == BM_IBC)
+        return CW_NONE;
+    const int kx = (int)k[0], ky = (int)k[1], kz = (int)k[2];
+    pack = (unsigned)(kx & 255) | (unsigned)(ky & 255) << 8 | (unsigned)(kz & 255) << 16;
+    return pack ? CW_SHIFT : CW_NONE;
+}
+
+// Column block of offset o from row block I, or -1: each unordered pair of
+// blocks belongs to one row block, and every row block gets half of the others.
+__device__ __forceinline__ int column_block(int I, int o, int nb)
+{
+    if (2 * o > nb || (2 * o == nb && I >= o))
+        return -1;
+    const int J = I + o;
+    return J < nb ? J : J - nb;
+}
+
+template <int BM, bool LO>
+__global__ void __launch_bounds__(kCellThreads, 1) k_cell_hist(CellHist p)
+{
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    CellStage &stage = reinterpret_cast<CellStage *>(smem)[warp];
+    unsigned *shist = nullptr;
+    if (p.smem_hist) {
+        shist = reinterpret_cast<unsigned *>(smem + kCellThreads / 32 * sizeof(CellStage));
+        for (unsigned k = tid; k < p.total; k += kCellThreads) shist[k] = 0u;
+        __syncthreads();
+    }
+    // byte offsets of a row: from the counters, less 2^23 and the quotient's 1
+    const unsigned rowbase = (shist ? smem_addr(shist) : 0u) - 4u * (kMagicBits + 1u);
+    const Basis2<BM> B2(p.B, p.negzero);
+    const CellBins bins(p, shist ? smem_addr(shist) : 0u);
+    const float reach = p.reach0 + p.reach1 * __uint_as_float(p.sc->amax);
+    const unsigned nitems = (unsigned)p.nb * (unsigned)p.nseg;
+    const unsigned nwarps = gridDim.x * (kCellThreads / 32);
+
+    // the next item is claimed while this one is evaluated
+    unsigned next = blockIdx.x * (kCellThreads / 32) + warp;
+    while (next < nitems) {
+        const unsigned item = next;
+        if (lane == 0)
+            next = nwarps + atomicAdd(&p.sc->next, 1u);
+        // the nearest offsets, which hold the most pairs, first
+        const int I = (int)(item % (unsigned)p.nb), o0 = (int)(item / (unsigned)p.nb) * p.segw;
+        CellRow row;
+        {
+            const int i = row.index = I * kCellBlock + lane;
+            row.x = -p.x[i];
+            row.y = -p.y[i];
+            row.z = -p.z[i];
+            const int4 m = p.meta[i];
+            row.meta = make_int4((int)(4u * m.x + rowbase), (int)(4u * m.y + rowbase), m.z, m.w);
+        }
+        const BlockBox a = block_box(p.bounds, I);
+        for (int o = o0; o < o0 + p.segw && 2 * o <= p.nb; o += 32) {
+            const int mine = o + lane < o0 + p.segw ? column_block(I, o + lane, p.nb) : -1;
+            unsigned pack = 0u;
+            int what = -1;
+            if (mine >= 0)
+                what = block_test<BM>(p, a, block_box(p.bounds, mine), reach, pack);
+            unsigned left = __ballot_sync(0xffffffffu, what >= 0);
+            // the next block's columns are loaded while one is evaluated
+            float nx = 0.f, ny = 0.f, nz = 0.f;
+            int4 nm = make_int4(0, 0, 0, 0);
+            int J = 0;
+            auto load = [&](unsigned m) {
+                J = __shfl_sync(0xffffffffu, mine, __ffs(m) - 1);
+                const int c = J * kCellBlock + lane;
+                nx = p.x[c];
+                ny = p.y[c];
+                nz = p.z[c];
+                nm = p.meta[c];
+            };
+            if (left)
+                load(left);
+            while (left) {
+                const int src = __ffs(left) - 1;
+                const int kind = __shfl_sync(0xffffffffu, what, src);
+                const unsigned pk = __shfl_sync(0xffffffffu, pack, src);
+                const int jcur = J;
+                const bool diag = J == I;
+                __syncwarp();
+                stage.x[lane] = nx;
+                stage.y[lane] = ny;
+                stage.z[lane] = nz;
+                stage.meta[lane] = make_int4((int)(4u * nm.x), (int)(4u * nm.y), nm.z, nm.w);
+                __syncwarp();
+                left &= left - 1;
+                if (left)
+                    load(left);
+                const float sh[3] = {(float)(signed char)(pk & 255u), (float)(signed char)(pk >> 8 & 255u),
+                                     (float)(signed char)(pk >> 16 & 255u)};
+                const int j0 = (int)(jcur * kCellBlock), after = diag ? lane : -1;
+                if (kind == CW_FAR)
+                    block_pairs<BM, LO, CW_FAR>(p, stage, row, sh, B2, bins, j0, after, shist);
+                else if (diag || kind == CW_WRAP)
+                    block_pairs<BM, LO, CW_WRAP>(p, stage, row, sh, B2, bins, j0, after, shist);
+                else if (kind == CW_NONE)
+                    block_pairs<BM, LO, CW_NONE>(p, stage, row, sh, B2, bins, j0, -1, shist);
+                else
+                    block_pairs<BM, LO, CW_SHIFT>(p, stage, row, sh, B2, bins, j0, -1, shist);
+            }
+        }
+        next = __shfl_sync(0xffffffffu, next, 0);
+    }
+    __syncthreads();
+    if (shist)
+        for (unsigned k = tid; k < p.total; k += kCellThreads) {
+            const unsigned v = shist[k];
+            if (v)
+                atomicAdd(p.inter + k, v);
+        }
+}
+
+// ================================================================ launchers
+static size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
+
+// Smallest |b w|-like widths of the box: w_k = 1 / |column k of B^-1|
+// (|real| >= |g_k| w_k, g = real B^-1).  False for a singular basis.
+static bool box_widths(const float *b, float w[3], double *volume)
+{
+    double B[9];
+    for (int k = 0; k < 9; ++k) B[k] = b[k];
+    const double c[9] = {B[4] * B[8] - B[5] * B[7], B[2] * B[7] - B[1] * B[8], B[1] * B[5] - B[2] * B[4],
+                         B[5] * B[6] - B[3] * B[8], B[0] * B[8] - B[2] * B[6], B[2] * B[3] - B[0] * B[5],
+                         B[3] * B[7] - B[4] * B[6], B[1] * B[6] - B[0] * B[7], B[0] * B[4] - B[1] * B[3]};
+    const double det = B[0] * c[0] + B[1] * c[3] + B[2] * c[6];
+    *volume = std::fabs(det);
+    if (!(*volume > 0.0) || !std::isfinite(*volume))
+        return false;
+    for (int k = 0; k < 3; ++k)
+        w[k] = (float)(*volume / std::sqrt(c[k] * c[k] + c[3 + k] * c[3 + k] + c[6 + k] * c[6 + k]));
+    return true;
+}
+
+// Largest bin a pair in range can take (the reference's float32 quotient).
+static long long largest_bin(float s_hi, float minD, float binw)
+{
+    const float d = std::sqrt(std::nextafterf(s_hi, 0.0f));
+    const float t = d - minD;
+    const float v = t / binw;
+    return v >= 0.0f && v < 1e9f ? (long long)v : -1;
+}
+
+bool cell_hist_applies(long long n, int bm, const Basis &B, float minD, float maxD, float binw, int ne, int hs)
+{
+    float s_lo, s_hi, w[3];
+    double vol;
+    const long long total = (long long)ne * ne * hs;
+    if (n < 2 || n > (1ll << 24) || !(maxD > 0.0f) || !std::isfinite(maxD) || !std::isfinite(minD))
+        return false;
+    sq_limits(minD, maxD, &s_lo, &s_hi);
+    if (!(s_hi > 0.0f) || !std::isfinite(s_hi))
+        return false;
+    const long long top = largest_bin(s_hi, minD, binw);
+    return top >= 0 && top < (1ll << 22) && top <= total && (bm == BM_IBC || box_widths(B.b, w, &vol));
+}
+
+size_t cell_hist_scratch(int n)
+{
+    const size_t np = (size_t)(n + kCellBlock - 1) / kCellBlock * kCellBlock;
+    return 256 + up256(4 * (size_t)kCellCap) + up256(8 * (size_t)n) + 3 * up256(4 * np) + up256(16 * np) +
+           up256(48 * (np / kCellBlock));
+}
+
+template <int BM>
+static int launch_cell_hist_bm(const CellHist &p, int grid, size_t smem, cudaStream_t st)
+{
+    auto kern = p.s_lo > 0.0f ? k_cell_hist<BM, true> : k_cell_hist<BM, false>;
+    FRMC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<grid, kCellThreads, smem, st>>>(p);
+    FRMC_CUDA(cudaGetLastError());
+    return FRMC_OK;
+}
+
+int launch_cell_hist(int sms, int max_smem_optin, const float *coords, const float4 *atoms4, const int *el,
+                     const int *mol, int n, int bm, const Basis &B, float minD, float maxD, float binw, int ne, int hs,
+                     unsigned *intra, unsigned *inter, void *scratch, cudaStream_t st)
+{
+    CellSort c{};
+    c.coords = coords;
+    c.atoms4 = atoms4;
+    c.el = el;
+    c.mol = mol;
+    c.n = n;
+    c.nb = (n + kCellBlock - 1) / kCellBlock;
+    c.ne = ne;
+    c.hs = hs;
+    c.pbc = bm != BM_IBC;
+    c.B = B;
+    CellHist h{};
+    h.B = B;
+    h.negzero = -0.0f;
+    h.w[0] = h.w[1] = h.w[2] = 1.0f;
+    double scale = 1.0;
+    if (c.pbc) {
+        if (!box_widths(B.b, h.w, &c.volume))
+            return set_error(FRMC_E_ARG, "all-pairs histogram: singular basis");
+        scale = 0.0;
+        for (int k = 0; k < 9; ++k) scale += std::fabs((double)B.b[k]);
+    }
+    // margin: float32 positions are off by a few 1e-7 of |coordinate| |B|
+    h.reach0 = (float)((double)maxD * 1.0001 + 1e-5 * scale);
+    h.reach1 = (float)(1e-5 * scale);
+    unsigned char *at = static_cast<unsigned char *>(scratch);
+    auto take = [&](size_t bytes) {
+        unsigned char *r = at;
+        at += up256(bytes);
+        return r;
+    };
+    const size_t np = (size_t)c.nb * kCellBlock;
+    c.sc = reinterpret_cast<CellScalars *>(take(sizeof(CellScalars)));
+    c.cells = reinterpret_cast<int *>(take(4 * (size_t)kCellCap));
+    c.place = reinterpret_cast<int2 *>(take(8 * (size_t)n));
+    c.x = reinterpret_cast<float *>(take(4 * np));
+    c.y = reinterpret_cast<float *>(take(4 * np));
+    c.z = reinterpret_cast<float *>(take(4 * np));
+    c.meta = reinterpret_cast<int4 *>(take(16 * np));
+    c.bounds = reinterpret_cast<float4 *>(take(48 * (size_t)c.nb));
+    h.nb = c.nb;
+    h.x = c.x;
+    h.y = c.y;
+    h.z = c.z;
+    h.meta = c.meta;
+    h.bounds = c.bounds;
+    h.sc = c.sc;
+    sq_limits(minD, maxD, &h.s_lo, &h.s_hi);
+    h.minD = minD;
+    h.binw = binw;
+    // relative errors: rsqrt.approx 2^-22.9, its product, 1 / bin and the fma
+    // 2^-24 each, the reference's square root, difference and quotient 2^-24
+    // each: 4.9e-7 of (d + |min|) / bin in all
+    // (the quotient is taken one higher, so that it is never negative)
+    h.inv = 1.0f / binw;
+    h.off = 1.0f - minD * h.inv;
+    h.slack = 0.5f - (5e-7f * (maxD + std::fabs(minD)) * std::fabs(h.inv) + 1e-6f);
+    if (largest_bin(h.s_hi, minD, binw) > hs)
+        h.slack = -1.0f;  // offsets past the histogram are possible: bin_exact checks them
+    h.total = (unsigned)((long long)ne * ne * hs);
+    h.intra = intra;
+    h.inter = inter;
+    // the row block's offsets in segments: about kCellItems items per warp
+    const int half = c.nb / 2 + 1;
+    const long long warps = (long long)sms * (kCellThreads / 32);
+    h.segw = 1;
+    while (h.segw < 512 && (long long)c.nb * half > kCellItems * warps * 2 * h.segw) h.segw *= 2;
+    h.nseg = (half + h.segw - 1) / h.segw;
+    const size_t stage = kCellThreads / 32 * sizeof(CellStage), hist = 4 * ((size_t)h.total + 33);  // + bin hs of the last row, 32 spare counters
+    h.smem_hist = stage + hist <= (size_t)max_smem_optin;
+    const size_t smem = stage + (h.smem_hist ? hist : 0);
+    const long long items = (long long)h.nb * h.nseg;
+    const int grid = (int)std::min<long long>(sms, (items + kCellThreads / 32 - 1) / (kCellThreads / 32));
+
+    FRMC_CUDA(cudaMemsetAsync(scratch, 0, 256 + 4 * (size_t)kCellCap, st));  // scalars and cell counts
+    k_cell_bounds<<<std::min((n + 255) / 256, sms), 256, 0, st>>>(c);
+    k_cell_count<<<(n + 255) / 256, 256, 0, st>>>(c);
+    k_cell_scan<<<1, 1024, 0, st>>>(c.cells, c.sc);
+    k_cell_scatter<<<(int)((np + 255) / 256), 256, 0, st>>>(c);
+    k_cell_blocks<<<(c.nb * 32 + 255) / 256, 256, 0, st>>>(c);
+    FRMC_CUDA(cudaGetLastError());
+    switch (bm) {
+    case BM_IBC: return launch_cell_hist_bm<BM_IBC>(h, grid, smem, st);
+    case BM_DIAG: return launch_cell_hist_bm<BM_DIAG>(h, grid, smem, st);
+    case BM_XYTRI: return launch_cell_hist_bm<BM_XYTRI>(h, grid, smem, st);
+    case BM_LOWER: return launch_cell_hist_bm<BM_LOWER>(h, grid, smem, st);
+    default: return launch_cell_hist_bm<BM_GENERAL>(h, grid, smem, st);
+    }
+}
+
+}  // namespace frmc

@@ -3441,7 +3441,16 @@ static int init_engine(EngineSet *s, int id)
     FullTune tn;
     if (D.n >= 2) {
         const double pairs = 0.5 * (double)D.n * (D.n - 1);
-        if (pairs < tn.min_pairs_tiled) {
+        if (pairs >= kMinPairsCells &&
+            cell_hist_applies(D.n, D.bm, D.B, D.minD, D.maxD, D.binw, D.ne, D.hs)) {
+            // the sort's scratch is the context's: finish before it is released
+            std::lock_guard<std::mutex> lk(c->mu);
+            FRMC_TRY(c->buf[BUF_CELLS].ensure(cell_hist_scratch(D.n)));
+            FRMC_TRY(launch_cell_hist(c->sms, c->max_smem_optin, nullptr, D.box, nullptr, D.mol, D.n, D.bm, D.B,
+                                      D.minD, D.maxD, D.binw, D.ne, D.hs, cnt, cnt + D.total, c->buf[BUF_CELLS].p,
+                                      s->stream));
+            FRMC_CUDA(cudaStreamSynchronize(s->stream));
+        } else if (pairs < tn.min_pairs_tiled) {
             // the row kernel reads AoS float coordinates: unpack once
             std::lock_guard<std::mutex> lk(c->mu);
             FRMC_TRY(launch_unpack_atoms(D.box, D.n, c->buf[BUF_AUX0].as<float>(), c->buf[BUF_AUX1].as<int>(),
