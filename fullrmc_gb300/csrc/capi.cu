@@ -776,12 +776,24 @@ int frmc_multiple_atomic_distances_coords(const int32_t *indexes, int64_t K, con
 {
     TRY(atomic_checks(n, K, ne, elementIndex, n));
     TRY(check_indexes(indexes, K, n));
+    // rows 0 .. n - 1, each against the columns after it (full_atomic_distances_coords)
+    bool all_rows = K == n && !allAtoms;
+    for (int64_t k = 0; all_rows && k < K; ++k) all_rows = indexes[k] == k;
     LOCKED_CTX(c);
     TRY(upload_atoms(c, boxCoords, moleculeIndex, elementIndex, n));
     TRY(c->buf[BUF_ROWS].ensure(K * 4 + 16));
     TRY(h2d(c->buf[BUF_ROWS].p, indexes, K * 4, c->stream));
     TRY(atomic_prepare(c, ne, lowerLimit, upperLimit, nullptr, nullptr, nullptr, nullptr));
-    TRY(atomic_run(c, nullptr, (int)K, (int)n, allAtoms, flags, ne, basis, isPBC));
+    int done = 0;
+    if (all_rows && 0.5 * (double)n * (double)(n - 1) >= kMinPairsContacts) {
+        const size_t m = (size_t)ne * ne;
+        float *lim = c->buf[BUF_ATOMIC_LIMITS].as<float>(), *acc = c->buf[BUF_ATOMIC_ACC].as<float>();
+        TRY(atomic_contacts_run(c, c->buf[BUF_COORDS].as<float>(), (int)n, flags, ne, basis, isPBC,
+                                c->buf[BUF_MOL].as<int>(), c->buf[BUF_EL].as<int>(), lowerLimit, upperLimit, lim,
+                                lim + m, acc, reinterpret_cast<int *>(acc + 2 * m), &done, c->stream));
+    }
+    if (!done)
+        TRY(atomic_run(c, nullptr, (int)K, (int)n, allAtoms, flags, ne, basis, isPBC));
     return atomic_finish(c, ne, nintra, dintra, ninter, dinter);
 }
 

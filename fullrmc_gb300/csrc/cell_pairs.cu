@@ -47,28 +47,13 @@
 #include <cmath>
 #include <cstdint>
 
-#include "frmc_math.cuh"
+#include "cell_walk.cuh"
 #include "frmc_ptx.cuh"
-#include "frmc_runtime.h"
 
 namespace frmc {
 
-constexpr int kCellBlock = 32;        // atoms of a block: one per lane
 constexpr int kCellCap = 1 << 16;     // cells at most (one CTA scans them)
 constexpr int kCellSub = 8;           // cells per block along a column
-constexpr int kCellThreads = 768;
-constexpr int kCellItems = 24;        // work items per warp
-
-// Range of the positions as ordered unsigned bits, the largest coordinate
-// magnitude and the work counter; zeroed (lo: inverted) by k_cell_bounds' memset.
-struct CellScalars {
-    unsigned nlo[3];   // ~ordered(lo): an atomicMax from zero
-    unsigned hi[3];
-    unsigned amax;     // bits of max |coordinate|
-    unsigned next;     // items claimed after each warp's first
-    int ncells;        // cells of the sort
-    unsigned bad;      // an element index is outside the histogram
-};
 
 struct CellSort {
     const float *coords;     // (n, 3), or null: atoms4
@@ -86,20 +71,12 @@ struct CellSort {
 };
 
 struct CellHist {
-    int nb, nseg, segw;
-    const float *x, *y, *z;
-    const int4 *meta;
-    const float4 *bounds;
-    CellScalars *sc;
-    Basis B;
-    float w[3];              // perpendicular widths of the box
-    float reach0, reach1;    // reach = reach0 + reach1 * max |coordinate|
+    CellWalk walk;
     float s_lo, s_hi, minD, binw;
     float inv, off, slack;   // 1 / bin, 1 - min / bin, see CellBins
     unsigned total;
     unsigned *intra, *inter;
     int smem_hist;
-    float negzero;           // -0 (mul2)
 };
 
 __device__ __forceinline__ unsigned ordered_bits(float f)
@@ -139,6 +116,8 @@ __global__ void __launch_bounds__(256) k_cell_bounds(CellSort p)
         const float3 c = cell_atom(p, i);
         const float3 r = cell_real(p, c);
         am = fmaxf(am, fmaxf(fabsf(c.x), fmaxf(fabsf(c.y), fabsf(c.z))));
+        if (!(fabsf(c.x) < INFINITY && fabsf(c.y) < INFINITY && fabsf(c.z) < INFINITY))
+            p.sc->strange = 1u;
         lo[0] = fminf(lo[0], r.x); lo[1] = fminf(lo[1], r.y); lo[2] = fminf(lo[2], r.z);
         hi[0] = fmaxf(hi[0], r.x); hi[1] = fmaxf(hi[1], r.y); hi[2] = fmaxf(hi[2], r.z);
     }
@@ -214,12 +193,13 @@ __global__ void __launch_bounds__(256) k_cell_count(CellSort p)
     p.place[i] = make_int2(cell, atomicAdd(p.cells + cell, 1));
 }
 
-// Exclusive scan of the cell counts in place, 4,096 cells a turn.
-__global__ void __launch_bounds__(1024) k_cell_scan(int *cells, const CellScalars *sc)
+// Exclusive scan in place of n counts (the sort's cells where n is 0), 4,096 a
+// turn; the array is zero up to the next multiple of 4,096.
+__global__ void __launch_bounds__(1024) k_cell_scan(int *cells, const CellScalars *sc, int n)
 {
     __shared__ int warp[2][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int turns = (sc->ncells + 4095) / 4096;
+    const int turns = ((n ? n : sc->ncells) + 4095) / 4096;
     int carry = 0;
     int4 *v = reinterpret_cast<int4 *>(cells) + threadIdx.x;
     int4 c = *v;
@@ -310,122 +290,14 @@ __global__ void __launch_bounds__(256) k_cell_blocks(CellSort p)
     }
 }
 
-// ------------------------------------------------------------ block pairs
-typedef unsigned long long f2;  // two float32 in one 64-bit register
-
-__device__ __forceinline__ f2 dup2(float v)
-{
-    const unsigned u = __float_as_uint(v);
-    return (f2)u << 32 | u;
-}
-__device__ __forceinline__ f2 add2(f2 a, f2 b)
-{
-    f2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-// a b, rounded once.  ptxas contracts mul.rn.f32x2 and add.rn.f32x2 into one
-// fma.rn.f32x2 (unlike the scalar forms, whose .rn keeps them apart), which
-// would change the last bit of a distance.  So a product is an fma that adds
-// nz = -0, which is exact for every product (x + -0 = x, also for x = +-0),
-// and nz comes from the kernel's parameters, so it is no constant to fold.
-__device__ __forceinline__ f2 mul2(f2 a, f2 b, f2 nz)
-{
-    f2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(nz));
-    return r;
-}
-
-// The basis terms that pair_s<BM> keeps, duplicated for f32x2, and -0.
-template <int BM>
-struct Basis2 {
-    f2 b[BM == BM_IBC ? 1 : 9], nz;
-    __device__ Basis2(const Basis &B, float negzero)
-    {
-        if (BM != BM_IBC)
-#pragma unroll
-            for (int k = 0; k < 9; ++k) b[k] = dup2(B.b[k]);
-        nz = dup2(negzero);
-    }
-};
-
-// Squared distances of two pairs from their wrapped box differences, in the
-// operation order of pair_s<BM>.
-template <int BM>
-__device__ __forceinline__ f2 square2(f2 dx, f2 dy, f2 dz, const Basis2<BM> &B)
-{
-    f2 x = dx, y = dy, z = dz;
-    if (BM == BM_DIAG) {
-        x = mul2(dx, B.b[0], B.nz);
-        y = mul2(dy, B.b[4], B.nz);
-        z = mul2(dz, B.b[8], B.nz);
-    } else if (BM == BM_XYTRI) {
-        x = add2(mul2(dx, B.b[0], B.nz), mul2(dy, B.b[3], B.nz));
-        y = mul2(dy, B.b[4], B.nz);
-        z = mul2(dz, B.b[8], B.nz);
-    } else if (BM == BM_LOWER) {
-        x = add2(add2(mul2(dx, B.b[0], B.nz), mul2(dy, B.b[3], B.nz)), mul2(dz, B.b[6], B.nz));
-        y = add2(mul2(dy, B.b[4], B.nz), mul2(dz, B.b[7], B.nz));
-        z = mul2(dz, B.b[8], B.nz);
-    } else if (BM == BM_GENERAL) {
-        x = add2(add2(mul2(dx, B.b[0], B.nz), mul2(dy, B.b[3], B.nz)), mul2(dz, B.b[6], B.nz));
-        y = add2(add2(mul2(dx, B.b[1], B.nz), mul2(dy, B.b[4], B.nz)), mul2(dz, B.b[7], B.nz));
-        z = add2(add2(mul2(dx, B.b[2], B.nz), mul2(dy, B.b[5], B.nz)), mul2(dz, B.b[8], B.nz));
-    }
-    return add2(add2(mul2(x, x, B.nz), mul2(y, y, B.nz)), mul2(z, z, B.nz));
-}
-
-// round() of one difference as pair_s takes it.
-__device__ __forceinline__ float round_ref(float d)
-{
-    return truncf(__fadd_rn(d, copysignf(0.5f, d)));
-}
-
 __device__ __forceinline__ float rsqrt_approx(float s)
 {
     float r;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(s));
     return r;
 }
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c)
-{
-    f2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ f2 pack2(float a, float b)
-{
-    return (f2)__float_as_uint(b) << 32 | __float_as_uint(a);
-}
-__device__ __forceinline__ float lo2(f2 a) { return __uint_as_float((unsigned)a); }
-__device__ __forceinline__ float hi2(f2 a) { return __uint_as_float((unsigned)(a >> 32)); }
 
-// One warp's column block in shared memory: x, y, z negated, and the atoms'
-// histogram offsets, molecule and original index.
-struct __align__(16) CellStage {
-    float x[kCellBlock], y[kCellBlock], z[kCellBlock];
-    int4 meta[kCellBlock];
-};
-
-// A row atom: sorted index, position, histogram offsets, molecule and original index.
-struct CellRow {
-    int index;
-    float x, y, z;
-    int4 meta;
-};
-
-constexpr float kMagic = 8388608.0f;           // 2^23: t + 2^23 rounded down is 2^23 + floor(t), 0 <= t < 2^22
-constexpr unsigned kMagicBits = 0x4b000000u;
-
-__device__ __forceinline__ f2 add2_down(f2 a, f2 b)
-{
-    f2 r;
-    asm("add.rz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-
-// What every pair needs, in registers: limits, the bin quotient's constants
-// and 2^23 for the packed minimum image.
+// What every pair needs, in registers: limits and the bin quotient's constants.
 struct CellBins {
     f2 inv, off, magic;
     float s_lo, s_hi;
@@ -436,7 +308,7 @@ struct CellBins {
     {
         s_lo = p.s_lo;
         s_hi = p.s_hi;
-        slack = p.sc->bad ? -1.0f : p.slack;
+        slack = p.walk.sc->bad ? -1.0f : p.slack;
         limit = p.smem_hist ? 0u : 4u * p.total;
         spare = shaddr + 4u * (p.total + 1u + (threadIdx.x & 31u));
     }
@@ -446,7 +318,7 @@ struct CellBins {
 // atoms of one molecule and checked offsets.  j: the column's sorted index.
 __device__ __noinline__ void bin_exact(const CellHist &p, float s, int i, int j, unsigned *shist)
 {
-    const int4 row = p.meta[i], col = p.meta[j];
+    const int4 row = p.walk.meta[i], col = p.walk.meta[j];
     const unsigned flat =
         (unsigned)(row.w < col.w ? row.x + col.y : col.x + row.y) + (unsigned)pair_bin(s, p.minD, p.binw);
     if (flat < p.total) {
@@ -517,145 +389,11 @@ __device__ __forceinline__ void bin_quad(const CellHist &p, const CellBins &k, f
     }
 }
 
-// The minimum image of two differences: x - trunc(x + copysign(0.5, x)) with
-// the sign set aside and the truncation by adding 2^23 rounded down, exact
-// for |x| < 2^22 (FRND runs on the quarter-rate pipe).
-__device__ __forceinline__ f2 wrap2(f2 x, f2 magic)
-{
-    const f2 sign = 0x8000000080000000ull;
-    const f2 a = x & ~sign;
-    const f2 n = add2(add2_down(add2(a, dup2(0.5f)), magic), dup2(-kMagic));
-    return fma2(n, dup2(-1.0f), a) ^ (x & sign);
-}
-
-// What two blocks need for the pairs' minimum image.
-enum CellWrap : int {
-    CW_NONE = 0,   // every image shift is 0
-    CW_SHIFT = 1,  // one constant shift
-    CW_WRAP = 2,   // the whole minimum image
-    CW_FAR = 3,    // the same for coordinates beyond wrap2's range
-};
-
-// One lane's row atom against the 32 staged columns (sorted indexes from j0).
-// CW_WRAP and CW_FAR take only the columns past `after` (a block against
-// itself: past the lane's own).
-template <int BM, bool LO, int WRAP>
-__device__ __forceinline__ void block_pairs(const CellHist &p, const CellStage &c, const CellRow &row, const float *sh,
-                                            const Basis2<BM> &B2, const CellBins &bins, int j0, int after,
-                                            unsigned *shist)
-{
-    const f2 rx2 = dup2(row.x), ry2 = dup2(row.y), rz2 = dup2(row.z);
-    const f2 kx = dup2(-sh[0]), ky = dup2(-sh[1]), kz = dup2(-sh[2]);
-#pragma unroll 1
-    for (int g = 0; g < kCellBlock; g += 4) {
-        f2 s[2];
-        if (WRAP != CW_FAR) {
-            const ulonglong2 X = *reinterpret_cast<const ulonglong2 *>(c.x + g);
-            const ulonglong2 Y = *reinterpret_cast<const ulonglong2 *>(c.y + g);
-            const ulonglong2 Z = *reinterpret_cast<const ulonglong2 *>(c.z + g);
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                f2 dx = add2(rx2, h ? X.y : X.x), dy = add2(ry2, h ? Y.y : Y.x), dz = add2(rz2, h ? Z.y : Z.x);
-                if (WRAP == CW_SHIFT) {
-                    dx = add2(dx, kx);
-                    dy = add2(dy, ky);
-                    dz = add2(dz, kz);
-                } else if (WRAP == CW_WRAP && BM != BM_IBC) {
-                    dx = wrap2(dx, bins.magic);
-                    dy = wrap2(dy, bins.magic);
-                    dz = wrap2(dz, bins.magic);
-                }
-                s[h] = square2<BM>(dx, dy, dz, B2);
-            }
-        } else {
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-                s[h] = pack2(pair_s<BM>(row.x, row.y, row.z, -c.x[g + 2 * h], -c.y[g + 2 * h], -c.z[g + 2 * h], p.B),
-                             pair_s<BM>(row.x, row.y, row.z, -c.x[g + 2 * h + 1], -c.y[g + 2 * h + 1],
-                                        -c.z[g + 2 * h + 1], p.B));
-        }
-        if (WRAP >= CW_WRAP)
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-                s[h] = pack2(g + 2 * h > after ? lo2(s[h]) : INFINITY, g + 2 * h + 1 > after ? hi2(s[h]) : INFINITY);
-        bin_quad<LO>(p, bins, s[0], s[1], row, c.meta + g, j0 + g, shist, B2.nz);
-    }
-}
-
-struct BlockBox {
-    float lo[3], hi[3], rlo[3], rhi[3];
-};
-
-__device__ __forceinline__ BlockBox block_box(const float4 *bounds, int b)
-{
-    const float4 u = bounds[3 * b], v = bounds[3 * b + 1], w = bounds[3 * b + 2];
-    BlockBox r;
-    r.lo[0] = u.x; r.lo[1] = u.y; r.lo[2] = u.z; r.hi[0] = u.w;
-    r.hi[1] = v.x; r.hi[2] = v.y; r.rlo[0] = v.z; r.rlo[1] = v.w;
-    r.rlo[2] = w.x; r.rhi[0] = w.y; r.rhi[1] = w.z; r.rhi[2] = w.w;
-    return r;
-}
-
-// The CellWrap of two blocks (`pack`: the shift of CW_SHIFT as three int8), or
-// -1 where every pair is out of range.
-template <int BM>
-__device__ __forceinline__ int block_test(const CellHist &p, const BlockBox &a, const BlockBox &b, float reach,
-                                          unsigned &pack)
-{
-    pack = 0u;
-    float k[3] = {0.f, 0.f, 0.f};
-    bool same = true, near = true;
-    if (BM != BM_IBC) {
-        bool far = false;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const float lo = __fsub_rn(a.lo[d], b.hi[d]), hi = __fsub_rn(a.hi[d], b.lo[d]);
-            const float k0 = round_ref(lo), k1 = round_ref(hi);
-            same &= k0 == k1 && fabsf(k0) < 100.f;
-            near &= lo > -4e6f && hi < 4e6f;
-            k[d] = k0;
-            // smallest |g| over the interval: 0 where it holds an integer
-            const float n = floorf(hi);
-            const float m = n >= lo ? 0.f : fminf(lo - n, n + 1.f - hi);
-            far |= m * p.w[d] > reach;
-        }
-        if (far)
-            return -1;
-        if (!same)
-            return near ? CW_WRAP : CW_FAR;
-    }
-    float gap2 = 0.f;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const float t = BM == BM_IBC ? 0.f : k[0] * p.B.b[d] + k[1] * p.B.b[3 + d] + k[2] * p.B.b[6 + d];
-        const float gap = fmaxf(0.f, fmaxf(a.rlo[d] - b.rhi[d] - t, t - (a.rhi[d] - b.rlo[d])));
-        gap2 += gap * gap;
-    }
-    if (gap2 > reach * reach)
-        return -1;
-    if (BM == BM_IBC)
-        return CW_NONE;
-    const int kx = (int)k[0], ky = (int)k[1], kz = (int)k[2];
-    pack = (unsigned)(kx & 255) | (unsigned)(ky & 255) << 8 | (unsigned)(kz & 255) << 16;
-    return pack ? CW_SHIFT : CW_NONE;
-}
-
-// Column block of offset o from row block I, or -1: each unordered pair of
-// blocks belongs to one row block, and every row block gets half of the others.
-__device__ __forceinline__ int column_block(int I, int o, int nb)
-{
-    if (2 * o > nb || (2 * o == nb && I >= o))
-        return -1;
-    const int J = I + o;
-    return J < nb ? J : J - nb;
-}
-
 template <int BM, bool LO>
 __global__ void __launch_bounds__(kCellThreads, 1) k_cell_hist(CellHist p)
 {
     extern __shared__ __align__(128) unsigned char smem[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    CellStage &stage = reinterpret_cast<CellStage *>(smem)[warp];
+    const int tid = threadIdx.x;
     unsigned *shist = nullptr;
     if (p.smem_hist) {
         shist = reinterpret_cast<unsigned *>(smem + kCellThreads / 32 * sizeof(CellStage));
@@ -664,81 +402,17 @@ __global__ void __launch_bounds__(kCellThreads, 1) k_cell_hist(CellHist p)
     }
     // byte offsets of a row: from the counters, less 2^23 and the quotient's 1
     const unsigned rowbase = (shist ? smem_addr(shist) : 0u) - 4u * (kMagicBits + 1u);
-    const Basis2<BM> B2(p.B, p.negzero);
     const CellBins bins(p, shist ? smem_addr(shist) : 0u);
-    const float reach = p.reach0 + p.reach1 * __uint_as_float(p.sc->amax);
-    const unsigned nitems = (unsigned)p.nb * (unsigned)p.nseg;
-    const unsigned nwarps = gridDim.x * (kCellThreads / 32);
-
-    // the next item is claimed while this one is evaluated
-    unsigned next = blockIdx.x * (kCellThreads / 32) + warp;
-    while (next < nitems) {
-        const unsigned item = next;
-        if (lane == 0)
-            next = nwarps + atomicAdd(&p.sc->next, 1u);
-        // the nearest offsets, which hold the most pairs, first
-        const int I = (int)(item % (unsigned)p.nb), o0 = (int)(item / (unsigned)p.nb) * p.segw;
-        CellRow row;
-        {
-            const int i = row.index = I * kCellBlock + lane;
-            row.x = -p.x[i];
-            row.y = -p.y[i];
-            row.z = -p.z[i];
-            const int4 m = p.meta[i];
-            row.meta = make_int4((int)(4u * m.x + rowbase), (int)(4u * m.y + rowbase), m.z, m.w);
-        }
-        const BlockBox a = block_box(p.bounds, I);
-        for (int o = o0; o < o0 + p.segw && 2 * o <= p.nb; o += 32) {
-            const int mine = o + lane < o0 + p.segw ? column_block(I, o + lane, p.nb) : -1;
-            unsigned pack = 0u;
-            int what = -1;
-            if (mine >= 0)
-                what = block_test<BM>(p, a, block_box(p.bounds, mine), reach, pack);
-            unsigned left = __ballot_sync(0xffffffffu, what >= 0);
-            // the next block's columns are loaded while one is evaluated
-            float nx = 0.f, ny = 0.f, nz = 0.f;
-            int4 nm = make_int4(0, 0, 0, 0);
-            int J = 0;
-            auto load = [&](unsigned m) {
-                J = __shfl_sync(0xffffffffu, mine, __ffs(m) - 1);
-                const int c = J * kCellBlock + lane;
-                nx = p.x[c];
-                ny = p.y[c];
-                nz = p.z[c];
-                nm = p.meta[c];
-            };
-            if (left)
-                load(left);
-            while (left) {
-                const int src = __ffs(left) - 1;
-                const int kind = __shfl_sync(0xffffffffu, what, src);
-                const unsigned pk = __shfl_sync(0xffffffffu, pack, src);
-                const int jcur = J;
-                const bool diag = J == I;
-                __syncwarp();
-                stage.x[lane] = nx;
-                stage.y[lane] = ny;
-                stage.z[lane] = nz;
-                stage.meta[lane] = make_int4((int)(4u * nm.x), (int)(4u * nm.y), nm.z, nm.w);
-                __syncwarp();
-                left &= left - 1;
-                if (left)
-                    load(left);
-                const float sh[3] = {(float)(signed char)(pk & 255u), (float)(signed char)(pk >> 8 & 255u),
-                                     (float)(signed char)(pk >> 16 & 255u)};
-                const int j0 = (int)(jcur * kCellBlock), after = diag ? lane : -1;
-                if (kind == CW_FAR)
-                    block_pairs<BM, LO, CW_FAR>(p, stage, row, sh, B2, bins, j0, after, shist);
-                else if (diag || kind == CW_WRAP)
-                    block_pairs<BM, LO, CW_WRAP>(p, stage, row, sh, B2, bins, j0, after, shist);
-                else if (kind == CW_NONE)
-                    block_pairs<BM, LO, CW_NONE>(p, stage, row, sh, B2, bins, j0, -1, shist);
-                else
-                    block_pairs<BM, LO, CW_SHIFT>(p, stage, row, sh, B2, bins, j0, -1, shist);
-            }
-        }
-        next = __shfl_sync(0xffffffffu, next, 0);
-    }
+    const f2 nz = dup2(p.walk.negzero);
+    walk_blocks<BM>(
+        p.walk, reinterpret_cast<CellStage *>(smem)[tid >> 5],
+        [&](const int4 &m, bool row) {
+            const unsigned base = row ? rowbase : 0u;
+            return make_int4((int)(4u * m.x + base), (int)(4u * m.y + base), m.z, m.w);
+        },
+        [&](f2 s01, f2 s23, const CellRow &row, const int4 *meta, int j0) {
+            bin_quad<LO>(p, bins, s01, s23, row, meta, j0, shist, nz);
+        });
     __syncthreads();
     if (shist)
         for (unsigned k = tid; k < p.total; k += kCellThreads) {
@@ -778,18 +452,25 @@ static long long largest_bin(float s_hi, float minD, float binw)
     return v >= 0.0f && v < 1e9f ? (long long)v : -1;
 }
 
+bool cell_walk_applies(long long n, int bm, const Basis &B, float reach)
+{
+    float w[3];
+    double vol;
+    return n >= 2 && n <= (1ll << 24) && reach > 0.0f && std::isfinite(reach) &&
+           (bm == BM_IBC || box_widths(B.b, w, &vol));
+}
+
 bool cell_hist_applies(long long n, int bm, const Basis &B, float minD, float maxD, float binw, int ne, int hs)
 {
-    float s_lo, s_hi, w[3];
-    double vol;
+    float s_lo, s_hi;
     const long long total = (long long)ne * ne * hs;
-    if (n < 2 || n > (1ll << 24) || !(maxD > 0.0f) || !std::isfinite(maxD) || !std::isfinite(minD))
+    if (!cell_walk_applies(n, bm, B, maxD) || !std::isfinite(minD))
         return false;
     sq_limits(minD, maxD, &s_lo, &s_hi);
     if (!(s_hi > 0.0f) || !std::isfinite(s_hi))
         return false;
     const long long top = largest_bin(s_hi, minD, binw);
-    return top >= 0 && top < (1ll << 22) && top <= total && (bm == BM_IBC || box_widths(B.b, w, &vol));
+    return top >= 0 && top < (1ll << 22) && top <= total;
 }
 
 size_t cell_hist_scratch(int n)
@@ -799,19 +480,8 @@ size_t cell_hist_scratch(int n)
            up256(48 * (np / kCellBlock));
 }
 
-template <int BM>
-static int launch_cell_hist_bm(const CellHist &p, int grid, size_t smem, cudaStream_t st)
-{
-    auto kern = p.s_lo > 0.0f ? k_cell_hist<BM, true> : k_cell_hist<BM, false>;
-    FRMC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<grid, kCellThreads, smem, st>>>(p);
-    FRMC_CUDA(cudaGetLastError());
-    return FRMC_OK;
-}
-
-int launch_cell_hist(int sms, int max_smem_optin, const float *coords, const float4 *atoms4, const int *el,
-                     const int *mol, int n, int bm, const Basis &B, float minD, float maxD, float binw, int ne, int hs,
-                     unsigned *intra, unsigned *inter, void *scratch, cudaStream_t st)
+int sort_cells(int sms, const float *coords, const float4 *atoms4, const int *el, const int *mol, int n, int bm,
+               const Basis &B, float reach, int ne, int hs, void *scratch, CellWalk *walk, cudaStream_t st)
 {
     CellSort c{};
     c.coords = coords;
@@ -824,19 +494,20 @@ int launch_cell_hist(int sms, int max_smem_optin, const float *coords, const flo
     c.hs = hs;
     c.pbc = bm != BM_IBC;
     c.B = B;
-    CellHist h{};
+    CellWalk &h = *walk;
+    h = CellWalk{};
     h.B = B;
     h.negzero = -0.0f;
     h.w[0] = h.w[1] = h.w[2] = 1.0f;
     double scale = 1.0;
     if (c.pbc) {
         if (!box_widths(B.b, h.w, &c.volume))
-            return set_error(FRMC_E_ARG, "all-pairs histogram: singular basis");
+            return set_error(FRMC_E_ARG, "sorted pairs: singular basis");
         scale = 0.0;
         for (int k = 0; k < 9; ++k) scale += std::fabs((double)B.b[k]);
     }
     // margin: float32 positions are off by a few 1e-7 of |coordinate| |B|
-    h.reach0 = (float)((double)maxD * 1.0001 + 1e-5 * scale);
+    h.reach0 = (float)((double)reach * 1.0001 + 1e-5 * scale);
     h.reach1 = (float)(1e-5 * scale);
     unsigned char *at = static_cast<unsigned char *>(scratch);
     auto take = [&](size_t bytes) {
@@ -860,6 +531,56 @@ int launch_cell_hist(int sms, int max_smem_optin, const float *coords, const flo
     h.meta = c.meta;
     h.bounds = c.bounds;
     h.sc = c.sc;
+    // the row block's offsets in segments: about eight items per warp, of at
+    // most one test of 32 offsets as long as the claims stay few.  Whole calls
+    // with 2 / 4 / 8 / 14 / 24 items per warp and no such limit: 11,303 atoms
+    // 170 / 150 / 150 / 158 / 159 us, 20,000 168 / 156 / 155 / 183 / 180 us,
+    // 100,000 1,430 / 1,232 / 945 / 818 / 781 us (its 24 items are one test).
+    const int half = c.nb / 2 + 1;
+    const long long warps = (long long)sms * (kCellThreads / 32), all = (long long)c.nb * half;
+    h.segw = 1;
+    while ((h.segw < 32 && all > 16 * warps * h.segw) || all > 256 * warps * h.segw) h.segw *= 2;
+    h.nseg = (half + h.segw - 1) / h.segw;
+
+    FRMC_CUDA(cudaMemsetAsync(scratch, 0, 256 + 4 * (size_t)kCellCap, st));  // scalars and cell counts
+    k_cell_bounds<<<std::min((n + 255) / 256, sms), 256, 0, st>>>(c);
+    k_cell_count<<<(n + 255) / 256, 256, 0, st>>>(c);
+    k_cell_scan<<<1, 1024, 0, st>>>(c.cells, c.sc, 0);
+    k_cell_scatter<<<(int)((np + 255) / 256), 256, 0, st>>>(c);
+    k_cell_blocks<<<(c.nb * 32 + 255) / 256, 256, 0, st>>>(c);
+    FRMC_CUDA(cudaGetLastError());
+    return FRMC_OK;
+}
+
+int launch_cell_scan(int *counts, int n, cudaStream_t st)
+{
+    k_cell_scan<<<1, 1024, 0, st>>>(counts, nullptr, n);
+    FRMC_CUDA(cudaGetLastError());
+    return FRMC_OK;
+}
+
+int walk_grid(int sms, const CellWalk &w)
+{
+    const long long items = (long long)w.nb * w.nseg;
+    return (int)std::min<long long>(sms, (items + kCellThreads / 32 - 1) / (kCellThreads / 32));
+}
+
+template <int BM>
+static int launch_cell_hist_bm(const CellHist &p, int grid, size_t smem, cudaStream_t st)
+{
+    auto kern = p.s_lo > 0.0f ? k_cell_hist<BM, true> : k_cell_hist<BM, false>;
+    FRMC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<grid, kCellThreads, smem, st>>>(p);
+    FRMC_CUDA(cudaGetLastError());
+    return FRMC_OK;
+}
+
+int launch_cell_hist(int sms, int max_smem_optin, const float *coords, const float4 *atoms4, const int *el,
+                     const int *mol, int n, int bm, const Basis &B, float minD, float maxD, float binw, int ne, int hs,
+                     unsigned *intra, unsigned *inter, void *scratch, cudaStream_t st)
+{
+    CellHist h{};
+    FRMC_TRY(sort_cells(sms, coords, atoms4, el, mol, n, bm, B, maxD, ne, hs, scratch, &h.walk, st));
     sq_limits(minD, maxD, &h.s_lo, &h.s_hi);
     h.minD = minD;
     h.binw = binw;
@@ -875,25 +596,11 @@ int launch_cell_hist(int sms, int max_smem_optin, const float *coords, const flo
     h.total = (unsigned)((long long)ne * ne * hs);
     h.intra = intra;
     h.inter = inter;
-    // the row block's offsets in segments: about kCellItems items per warp
-    const int half = c.nb / 2 + 1;
-    const long long warps = (long long)sms * (kCellThreads / 32);
-    h.segw = 1;
-    while (h.segw < 512 && (long long)c.nb * half > kCellItems * warps * 2 * h.segw) h.segw *= 2;
-    h.nseg = (half + h.segw - 1) / h.segw;
-    const size_t stage = kCellThreads / 32 * sizeof(CellStage), hist = 4 * ((size_t)h.total + 33);  // + bin hs of the last row, 32 spare counters
+    const size_t stage = kCellThreads / 32 * sizeof(CellStage);
+    const size_t hist = 4 * ((size_t)h.total + 33);  // + bin hs of the last row, 32 spare counters
     h.smem_hist = stage + hist <= (size_t)max_smem_optin;
     const size_t smem = stage + (h.smem_hist ? hist : 0);
-    const long long items = (long long)h.nb * h.nseg;
-    const int grid = (int)std::min<long long>(sms, (items + kCellThreads / 32 - 1) / (kCellThreads / 32));
-
-    FRMC_CUDA(cudaMemsetAsync(scratch, 0, 256 + 4 * (size_t)kCellCap, st));  // scalars and cell counts
-    k_cell_bounds<<<std::min((n + 255) / 256, sms), 256, 0, st>>>(c);
-    k_cell_count<<<(n + 255) / 256, 256, 0, st>>>(c);
-    k_cell_scan<<<1, 1024, 0, st>>>(c.cells, c.sc);
-    k_cell_scatter<<<(int)((np + 255) / 256), 256, 0, st>>>(c);
-    k_cell_blocks<<<(c.nb * 32 + 255) / 256, 256, 0, st>>>(c);
-    FRMC_CUDA(cudaGetLastError());
+    const int grid = walk_grid(sms, h.walk);
     switch (bm) {
     case BM_IBC: return launch_cell_hist_bm<BM_IBC>(h, grid, smem, st);
     case BM_DIAG: return launch_cell_hist_bm<BM_DIAG>(h, grid, smem, st);
