@@ -14,10 +14,11 @@
 //   k_coord_accumulate  one warp per definition: the sum of its terms' counts
 //                       when every partial sum is an exact integer, else the
 //                       float32 additions one by one in term order.
+#include <cmath>
 #include <cstdint>
+#include <cstring>
 
-#include "frmc_math.cuh"
-#include "frmc_runtime.h"
+#include "cell_walk.cuh"
 
 namespace frmc {
 
@@ -158,6 +159,123 @@ int coordination_run(const CoordLaunch &L, cudaStream_t st)
         k_coord_accumulate<<<g, threads, 0, st>>>(L.counts, L.def_ids, L.def_off, L.def_terms, L.ndefs, L.data);
         FRMC_CUDA(cudaGetLastError());
     }
+    return FRMC_OK;
+}
+
+// ------------------------------------------------- all atoms, by the walk
+// all_atoms_coord_number_coords meets every core with every shell atom of a
+// definition: 2.2e9 distances for 52,000 atoms, of which a few per atom lie in
+// a window.  Where every window's upper end bounds the distance, every list
+// holds an atom once and every row a (list, definition) once, the counts come
+// from the walk over sorted atoms: an atom carries one bit per slot (list,
+// definition) as a row and one as a member of the slot's list, and a pair
+// adds to the slots where one atom is a row and the other a member, both ways
+// round.  The sums are whole numbers, so their order is free; k_coord_count
+// takes the rest.  Measured, 52,000 atoms, four definitions: 4.82 ms -> 68 us
+// and 27 us for the sort; the native call 6.2 -> 0.6 ms.
+struct CoordWalk {
+    CellWalk walk;
+    float s_hi;              // s < s_hi for every distance up to the largest upper end
+    const float *lower, *upper;  // per slot
+    unsigned long long *totals;  // per slot
+};
+
+template <int BM>
+__global__ void __launch_bounds__(kCellThreads, 1) k_coord_walk(CoordWalk p)
+{
+    __shared__ CellStage stage[kCellThreads / 32];
+    __shared__ unsigned count[kCoordSlots];
+    __shared__ float lower[kCoordSlots], upper[kCoordSlots];
+    if (threadIdx.x < kCoordSlots) {
+        count[threadIdx.x] = 0u;
+        lower[threadIdx.x] = p.lower[threadIdx.x];
+        upper[threadIdx.x] = p.upper[threadIdx.x];
+    }
+    __syncthreads();
+    const float s_hi = p.s_hi;
+    walk_blocks<BM>(
+        p.walk, stage[threadIdx.x >> 5], [](const int4 &m, bool) { return m; },
+        [&](f2 s01, f2 s23, const CellRow &row, const int4 *meta, int) {
+            const float s[4] = {lo2(s01), hi2(s01), lo2(s23), hi2(s23)};
+            unsigned in = 0u;
+#pragma unroll
+            for (int h = 0; h < 4; ++h) in |= s[h] < s_hi ? 1u << h : 0u;
+            while (in) {
+                const int h = __ffs(in) - 1;
+                in &= in - 1;
+                // meta: (slots as a row, the same, slots as a member, original index)
+                const int4 b = meta[h];
+                const unsigned ab = (unsigned)(row.meta.x & b.z), ba = (unsigned)(b.x & row.meta.z);
+                unsigned left = ab | ba;
+                if (!left)
+                    continue;
+                const float d = __fsqrt_rn(h < 2 ? (h ? s[1] : s[0]) : (h == 2 ? s[2] : s[3]));
+                while (left) {
+                    const int k = __ffs(left) - 1;
+                    left &= left - 1;
+                    if (lower[k] <= d && d <= upper[k])
+                        atomicAdd(count + k, (ab >> k & 1u) + (ba >> k & 1u));
+                }
+            }
+        });
+    __syncthreads();
+    if (threadIdx.x < kCoordSlots && count[threadIdx.x])
+        atomicAdd(p.totals + threadIdx.x, (unsigned long long)count[threadIdx.x]);
+}
+
+int coordination_walk(Context *c, const float *coords, const int *row_mask, const int *member_mask, int n,
+                      const float *basis, int isPBC, const float *lower, const float *upper, int nslots,
+                      long long *totals, int *done, cudaStream_t st)
+{
+    *done = 0;
+    float low[kCoordSlots], up[kCoordSlots], reach = 0.0f;
+    for (int k = 0; k < kCoordSlots; ++k) {
+        low[k] = k < nslots ? lower[k] : 0.0f;
+        up[k] = k < nslots ? upper[k] : -1.0f;
+        if (!(up[k] <= 3.0e38f) || !(low[k] == low[k]))
+            return FRMC_OK;
+        reach = up[k] > reach ? up[k] : reach;
+    }
+    static const float kId[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
+    const float *Bh = isPBC && basis ? basis : kId;
+    const int bm = basis_mode(Bh, isPBC);
+    const Basis B = make_basis(Bh);
+    reach = nextafterf(reach, 3.4e38f);  // windows include their upper end
+    if (!cell_walk_applies(n, bm, B, reach))
+        return FRMC_OK;
+    CoordWalk p{};
+    float s_lo;
+    sq_limits(0.0f, reach, &s_lo, &p.s_hi);
+    FRMC_TRY(c->buf[BUF_CELLS].ensure(cell_hist_scratch(n)));
+    FRMC_TRY(c->buf[BUF_ATOMIC_LIMITS].ensure(16 * kCoordSlots));
+    p.totals = c->buf[BUF_ATOMIC_LIMITS].as<unsigned long long>();
+    float *limits = reinterpret_cast<float *>(p.totals + kCoordSlots);
+    p.lower = limits;
+    p.upper = limits + kCoordSlots;
+    unsigned char block[16 * kCoordSlots] = {0};
+    memcpy(block + 8 * kCoordSlots, low, sizeof(low));
+    memcpy(block + 12 * kCoordSlots, up, sizeof(up));
+    FRMC_CUDA(cudaMemcpyAsync(p.totals, block, sizeof(block), cudaMemcpyHostToDevice, st));
+    FRMC_TRY(sort_cells(c->sms, coords, nullptr, row_mask, member_mask, n, bm, B, reach, 1, 1, c->buf[BUF_CELLS].p,
+                        &p.walk, st));
+    const int grid = walk_grid(c->sms, p.walk);
+    switch (bm) {
+    case BM_IBC: k_coord_walk<BM_IBC><<<grid, kCellThreads, 0, st>>>(p); break;
+    case BM_DIAG: k_coord_walk<BM_DIAG><<<grid, kCellThreads, 0, st>>>(p); break;
+    case BM_XYTRI: k_coord_walk<BM_XYTRI><<<grid, kCellThreads, 0, st>>>(p); break;
+    case BM_LOWER: k_coord_walk<BM_LOWER><<<grid, kCellThreads, 0, st>>>(p); break;
+    default: k_coord_walk<BM_GENERAL><<<grid, kCellThreads, 0, st>>>(p); break;
+    }
+    FRMC_CUDA(cudaGetLastError());
+    long long got[kCoordSlots];
+    unsigned odd = 0;
+    FRMC_CUDA(cudaMemcpyAsync(got, p.totals, sizeof(got), cudaMemcpyDeviceToHost, st));
+    FRMC_CUDA(cudaMemcpyAsync(&odd, &p.walk.sc->strange, sizeof(odd), cudaMemcpyDeviceToHost, st));
+    FRMC_CUDA(cudaStreamSynchronize(st));
+    if (odd)
+        return FRMC_OK;
+    for (int k = 0; k < nslots; ++k) totals[k] = got[k];
+    *done = 1;
     return FRMC_OK;
 }
 

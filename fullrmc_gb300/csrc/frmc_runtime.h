@@ -229,6 +229,15 @@ struct CoordLaunch {
     float *data = nullptr;          // device accumulators, updated in place
 };
 int coordination_run(const CoordLaunch &L, cudaStream_t st);
+// Window counts of all terms by the walk over sorted atoms (coord_kernels.cu):
+// per atom, one bit per slot (list, definition) as a row and one as a member of
+// the list, below bit kCoordSlots (device arrays); the windows (host) and the
+// totals per slot (host), without the pairs of an atom with itself.  *done is 0
+// where it does not apply.  Synchronises `st`.
+constexpr int kCoordSlots = 30;
+int coordination_walk(Context *c, const float *coords, const int *row_mask, const int *member_mask, int n,
+                      const float *basis, int isPBC, const float *lower, const float *upper, int nslots,
+                      long long *totals, int *done, cudaStream_t st);
 // List entries handled by one CTA of the counting kernel.
 int coordination_chunk();
 
