@@ -31,7 +31,7 @@ import operator
 import numpy as np
 
 from . import _args as A
-from ._native import I32P, I64P, call, ptr
+from ._native import I32P, I64P, call, fastcall, ptr
 from .pairs_distances import pairs_distances_to_point  # noqa: F401  (the reference module imports it too)
 
 NUMPY_FLOAT32 = np.float32
@@ -184,6 +184,21 @@ def _atoms_terms(T, indexes, rows, coresIndexes, shellsIndexes, lowerShells, upp
     against their cores (``atomic_coordination.pyx:207-240``)."""
     K = len(indexes)
     if K == 0:
+        return
+    fast = fastcall()
+    got = None
+    if fast is not None:
+        got = fast.atom_terms(np.asarray(indexes, np.int32), np.asarray(rows, np.int32), first, second)
+    if got is not None:
+        row, code, defs = got
+        used = np.flatnonzero(np.bincount(code))  # codes: 2 def, + 1 against the cores
+        lut = np.empty(int(used[-1]) + 1 if used.size else 0, np.int32)
+        for kind, lists in ((0, shellsIndexes), (1, coresIndexes)):
+            for c in used[(used & 1) == kind].tolist():
+                d = c >> 1
+                T.window(d, _item(lowerShells, "list", d), _item(upperShells, "list", d))
+                lut[c] = T.list_id((kind, d), _item(lists, "list", d), "shellIndexes")
+        T.add_many(row, lut[code], defs)
         return
     idx = np.asarray(indexes, np.int64)
     for seq in (first, second):

@@ -96,13 +96,16 @@ def build_fastcall(force=False):
     compiled with the host C compiler against this interpreter's headers and
     linked to the library beside it."""
     import sysconfig
+
+    import numpy
     src = os.path.join(CSRC, "fastcall.c")
     out = os.path.join(LIBDIR, "_fastcall" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
     if not force and not _stale(out, [src, LIB, os.path.join(INCLUDE, "frmc_gpu.h")]):
         return out
     cc = os.environ.get("CC", "gcc")
     tmp = out + ".tmp%d" % os.getpid()
-    cmd = [cc, "-shared", "-fPIC", "-O2", "-std=c11", "-I" + sysconfig.get_paths()["include"], "-I" + INCLUDE, src,
+    cmd = [cc, "-shared", "-fPIC", "-O2", "-std=c11", "-I" + sysconfig.get_paths()["include"],
+           "-I" + numpy.get_include(), "-I" + INCLUDE, src,
            "-L" + LIBDIR, "-lfrmc_gpu", "-Wl,-rpath,$ORIGIN", "-o", tmp]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
