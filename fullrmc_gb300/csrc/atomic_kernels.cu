@@ -16,6 +16,7 @@
 //                          order, at their offsets;
 //   k_atomic_sum           adds the list in order into the accumulators.
 #include <cstdint>
+#include <cstring>
 
 #include "cell_walk.cuh"
 
@@ -511,7 +512,7 @@ static int atomic_distances_device(AtomicParams p, DevBuf &counts, DevBuf &total
 //   k_contact_place  every entry to its row's part of the list;
 //   k_contact_order  every entry to its place by column within the row.
 // Measured: 19,994 atoms (43,000 contacts): two passes 1,814 us, the walk 44 us
-// and its sort, scan and ordering 37 us; the whole call 2.07 -> 0.31 ms.
+// and its sort, scan and ordering 37 us; the whole call 2.07 -> 0.23 ms.
 struct ContactParams {
     CellWalk walk;
     float s_hi;              // s < s_hi for every distance below the largest upper limit
@@ -601,8 +602,10 @@ __global__ void __launch_bounds__(kCellThreads, 1) k_contacts(ContactParams p)
         contact_flush(p, q, fill, fill);
 }
 
-__global__ void __launch_bounds__(256) k_contact_place(ContactParams p, ListGuard guard)
+__global__ void __launch_bounds__(256) k_contact_place(ContactParams p, ListGuard guard, unsigned *strange)
 {
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        *strange = *guard.strange;  // to the host with the results
     if (guard.closed())
         return;
     const long long len = *p.count;
@@ -636,7 +639,7 @@ constexpr long long kContactsPerAtom = 128;
 // that are not finite or more contacts than the walk lists.
 int atomic_contacts_run(Context *c, const float *coords, int n, int flags, int ne, const float *basis_host, int isPBC,
                         const int *mol, const int *el, const float *lower_host, const float *upper_host,
-                        const float *lower, const float *upper, float *dsum, int *nsum, int *done, cudaStream_t st)
+                        const AtomicBlock &block, unsigned char *results, int *done, cudaStream_t st)
 {
     *done = 0;
     float reach = 0.0f;
@@ -656,17 +659,13 @@ int atomic_contacts_run(Context *c, const float *coords, int n, int flags, int n
     sq_limits(0.0f, reach, &s_lo, &p.s_hi);
     p.flags = flags;
     p.ne = ne;
-    p.lower = lower;
-    p.upper = upper;
-    FRMC_TRY(c->buf[BUF_CELLS].ensure(cell_hist_scratch(n)));
-    const size_t rows = ((size_t)n + 1 + 4095) / 4096 * 4096;
-    FRMC_TRY(c->buf[BUF_ATOMIC_COUNTS].ensure(16 + 4 * rows));
-    p.count = c->buf[BUF_ATOMIC_COUNTS].as<long long>();
-    p.row = reinterpret_cast<int *>(p.count + 2);
-    FRMC_TRY(sort_cells(c->sms, coords, nullptr, el, mol, n, bm, B, reach, ne, 1, c->buf[BUF_CELLS].p, &p.walk, st));
-    const unsigned *strange = &p.walk.sc->strange;
+    p.lower = block.lower();
+    p.upper = block.upper();
+    p.count = block.length();
     p.cap = 4ll * n + 1024;
     for (int turn = 0; turn < 2; ++turn) {
+        const size_t rows = 4 * (((size_t)n + 1 + 4095) / 4096 * 4096);
+        FRMC_TRY(c->buf[BUF_CELLS].ensure(cell_hist_scratch(n, rows)));
         FRMC_TRY(c->buf[BUF_ATOMIC_TOTALS].ensure(36 * (size_t)p.cap));
         FRMC_TRY(c->buf[BUF_ATOMIC_LIST_B].ensure(4 * (size_t)p.cap + 4 * kSumPer));
         FRMC_TRY(c->buf[BUF_ATOMIC_LIST_V].ensure(4 * (size_t)p.cap + 4 * kSumPer));
@@ -675,8 +674,11 @@ int atomic_contacts_run(Context *c, const float *coords, int n, int flags, int n
         p.rank = reinterpret_cast<int *>(p.placed + p.cap);
         p.list_bucket = c->buf[BUF_ATOMIC_LIST_B].as<int>();
         p.list_value = c->buf[BUF_ATOMIC_LIST_V].as<float>();
-        FRMC_CUDA(cudaMemsetAsync(p.count, 0, 16 + 4 * rows, st));
-        FRMC_CUDA(cudaMemsetAsync(&p.walk.sc->next, 0, sizeof(unsigned), st));
+        if (turn)
+            FRMC_CUDA(cudaMemsetAsync(p.count, 0, 8, st));
+        FRMC_TRY(sort_cells(c->sms, coords, nullptr, el, mol, n, bm, B, reach, ne, 1, c->buf[BUF_CELLS].p, &p.walk, st,
+                            rows, reinterpret_cast<void **>(&p.row)));
+        const unsigned *strange = &p.walk.sc->strange;
         const int grid = walk_grid(c->sms, p.walk);
         switch (bm) {
         case BM_IBC: k_contacts<BM_IBC><<<grid, kCellThreads, 0, st>>>(p); break;
@@ -689,15 +691,17 @@ int atomic_contacts_run(Context *c, const float *coords, int n, int flags, int n
         FRMC_TRY(launch_cell_scan(p.row, n + 1, st));
         const ListGuard guard{p.count, p.cap, strange};
         const int g = (int)((p.cap + 255) / 256 < 4ll * c->sms ? (p.cap + 255) / 256 : 4ll * c->sms);
-        k_contact_place<<<g, 256, 0, st>>>(p, guard);
+        k_contact_place<<<g, 256, 0, st>>>(p, guard, block.strange());
         k_contact_order<<<g, 256, 0, st>>>(p, guard);
-        k_atomic_sum<<<2 * ne * ne, kSumThreads, 0, st>>>(p.list_bucket, p.list_value, p.count, guard, dsum, nsum);
+        k_atomic_sum<<<2 * ne * ne, kSumThreads, 0, st>>>(p.list_bucket, p.list_value, p.count, guard, block.dsum(),
+                                                          block.nsum());
         FRMC_CUDA(cudaGetLastError());
-        long long count = 0;
-        unsigned odd = 0;
-        FRMC_CUDA(cudaMemcpyAsync(&count, p.count, sizeof(count), cudaMemcpyDeviceToHost, st));
-        FRMC_CUDA(cudaMemcpyAsync(&odd, strange, sizeof(odd), cudaMemcpyDeviceToHost, st));
+        FRMC_CUDA(cudaMemcpyAsync(results, block.p, block.results(), cudaMemcpyDeviceToHost, st));
         FRMC_CUDA(cudaStreamSynchronize(st));
+        long long count;
+        unsigned odd;
+        memcpy(&count, results + 16 * block.m, sizeof(count));
+        memcpy(&odd, results + 16 * block.m + 8, sizeof(odd));
         if (odd)
             return FRMC_OK;
         if (count <= p.cap) {
@@ -708,6 +712,133 @@ int atomic_contacts_run(Context *c, const float *coords, int n, int flags, int n
             return FRMC_OK;
         p.cap = count;
     }
+    return FRMC_OK;
+}
+
+// ------------------------------------------------------------ a few rows
+// The constraint's call on a moved molecule: K rows against every column, read
+// once from the caller's arrays; the contacts (a few dozen) go to one list,
+// and one CTA per accumulator orders and adds its own.  Six launches, a wait
+// for the list's length and nine copies made a whole call of 161 us for 13 rows
+// of 19,994 atoms; with these two launches and two copies it takes 75 us.
+constexpr int kFewHits = 2048;
+
+struct FewParams {
+    AtomicParams a;
+    long long *length;
+    int4 *hits;  // (row position, column, bucket, value bits)
+};
+
+template <int BM>
+__global__ void __launch_bounds__(256) k_few_rows(FewParams p)
+{
+    __shared__ float4 row[kFewRows];
+    __shared__ int atom[kFewRows], mol[kFewRows];
+    const AtomicParams &a = p.a;
+    if ((int)threadIdx.x < a.K) {
+        const int r = a.rows[threadIdx.x];
+        row[threadIdx.x] =
+            make_float4(a.coords[3ll * r], a.coords[3ll * r + 1], a.coords[3ll * r + 2], __int_as_float(a.el[r]));
+        atom[threadIdx.x] = r;
+        mol[threadIdx.x] = a.mol[r];
+    }
+    __syncthreads();
+    const int j = blockIdx.x * 256 + threadIdx.x;
+    if (j >= a.n)
+        return;
+    const float x = a.coords[3ll * j], y = a.coords[3ll * j + 1], z = a.coords[3ll * j + 2];
+    const int elj = a.el[j], molj = a.mol[j];
+    for (int k = 0; k < a.K; ++k) {
+        if (j == atom[k] || (!a.allAtoms && j < atom[k]))
+            continue;
+        const bool same = molj == mol[k];
+        if (!(a.flags & (same ? AF_INTRA : AF_INTER)))
+            continue;
+        const int ela = __float_as_int(row[k].w);
+        float d = __fsqrt_rn(pair_s<BM>(row[k].x, row[k].y, row[k].z, x, y, z, a.B));
+        if (!contact_value(a.flags, a.lower[elj * a.ne + ela], a.upper[elj * a.ne + ela], d))
+            continue;
+        const long long at = (long long)atomicAdd(reinterpret_cast<unsigned long long *>(p.length), 1ull);
+        if (at < kFewHits)
+            p.hits[at] = make_int4(k, j, (same ? 0 : a.ne * a.ne) + ela * a.ne + elj, __float_as_int(d));
+    }
+}
+
+// One CTA per accumulator: its contacts in (row, column) order, added one
+// after the other.
+__global__ void __launch_bounds__(256) k_few_sum(FewParams p, float *dsum, int *nsum)
+{
+    __shared__ unsigned long long key[kFewHits];
+    __shared__ float value[kFewHits], sorted[kFewHits];
+    __shared__ int count;
+    const long long len = *p.length;
+    if (len > kFewHits)
+        return;
+    if (threadIdx.x == 0)
+        count = 0;
+    __syncthreads();
+    for (int e = threadIdx.x; e < (int)len; e += 256) {
+        const int4 h = p.hits[e];
+        if (h.z == (int)blockIdx.x) {
+            const int at = atomicAdd(&count, 1);
+            key[at] = (unsigned long long)h.x << 32 | (unsigned)h.y;
+            value[at] = __int_as_float(h.w);
+        }
+    }
+    __syncthreads();
+    const int m = count;
+    for (int e = threadIdx.x; e < m; e += 256) {
+        int at = 0;
+        for (int q = 0; q < m; ++q) at += key[q] < key[e] ? 1 : 0;
+        sorted[at] = value[e];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && m) {
+        float s = dsum[blockIdx.x];
+        for (int e = 0; e < m; ++e) s = __fadd_rn(s, sorted[e]);
+        dsum[blockIdx.x] = s;
+        nsum[blockIdx.x] += m;
+    }
+}
+
+int atomic_few_run(Context *c, const float *coords, const int *rows, int K, int n, int allAtoms, int flags, int ne,
+                   const float *basis_host, int isPBC, const int *mol, const int *el, const AtomicBlock &block,
+                   unsigned char *results, int *done, cudaStream_t st)
+{
+    *done = 0;
+    static const float kId[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
+    const float *Bh = isPBC && basis_host ? basis_host : kId;
+    FewParams p{};
+    p.a.coords = coords;
+    p.a.rows = rows;
+    p.a.K = K;
+    p.a.n = n;
+    p.a.allAtoms = allAtoms;
+    p.a.flags = flags;
+    p.a.ne = ne;
+    p.a.B = make_basis(Bh);
+    p.a.mol = mol;
+    p.a.el = el;
+    p.a.lower = block.lower();
+    p.a.upper = block.upper();
+    p.length = block.length();
+    FRMC_TRY(c->buf[BUF_ATOMIC_TOTALS].ensure(16 * kFewHits));
+    p.hits = c->buf[BUF_ATOMIC_TOTALS].as<int4>();
+    const unsigned g = (unsigned)((n + 255) / 256);
+    switch (basis_mode(Bh, isPBC)) {
+    case BM_IBC: k_few_rows<BM_IBC><<<g, 256, 0, st>>>(p); break;
+    case BM_DIAG: k_few_rows<BM_DIAG><<<g, 256, 0, st>>>(p); break;
+    case BM_XYTRI: k_few_rows<BM_XYTRI><<<g, 256, 0, st>>>(p); break;
+    case BM_LOWER: k_few_rows<BM_LOWER><<<g, 256, 0, st>>>(p); break;
+    default: k_few_rows<BM_GENERAL><<<g, 256, 0, st>>>(p); break;
+    }
+    k_few_sum<<<2 * ne * ne, 256, 0, st>>>(p, block.dsum(), block.nsum());
+    FRMC_CUDA(cudaGetLastError());
+    FRMC_CUDA(cudaMemcpyAsync(results, block.p, block.results(), cudaMemcpyDeviceToHost, st));
+    FRMC_CUDA(cudaStreamSynchronize(st));
+    long long len;
+    memcpy(&len, results + 16 * block.m, sizeof(len));
+    *done = len <= kFewHits;
     return FRMC_OK;
 }
 

@@ -132,10 +132,30 @@ static int upload_atoms(Context *c, const float *coords, const int32_t *mol, con
     return FRMC_OK;
 }
 
-// Full histogram counts of the atoms already uploaded by upload_atoms.
-static int full_counts(Context *c, int64_t n, const float *basis, int isPBC, int32_t ne, float minD, float maxD,
-                       float bin, int32_t hs, int64_t total, unsigned *counts)
+// The atoms' arrays as kernels may read them: the caller's own where the device
+// reads pageable host memory, else copies.
+static int device_atoms(Context *c, int64_t n, const float **coords, const int32_t **mol, const int32_t **el)
 {
+    if (c->pageable)
+        return FRMC_OK;
+    TRY(upload_atoms(c, *coords, *mol, *el, n));
+    *coords = c->buf[BUF_COORDS].as<float>();
+    *mol = c->buf[BUF_MOL].as<int>();
+    *el = c->buf[BUF_EL].as<int>();
+    return FRMC_OK;
+}
+
+// Below this many atoms the row kernel reads the caller's arrays itself (it
+// reads each column once per 64 rows), above it one kernel gathers them.
+constexpr int64_t kDirectAtoms = 512;
+
+// Full histogram counts of the caller's atoms; *waits: the kernel has device
+// waits and reports through the status word.
+static int full_counts(Context *c, const float *coords, const int32_t *mol, const int32_t *el, int64_t n,
+                       const float *basis, int isPBC, int32_t ne, float minD, float maxD, float bin, int32_t hs,
+                       int64_t total, unsigned *counts, bool *waits)
+{
+    *waits = false;
     const float *B = isPBC ? basis : kIdentity;
     const int bm = basis_mode(B, isPBC);
     Basis Bs = make_basis(B);
@@ -144,15 +164,33 @@ static int full_counts(Context *c, int64_t n, const float *basis, int isPBC, int
     // a tile configuration set by the caller keeps the tiled kernel
     if (tn == FullTune() && pairs >= kMinPairsCells && cell_hist_applies(n, bm, Bs, minD, maxD, bin, ne, hs)) {
         TRY(c->buf[BUF_CELLS].ensure(cell_hist_scratch((int)n)));
-        return launch_cell_hist(c->sms, c->max_smem_optin, c->buf[BUF_COORDS].as<float>(), nullptr,
-                                c->buf[BUF_EL].as<int>(), c->buf[BUF_MOL].as<int>(), (int)n, bm, Bs, minD, maxD, bin,
+        TRY(device_atoms(c, n, &coords, &mol, &el));
+        return launch_cell_hist(c->sms, c->max_smem_optin, coords, nullptr, el, mol, (int)n, bm, Bs, minD, maxD, bin,
                                 ne, hs, counts, counts + total, c->buf[BUF_CELLS].p, c->stream);
     }
-    if (pairs < tn.min_pairs_tiled) {
+    const bool rows = pairs < tn.min_pairs_tiled;
+    if (rows && c->pageable) {
+        if (n > kDirectAtoms) {
+            TRY(c->buf[BUF_COORDS].ensure(n * 12 + 16));
+            TRY(c->buf[BUF_EL].ensure(n * 4 + 16));
+            TRY(c->buf[BUF_MOL].ensure(n * 4 + 16));
+            TRY(launch_gather_atoms(coords, el, mol, (int)n, c->buf[BUF_COORDS].as<float>(), c->buf[BUF_EL].as<int>(),
+                                    c->buf[BUF_MOL].as<int>(), c->stream));
+            coords = c->buf[BUF_COORDS].as<float>();
+            el = c->buf[BUF_EL].as<int>();
+            mol = c->buf[BUF_MOL].as<int>();
+        }
+        return launch_rows_hist(coords, el, mol, (int)n, nullptr, (int)n, 0, bm, Bs, minD, maxD, bin, ne, hs, counts,
+                                counts + total, c->stream);
+    }
+    TRY(upload_atoms(c, coords, mol, el, n));
+    if (rows) {
         return launch_rows_hist(c->buf[BUF_COORDS].as<float>(), c->buf[BUF_EL].as<int>(), c->buf[BUF_MOL].as<int>(),
                                 (int)n, nullptr, (int)n, 0, bm, Bs, minD, maxD, bin, ne, hs, counts, counts + total,
                                 c->stream);
     }
+    *waits = true;
+    FRMC_CUDA(cudaMemsetAsync(c->buf[BUF_STATUS].p, 0, 4, c->stream));
     TRY(c->buf[BUF_ATOMS4].ensure(n * 16 + 16));
     float4 *a4 = c->buf[BUF_ATOMS4].as<float4>();
     TRY(launch_pack_atoms(c->buf[BUF_COORDS].as<float>(), c->buf[BUF_EL].as<int>(), (int)n, a4, c->stream));
@@ -162,9 +200,8 @@ static int full_counts(Context *c, int64_t n, const float *basis, int isPBC, int
 }
 
 // Zeroed counts for a call (skipping the memset where the previous call's
-// conversion left them zero) and, unless the call's kernels never set it, a
-// zero device status word.
-static int prepare_counts(Context *c, int64_t total, bool status = true)
+// conversion left them zero).
+static int prepare_counts(Context *c, int64_t total)
 {
     const size_t need = 2 * (size_t)total * 4;
     const void *before = c->buf[BUF_COUNTS].p;
@@ -176,42 +213,8 @@ static int prepare_counts(Context *c, int64_t total, bool status = true)
     if (c->counts_clean < need)
         FRMC_CUDA(cudaMemsetAsync(c->buf[BUF_COUNTS].p, 0, need, c->stream));
     c->counts_clean = 0;  // in use until a conversion resets them
-    if (status)
-        FRMC_CUDA(cudaMemsetAsync(c->buf[BUF_STATUS].p, 0, 4, c->stream));
     return FRMC_OK;
 }
-
-// Convert counts to float32 and copy both histograms back; checks the status.
-static int counts_out(Context *c, int64_t total, const float *h0intra, const float *h0inter, float *hintra,
-                      float *hinter)
-{
-    unsigned *cnt = c->buf[BUF_COUNTS].as<unsigned>();
-    float *out = c->buf[BUF_OUT].as<float>();
-    const float *d0i = nullptr, *d0e = nullptr;
-    if (h0intra) {
-        TRY(c->buf[BUF_AUX2].ensure(2 * total * 4 + 16));
-        float *h0 = c->buf[BUF_AUX2].as<float>();
-        TRY(h2d(h0, h0intra, total * 4, c->stream));
-        TRY(h2d(h0 + total, h0inter, total * 4, c->stream));
-        d0i = h0;
-        d0e = h0 + total;
-    }
-    TRY(launch_counts_to_f32(cnt, d0i, out, total, c->stream));
-    TRY(launch_counts_to_f32(cnt + total, d0e, out + total, total, c->stream));
-    TRY(d2h(hintra, out, total * 4, c->stream));
-    TRY(d2h(hinter, out + total, total * 4, c->stream));
-    uint32_t status = 0;
-    TRY(d2h(&status, c->buf[BUF_STATUS].p, 4, c->stream));
-    TRY(finish(c));
-    if (status)
-        return set_error(FRMC_E_TIMEOUT, "device wait gave up (status 0x%x)", status);
-    return FRMC_OK;
-}
-
-// Host-buffer calls with at most this many rows read the caller's arrays
-// directly where the device accesses pageable memory: the row kernel reads
-// every column once per 64 rows, so up to 64 rows read no more than a copy.
-constexpr int64_t kDirectRows = 64;
 
 // counts_out for pageable-access devices after kernels without device waits
 // (no status to read): one conversion kernel writes the caller's float32
@@ -223,6 +226,52 @@ static int counts_out_direct(Context *c, int64_t total, float *hintra, float *hi
     c->counts_clean = 2 * (size_t)total * 4;
     return finish(c);
 }
+
+// Histograms of at most this many bytes are written to the caller's arrays by
+// the conversion; larger ones, which may be pages that nothing has touched yet
+// (a kernel's first write to one takes 20 us, a copy's 4), are copied.
+constexpr int64_t kDirectBytes = 65536;
+
+// Convert counts to float32 and bring both histograms back; checks the status
+// of kernels with device waits.
+static int counts_out(Context *c, int64_t total, const float *h0intra, const float *h0inter, float *hintra,
+                      float *hinter, bool waits)
+{
+    if (!h0intra && !waits && c->pageable && total * 4 <= kDirectBytes)
+        return counts_out_direct(c, total, hintra, hinter);
+    unsigned *cnt = c->buf[BUF_COUNTS].as<unsigned>();
+    float *out = c->buf[BUF_OUT].as<float>();
+    const float *d0i = nullptr, *d0e = nullptr;
+    if (h0intra) {
+        TRY(c->buf[BUF_AUX2].ensure(2 * total * 4 + 16));
+        float *h0 = c->buf[BUF_AUX2].as<float>();
+        TRY(h2d(h0, h0intra, total * 4, c->stream));
+        TRY(h2d(h0 + total, h0inter, total * 4, c->stream));
+        d0i = h0;
+        d0e = h0 + total;
+    }
+    if (h0intra) {
+        TRY(launch_counts_to_f32(cnt, d0i, out, total, c->stream));
+        TRY(launch_counts_to_f32(cnt + total, d0e, out + total, total, c->stream));
+    } else {
+        TRY(launch_counts_pair_to_f32_zero(cnt, total, out, out + total, c->stream));
+        c->counts_clean = 2 * (size_t)total * 4;
+    }
+    TRY(d2h(hintra, out, total * 4, c->stream));
+    TRY(d2h(hinter, out + total, total * 4, c->stream));
+    uint32_t status = 0;
+    if (waits)
+        TRY(d2h(&status, c->buf[BUF_STATUS].p, 4, c->stream));
+    TRY(finish(c));
+    if (status)
+        return set_error(FRMC_E_TIMEOUT, "device wait gave up (status 0x%x)", status);
+    return FRMC_OK;
+}
+
+// Host-buffer calls with at most this many rows read the caller's arrays
+// directly where the device accesses pageable memory: the row kernel reads
+// every column once per 64 rows, so up to 64 rows read no more than a copy.
+constexpr int64_t kDirectRows = 64;
 
 }  // namespace frmc
 
@@ -461,11 +510,11 @@ int frmc_full_pairs_histograms_coords(const float *boxCoords, int64_t n, const f
         return FRMC_OK;
     }
     LOCKED_CTX(c);
-    TRY(upload_atoms(c, boxCoords, moleculeIndex, elementIndex, n));
+    bool waits = false;
     TRY(prepare_counts(c, total));
-    TRY(full_counts(c, n, basis, isPBC, ne, minDistance, maxDistance, bin, hs, total,
-                    c->buf[BUF_COUNTS].as<unsigned>()));
-    return counts_out(c, total, nullptr, nullptr, hintra, hinter);
+    TRY(full_counts(c, boxCoords, moleculeIndex, elementIndex, n, basis, isPBC, ne, minDistance, maxDistance, bin, hs,
+                    total, c->buf[BUF_COUNTS].as<unsigned>(), &waits));
+    return counts_out(c, total, nullptr, nullptr, hintra, hinter, waits);
 }
 
 int frmc_shape_function(const float *boxCoords, int64_t n, const float *basis, int isPBC,
@@ -487,41 +536,48 @@ int frmc_shape_function(const float *boxCoords, int64_t n, const float *basis, i
         if (elementIndex[i] < 0 || elementIndex[i] >= ne)
             return set_error(FRMC_E_INDEX, "element index %d out of range for %d elements", elementIndex[i], ne);
     LOCKED_CTX(c);
+    bool waits = false;
     TRY(prepare_counts(c, total));
     if (n >= 2) {
-        TRY(upload_atoms(c, boxCoords, moleculeIndex, elementIndex, n));
-        TRY(full_counts(c, n, basis, isPBC, ne, minDistance, maxDistance, bin, hs, total,
-                        c->buf[BUF_COUNTS].as<unsigned>()));
+        TRY(full_counts(c, boxCoords, moleculeIndex, elementIndex, n, basis, isPBC, ne, minDistance, maxDistance, bin,
+                        hs, total, c->buf[BUF_COUNTS].as<unsigned>(), &waits));
     }
-    // FP64 block: pc, r, vol, q, rv, G, S, Gs, w1, w2 (doubles), then pair_i, pair_j (ints)
-    const size_t nd = (size_t)npairs + 2 * (size_t)hs + (size_t)nq + (size_t)nr + (size_t)hs + (size_t)nq +
-                      (size_t)nr + (size_t)hs + (size_t)nq;
-    TRY(c->buf[BUF_AUX1].ensure(8 * nd + 8 * (size_t)npairs + 64));
+    // inputs in one copy: pair_i, pair_j (ints), pc, r, vol, q, rv (doubles);
+    // then G, S, Gs (one copy back), w1, w2
+    const size_t np2 = (size_t)npairs + (npairs & 1), ni = np2 + npairs + 2 * (size_t)hs + (size_t)nq + (size_t)nr;
+    const size_t nout = (size_t)hs + nq + nr, nd = ni + nout + (size_t)hs + (size_t)nq;
+    TRY(c->buf[BUF_AUX1].ensure(8 * nd + 64));
+    std::vector<double> in(ni, 0.0), out(nout);
+    int *hp = reinterpret_cast<int *>(in.data());
+    memcpy(hp, pair_i, 4 * (size_t)npairs);
+    memcpy(hp + np2, pair_j, 4 * (size_t)npairs);
+    double *h = in.data() + np2;
+    memcpy(h, pair_coef, 8 * (size_t)npairs);
+    memcpy(h + npairs, shellCenters, 8 * (size_t)hs);
+    memcpy(h + npairs + hs, shellVolumes, 8 * (size_t)hs);
+    memcpy(h + npairs + 2 * (size_t)hs, qValues, 8 * (size_t)nq);
+    memcpy(h + npairs + 2 * (size_t)hs + nq, rValues, 8 * (size_t)nr);
     double *d = c->buf[BUF_AUX1].as<double>();
-    double *pc = d, *r = pc + npairs, *vol = r + hs, *q = vol + hs, *rv = q + nq, *G = rv + nr, *S = G + hs,
+    TRY(h2d(d, in.data(), 8 * ni, c->stream));
+    const int *pij = reinterpret_cast<const int *>(d);
+    double *pc = d + np2, *r = pc + npairs, *vol = r + hs, *q = vol + hs, *rv = q + nq, *G = rv + nr, *S = G + hs,
            *Gs = S + nq, *w1 = Gs + nr, *w2 = w1 + hs;
-    int *pij = reinterpret_cast<int *>(w2 + nq);
-    TRY(h2d(pc, pair_coef, 8 * (size_t)npairs, c->stream));
-    TRY(h2d(r, shellCenters, 8 * (size_t)hs, c->stream));
-    TRY(h2d(vol, shellVolumes, 8 * (size_t)hs, c->stream));
-    TRY(h2d(q, qValues, 8 * (size_t)nq, c->stream));
-    TRY(h2d(rv, rValues, 8 * (size_t)nr, c->stream));
-    TRY(h2d(pij, pair_i, 4 * (size_t)npairs, c->stream));
-    TRY(h2d(pij + npairs, pair_j, 4 * (size_t)npairs, c->stream));
-    TRY(launch_shape_function(c->buf[BUF_COUNTS].as<unsigned>(), ne, hs, npairs, pij, pij + npairs, pc, r, vol, rho0,
+    TRY(launch_shape_function(c->buf[BUF_COUNTS].as<unsigned>(), ne, hs, npairs, pij, pij + np2, pc, r, vol, rho0,
                               shellCenters[1] - shellCenters[0], q, nq, qValues[1] - qValues[0], rv, nr, G, S, Gs,
                               w1, w2, c->stream));
-    if (Gr)
-        TRY(d2h(Gr, G, 8 * (size_t)hs, c->stream));
-    if (Sq)
-        TRY(d2h(Sq, S, 8 * (size_t)nq, c->stream));
-    if (Gshape)
-        TRY(d2h(Gshape, Gs, 8 * (size_t)nr, c->stream));
+    TRY(d2h(out.data(), G, 8 * nout, c->stream));
     uint32_t status = 0;
-    TRY(d2h(&status, c->buf[BUF_STATUS].p, 4, c->stream));
+    if (waits)
+        TRY(d2h(&status, c->buf[BUF_STATUS].p, 4, c->stream));
     TRY(finish(c));
     if (status)
         return set_error(FRMC_E_TIMEOUT, "device wait gave up (status 0x%x)", status);
+    if (Gr)
+        memcpy(Gr, out.data(), 8 * (size_t)hs);
+    if (Sq)
+        memcpy(Sq, out.data() + hs, 8 * (size_t)nq);
+    if (Gshape)
+        memcpy(Gshape, out.data() + hs + nq, 8 * (size_t)nr);
     return FRMC_OK;
 }
 
@@ -547,7 +603,7 @@ int frmc_multiple_pairs_histograms_coords(const int32_t *indexes, int64_t K, con
     const float *B = isPBC ? basis : kIdentity;
     LOCKED_CTX(c);
     const bool direct = c->pageable && K <= kDirectRows;
-    TRY(prepare_counts(c, total, !direct));  // the row kernels have no device waits
+    TRY(prepare_counts(c, total));
     unsigned *cnt = c->buf[BUF_COUNTS].as<unsigned>();
     if (direct) {
         // the per-move call (fullrmc's moved atoms, PairDistributionConstraints.py:1016-1026):
@@ -563,7 +619,7 @@ int frmc_multiple_pairs_histograms_coords(const int32_t *indexes, int64_t K, con
     TRY(launch_rows_hist(c->buf[BUF_COORDS].as<float>(), c->buf[BUF_EL].as<int>(), c->buf[BUF_MOL].as<int>(), (int)n,
                          c->buf[BUF_ROWS].as<int>(), (int)K, allAtoms, basis_mode(B, isPBC), make_basis(B),
                          minDistance, maxDistance, bin, ne, hs, cnt, cnt + total, c->stream));
-    return counts_out(c, total, nullptr, nullptr, hintra, hinter);
+    return counts_out(c, total, nullptr, nullptr, hintra, hinter, false);
 }
 
 int frmc_group_move_delta_histograms(const int32_t *indexes, int64_t K, const float *boxCoords, int64_t n,
@@ -647,7 +703,7 @@ int frmc_multiple_pairs_histograms_dists(const int32_t *indexes, int64_t K, cons
     TRY(launch_dists_hist(c->buf[BUF_AUX0].as<float>(), (int)n, (int)K, c->buf[BUF_ROWS].as<int>(),
                           c->buf[BUF_EL].as<int>(), c->buf[BUF_MOL].as<int>(), allAtoms, minDistance, maxDistance, bin,
                           ne, hs, cnt, cnt + total, c->stream));
-    return counts_out(c, total, nullptr, nullptr, hintra, hinter);
+    return counts_out(c, total, nullptr, nullptr, hintra, hinter, false);
 }
 
 int frmc_single_pairs_histograms(int32_t atomIndex, const float *distances, int64_t n, const int32_t *moleculeIndex,
@@ -675,7 +731,7 @@ int frmc_single_pairs_histograms(int32_t atomIndex, const float *distances, int6
     TRY(launch_dists_hist(c->buf[BUF_AUX0].as<float>(), (int)n, 1, c->buf[BUF_ROWS].as<int>(), c->buf[BUF_EL].as<int>(),
                           c->buf[BUF_MOL].as<int>(), allAtoms, minDistance, maxDistance, bin, ne, hs, cnt, cnt + total,
                           c->stream));
-    return counts_out(c, total, hintra, hinter, hintra, hinter);
+    return counts_out(c, total, hintra, hinter, hintra, hinter, false);
 }
 
 // ------------------------------------------------------------ FP64 transforms
@@ -722,50 +778,52 @@ static int atomic_checks(int64_t n, int64_t K, int32_t ne, const int32_t *el, in
     return FRMC_OK;
 }
 
-// Device accumulators [dsum 2 ne^2 floats][nsum 2 ne^2 ints], limits
-// [lower ne^2][upper ne^2]; starting values from the given arrays (or 0).
+// The call's AtomicBlock, in one copy: starting sums and numbers (the given
+// arrays, or 0), length 0 and the limits.
 static int atomic_prepare(Context *c, int32_t ne, const float *lower, const float *upper, const int32_t *nintra0,
-                          const float *dintra0, const int32_t *ninter0, const float *dinter0)
+                          const float *dintra0, const int32_t *ninter0, const float *dinter0, AtomicBlock *block)
 {
-    const size_t m = (size_t)ne * ne;
-    TRY(c->buf[BUF_ATOMIC_LIMITS].ensure(8 * m + 16));
-    TRY(c->buf[BUF_ATOMIC_ACC].ensure(16 * m + 16));
-    float *lim = c->buf[BUF_ATOMIC_LIMITS].as<float>();
-    TRY(h2d(lim, lower, 4 * m, c->stream));
-    TRY(h2d(lim + m, upper, 4 * m, c->stream));
-    float *acc = c->buf[BUF_ATOMIC_ACC].as<float>();
+    block->m = (size_t)ne * ne;
+    const size_t m = block->m;
+    TRY(c->buf[BUF_ATOMIC_ACC].ensure(block->bytes()));
+    block->p = c->buf[BUF_ATOMIC_ACC].as<unsigned char>();
+    std::vector<unsigned char> &host = block->host;
+    host.assign(block->bytes(), 0);
     if (dintra0) {
-        TRY(h2d(acc, dintra0, 4 * m, c->stream));
-        TRY(h2d(acc + m, dinter0, 4 * m, c->stream));
-        TRY(h2d(acc + 2 * m, nintra0, 4 * m, c->stream));
-        TRY(h2d(acc + 3 * m, ninter0, 4 * m, c->stream));
-    } else {
-        FRMC_CUDA(cudaMemsetAsync(acc, 0, 16 * m, c->stream));
+        memcpy(host.data(), dintra0, 4 * m);
+        memcpy(host.data() + 4 * m, dinter0, 4 * m);
+        memcpy(host.data() + 8 * m, nintra0, 4 * m);
+        memcpy(host.data() + 12 * m, ninter0, 4 * m);
     }
+    memcpy(host.data() + block->results(), lower, 4 * m);
+    memcpy(host.data() + block->results() + 4 * m, upper, 4 * m);
+    return h2d(block->p, host.data(), host.size(), c->stream);
+}
+
+static void atomic_results(const AtomicBlock &block, const unsigned char *r, int32_t *nintra, float *dintra,
+                           int32_t *ninter, float *dinter)
+{
+    const size_t m = block.m;
+    memcpy(dintra, r, 4 * m);
+    memcpy(dinter, r + 4 * m, 4 * m);
+    memcpy(nintra, r + 8 * m, 4 * m);
+    memcpy(ninter, r + 12 * m, 4 * m);
+}
+
+// The passes over all pairs, and the results.
+static int atomic_run(Context *c, const AtomicBlock &block, const float *dists_dev, int K, int n, int allAtoms,
+                      int flags, int ne, const float *basis, int isPBC, int32_t *nintra, float *dintra,
+                      int32_t *ninter, float *dinter)
+{
+    TRY(atomic_distances_run(c, dists_dev ? nullptr : c->buf[BUF_COORDS].as<float>(), dists_dev,
+                             c->buf[BUF_ROWS].as<int>(), K, n, allAtoms, flags, ne, basis, isPBC,
+                             c->buf[BUF_MOL].as<int>(), c->buf[BUF_EL].as<int>(), block.lower(), block.upper(),
+                             block.dsum(), block.nsum(), c->stream));
+    std::vector<unsigned char> r(block.results());
+    TRY(d2h(r.data(), block.p, r.size(), c->stream));
+    TRY(finish(c));
+    atomic_results(block, r.data(), nintra, dintra, ninter, dinter);
     return FRMC_OK;
-}
-
-static int atomic_finish(Context *c, int32_t ne, int32_t *nintra, float *dintra, int32_t *ninter, float *dinter)
-{
-    const size_t m = (size_t)ne * ne;
-    const float *acc = c->buf[BUF_ATOMIC_ACC].as<float>();
-    TRY(d2h(dintra, acc, 4 * m, c->stream));
-    TRY(d2h(dinter, acc + m, 4 * m, c->stream));
-    TRY(d2h(nintra, acc + 2 * m, 4 * m, c->stream));
-    TRY(d2h(ninter, acc + 3 * m, 4 * m, c->stream));
-    return finish(c);
-}
-
-static int atomic_run(Context *c, const float *dists_dev, int K, int n, int allAtoms, int flags, int ne,
-                      const float *basis, int isPBC)
-{
-    const size_t m = (size_t)ne * ne;
-    float *lim = c->buf[BUF_ATOMIC_LIMITS].as<float>();
-    float *acc = c->buf[BUF_ATOMIC_ACC].as<float>();
-    return atomic_distances_run(c, dists_dev ? nullptr : c->buf[BUF_COORDS].as<float>(), dists_dev,
-                                c->buf[BUF_ROWS].as<int>(), K, n, allAtoms, flags, ne, basis, isPBC,
-                                c->buf[BUF_MOL].as<int>(), c->buf[BUF_EL].as<int>(), lim, lim + m, acc,
-                                reinterpret_cast<int *>(acc + 2 * m), c->stream);
 }
 
 int frmc_multiple_atomic_distances_coords(const int32_t *indexes, int64_t K, const float *boxCoords, int64_t n,
@@ -780,21 +838,36 @@ int frmc_multiple_atomic_distances_coords(const int32_t *indexes, int64_t K, con
     bool all_rows = K == n && !allAtoms;
     for (int64_t k = 0; all_rows && k < K; ++k) all_rows = indexes[k] == k;
     LOCKED_CTX(c);
+    AtomicBlock block;
+    TRY(atomic_prepare(c, ne, lowerLimit, upperLimit, nullptr, nullptr, nullptr, nullptr, &block));
+    const float *dc = boxCoords;
+    const int *dm = moleculeIndex, *de = elementIndex, *rows = indexes;
+    const bool walk = all_rows && 0.5 * (double)n * (double)(n - 1) >= kMinPairsContacts;
+    if (walk || (K > 0 && n > 0 && K <= kFewRows)) {
+        std::vector<unsigned char> r(block.results());
+        int done = 0;
+        TRY(device_atoms(c, n, &dc, &dm, &de));
+        if (!c->pageable) {
+            TRY(c->buf[BUF_ROWS].ensure(K * 4 + 16));
+            TRY(h2d(c->buf[BUF_ROWS].p, indexes, K * 4, c->stream));
+            rows = c->buf[BUF_ROWS].as<int>();
+        }
+        if (walk)
+            TRY(atomic_contacts_run(c, dc, (int)n, flags, ne, basis, isPBC, dm, de, lowerLimit, upperLimit, block,
+                                    r.data(), &done, c->stream));
+        else
+            TRY(atomic_few_run(c, dc, rows, (int)K, (int)n, allAtoms, flags, ne, basis, isPBC, dm, de, block, r.data(),
+                               &done, c->stream));
+        if (done) {
+            atomic_results(block, r.data(), nintra, dintra, ninter, dinter);
+            return FRMC_OK;
+        }
+    }
     TRY(upload_atoms(c, boxCoords, moleculeIndex, elementIndex, n));
     TRY(c->buf[BUF_ROWS].ensure(K * 4 + 16));
     TRY(h2d(c->buf[BUF_ROWS].p, indexes, K * 4, c->stream));
-    TRY(atomic_prepare(c, ne, lowerLimit, upperLimit, nullptr, nullptr, nullptr, nullptr));
-    int done = 0;
-    if (all_rows && 0.5 * (double)n * (double)(n - 1) >= kMinPairsContacts) {
-        const size_t m = (size_t)ne * ne;
-        float *lim = c->buf[BUF_ATOMIC_LIMITS].as<float>(), *acc = c->buf[BUF_ATOMIC_ACC].as<float>();
-        TRY(atomic_contacts_run(c, c->buf[BUF_COORDS].as<float>(), (int)n, flags, ne, basis, isPBC,
-                                c->buf[BUF_MOL].as<int>(), c->buf[BUF_EL].as<int>(), lowerLimit, upperLimit, lim,
-                                lim + m, acc, reinterpret_cast<int *>(acc + 2 * m), &done, c->stream));
-    }
-    if (!done)
-        TRY(atomic_run(c, nullptr, (int)K, (int)n, allAtoms, flags, ne, basis, isPBC));
-    return atomic_finish(c, ne, nintra, dintra, ninter, dinter);
+    return atomic_run(c, block, nullptr, (int)K, (int)n, allAtoms, flags, ne, basis, isPBC, nintra, dintra, ninter,
+                      dinter);
 }
 
 int frmc_multiple_atomic_distances_dists(const int32_t *indexes, int64_t K, const float *distances, int64_t n,
@@ -813,9 +886,10 @@ int frmc_multiple_atomic_distances_dists(const int32_t *indexes, int64_t K, cons
     TRY(h2d(c->buf[BUF_AUX0].p, distances, (size_t)n * K * 4, c->stream));
     TRY(c->buf[BUF_ROWS].ensure(K * 4 + 16));
     TRY(h2d(c->buf[BUF_ROWS].p, indexes, K * 4, c->stream));
-    TRY(atomic_prepare(c, ne, lowerLimit, upperLimit, nullptr, nullptr, nullptr, nullptr));
-    TRY(atomic_run(c, c->buf[BUF_AUX0].as<float>(), (int)K, (int)n, allAtoms, flags, ne, nullptr, 0));
-    return atomic_finish(c, ne, nintra, dintra, ninter, dinter);
+    AtomicBlock block;
+    TRY(atomic_prepare(c, ne, lowerLimit, upperLimit, nullptr, nullptr, nullptr, nullptr, &block));
+    return atomic_run(c, block, c->buf[BUF_AUX0].as<float>(), (int)K, (int)n, allAtoms, flags, ne, nullptr, 0, nintra,
+                      dintra, ninter, dinter);
 }
 
 int frmc_single_atomic_distances_dists(int32_t atomIndex, const float *distances, int64_t n,
@@ -835,9 +909,10 @@ int frmc_single_atomic_distances_dists(int32_t atomIndex, const float *distances
     TRY(h2d(c->buf[BUF_AUX0].p, distances, (size_t)n * 4, c->stream));
     TRY(c->buf[BUF_ROWS].ensure(16));
     TRY(h2d(c->buf[BUF_ROWS].p, &atomIndex, 4, c->stream));
-    TRY(atomic_prepare(c, ne, lowerLimit, upperLimit, nintra, dintra, ninter, dinter));
-    TRY(atomic_run(c, c->buf[BUF_AUX0].as<float>(), 1, (int)n, allAtoms, flags, ne, nullptr, 0));
-    return atomic_finish(c, ne, nintra, dintra, ninter, dinter);
+    AtomicBlock block;
+    TRY(atomic_prepare(c, ne, lowerLimit, upperLimit, nintra, dintra, ninter, dinter, &block));
+    return atomic_run(c, block, c->buf[BUF_AUX0].as<float>(), 1, (int)n, allAtoms, flags, ne, nullptr, 0, nintra,
+                      dintra, ninter, dinter);
 }
 
 int frmc_pair_elements_stats(const int32_t *elementIndex, const int32_t *moleculeIndex, int64_t n, int32_t ne,
@@ -928,8 +1003,10 @@ static int coordination_by_walk(const float *boxCoords, int64_t n, const float *
         }
     }
     LOCKED_CTX(c);
-    TRY(upload_atoms(c, boxCoords, members, rows, n));
-    TRY(coordination_walk(c, c->buf[BUF_COORDS].as<float>(), c->buf[BUF_EL].as<int>(), c->buf[BUF_MOL].as<int>(), (int)n,
+    const float *dc = boxCoords;
+    const int *drows = rows, *dmembers = members;
+    TRY(device_atoms(c, n, &dc, &dmembers, &drows));
+    TRY(coordination_walk(c, dc, drows, dmembers, (int)n,
                           basis ? basis : kIdentity, isPBC, low, up, nslots, totals, done, c->stream));
     if (!*done)
         return FRMC_OK;

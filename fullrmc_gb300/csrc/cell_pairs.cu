@@ -39,10 +39,10 @@
 // an evaluated pair counts; per-lane queues of the counted pairs, as in
 // k_full_tiles, measured slower here (1.10 against 0.90 ms per call: the lanes
 // of a block have unequal numbers of neighbours).  Measured (whole host calls):
-// 100,000 atoms, 103 A box with gamma = 120, r 0-20 A: 6.92 -> 0.78 ms, the
+// 100,000 atoms, 103 A box with gamma = 120, r 0-20 A: 6.92 -> 0.73 ms, the
 // kernel 6.81 -> 0.62 ms for 5.1e5 of 4.9e6 block pairs, 34 issue slots per
-// column of 32 rows; 11,303 atoms, r 0-12 A: 335 -> 158 us; a 100,000-atom
-// particle with every pair counted (shape function): 12.5 -> 5.2 ms.
+// column of 32 rows; 11,303 atoms, r 0-12 A: 335 -> 118 us; a 100,000-atom
+// particle with every pair counted (shape function): 12.5 -> 5.3 ms.
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -56,9 +56,12 @@ constexpr int kCellCap = 1 << 16;     // cells at most (one CTA scans them)
 constexpr int kCellSub = 8;           // cells per block along a column
 
 struct CellSort {
-    const float *coords;     // (n, 3), or null: atoms4
-    const float4 *atoms4;    // (x, y, z, el bits)
-    const int *el, *mol;
+    // the caller's arrays (k_cell_bounds packs them; host memory where the
+    // device reads it), or null: the atoms are packed already
+    const float *coords;     // (n, 3)
+    const int *el, *src_mol;
+    float4 *atoms4;          // (x, y, z, el bits)
+    int *mol;
     int n, nb, ne, hs, pbc;
     Basis B;
     double volume;           // of the box (0: of the range of positions)
@@ -90,15 +93,6 @@ __device__ __forceinline__ float from_ordered(unsigned u)
     return __uint_as_float(u & 0x80000000u ? u & 0x7fffffffu : ~u);
 }
 
-__device__ __forceinline__ float3 cell_atom(const CellSort &p, int i)
-{
-    if (p.atoms4) {
-        const float4 a = p.atoms4[i];
-        return make_float3(a.x, a.y, a.z);
-    }
-    return make_float3(p.coords[3ll * i], p.coords[3ll * i + 1], p.coords[3ll * i + 2]);
-}
-
 // Position in real space (sorting and bounds only; the margin covers its rounding).
 __device__ __forceinline__ float3 cell_real(const CellSort &p, float3 c)
 {
@@ -109,30 +103,70 @@ __device__ __forceinline__ float3 cell_real(const CellSort &p, float3 c)
                        c.x * p.B.b[2] + c.y * p.B.b[5] + c.z * p.B.b[8]);
 }
 
+// The atoms' range, and their packed form where they come as three arrays:
+// 256 atoms a turn, whose 768 coordinates are read in order.  Bound by the link
+// to host memory: 100,000 atoms (2 MB) in 14 us, where three copies and an 8 us
+// kernel went before.
 __global__ void __launch_bounds__(256) k_cell_bounds(CellSort p)
 {
+    __shared__ float tile[3 * 256];
+    __shared__ unsigned red[7];
+    const int tid = threadIdx.x;
+    if (tid < 7)
+        red[tid] = 0u;
     float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY}, am = 0.f;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < p.n; i += gridDim.x * blockDim.x) {
-        const float3 c = cell_atom(p, i);
-        const float3 r = cell_real(p, c);
-        am = fmaxf(am, fmaxf(fabsf(c.x), fmaxf(fabsf(c.y), fabsf(c.z))));
-        if (!(fabsf(c.x) < INFINITY && fabsf(c.y) < INFINITY && fabsf(c.z) < INFINITY))
-            p.sc->strange = 1u;
+    bool strange = false;
+    for (int i0 = blockIdx.x * 256; i0 < p.n; i0 += gridDim.x * 256) {
+        const int i = i0 + tid;
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (p.coords) {
+            int el = 0, mol = 0;
+            if (i < p.n) {
+                el = p.el[i];
+                mol = p.src_mol[i];
+            }
+            const int m = 3 * min(256, p.n - i0);
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                if (tid + 256 * k < m)
+                    tile[tid + 256 * k] = p.coords[3ll * i0 + tid + 256 * k];
+            __syncthreads();
+            if (i < p.n) {
+                a = make_float4(tile[3 * tid], tile[3 * tid + 1], tile[3 * tid + 2], __int_as_float(el));
+                p.atoms4[i] = a;
+                p.mol[i] = mol;
+            }
+        } else if (i < p.n) {
+            a = p.atoms4[i];
+        }
+        if (i >= p.n)
+            continue;  // (every thread takes the same turns)
+        const float3 r = cell_real(p, make_float3(a.x, a.y, a.z));
+        am = fmaxf(am, fmaxf(fabsf(a.x), fmaxf(fabsf(a.y), fabsf(a.z))));
+        strange |= !(fabsf(a.x) < INFINITY && fabsf(a.y) < INFINITY && fabsf(a.z) < INFINITY);
         lo[0] = fminf(lo[0], r.x); lo[1] = fminf(lo[1], r.y); lo[2] = fminf(lo[2], r.z);
         hi[0] = fmaxf(hi[0], r.x); hi[1] = fmaxf(hi[1], r.y); hi[2] = fmaxf(hi[2], r.z);
     }
+    __syncthreads();
+    unsigned v[7];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        const unsigned a = __reduce_max_sync(0xffffffffu, ~ordered_bits(lo[k]));
-        const unsigned b = __reduce_max_sync(0xffffffffu, ordered_bits(hi[k]));
-        if ((threadIdx.x & 31u) == 0) {
-            atomicMax(&p.sc->nlo[k], a);
-            atomicMax(&p.sc->hi[k], b);
-        }
+        v[k] = ~ordered_bits(lo[k]);
+        v[3 + k] = ordered_bits(hi[k]);
     }
-    const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(am));
-    if ((threadIdx.x & 31u) == 0)
-        atomicMax(&p.sc->amax, m);
+    v[6] = __float_as_uint(am);
+#pragma unroll
+    for (int k = 0; k < 7; ++k) {
+        v[k] = __reduce_max_sync(0xffffffffu, v[k]);
+        if ((tid & 31) == 0)
+            atomicMax(&red[k], v[k]);
+    }
+    if (strange)
+        p.sc->strange = 1u;
+    __syncthreads();
+    if (tid < 7)
+        atomicMax(tid < 3 ? &p.sc->nlo[tid] : tid < 6 ? &p.sc->hi[tid - 3] : &p.sc->amax, red[tid]);
 }
 
 struct CellGeom {
@@ -185,7 +219,8 @@ __global__ void __launch_bounds__(256) k_cell_count(CellSort p)
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= p.n)
         return;
-    const float3 r = cell_real(p, cell_atom(p, i));
+    const float4 a = p.atoms4[i];
+    const float3 r = cell_real(p, make_float3(a.x, a.y, a.z));
     const int ix = cell_axis(g, 0, r.x), iy = cell_axis(g, 1, r.y), iz = cell_axis(g, 2, r.z);
     // serpentine: neighbouring columns join at the same end
     const int col = ix * g.n[1] + (ix & 1 ? g.n[1] - 1 - iy : iy);
@@ -250,8 +285,8 @@ __global__ void __launch_bounds__(256) k_cell_scatter(CellSort p)
     }
     const int2 pl = p.place[i];
     const int at = p.cells[pl.x] + pl.y;
-    const float3 c = cell_atom(p, i);
-    const int el = p.atoms4 ? __float_as_int(p.atoms4[i].w) : p.el[i];
+    const float4 c = p.atoms4[i];
+    const int el = __float_as_int(c.w);
     p.x[at] = -c.x;
     p.y[at] = -c.y;
     p.z[at] = -c.z;
@@ -473,21 +508,21 @@ bool cell_hist_applies(long long n, int bm, const Basis &B, float minD, float ma
     return top >= 0 && top < (1ll << 22) && top <= total;
 }
 
-size_t cell_hist_scratch(int n)
+size_t cell_hist_scratch(int n, size_t zeroed)
 {
     const size_t np = (size_t)(n + kCellBlock - 1) / kCellBlock * kCellBlock;
-    return 256 + up256(4 * (size_t)kCellCap) + up256(8 * (size_t)n) + 3 * up256(4 * np) + up256(16 * np) +
-           up256(48 * (np / kCellBlock));
+    return 256 + up256(4 * (size_t)kCellCap) + up256(zeroed) + up256(8 * (size_t)n) + 3 * up256(4 * np) +
+           up256(16 * np) + up256(48 * (np / kCellBlock)) + up256(16 * (size_t)n) + up256(4 * (size_t)n);
 }
 
 int sort_cells(int sms, const float *coords, const float4 *atoms4, const int *el, const int *mol, int n, int bm,
-               const Basis &B, float reach, int ne, int hs, void *scratch, CellWalk *walk, cudaStream_t st)
+               const Basis &B, float reach, int ne, int hs, void *scratch, CellWalk *walk, cudaStream_t st,
+               size_t zeroed, void **zero)
 {
     CellSort c{};
     c.coords = coords;
-    c.atoms4 = atoms4;
     c.el = el;
-    c.mol = mol;
+    c.src_mol = mol;
     c.n = n;
     c.nb = (n + kCellBlock - 1) / kCellBlock;
     c.ne = ne;
@@ -518,12 +553,21 @@ int sort_cells(int sms, const float *coords, const float4 *atoms4, const int *el
     const size_t np = (size_t)c.nb * kCellBlock;
     c.sc = reinterpret_cast<CellScalars *>(take(sizeof(CellScalars)));
     c.cells = reinterpret_cast<int *>(take(4 * (size_t)kCellCap));
+    unsigned char *extra = take(zeroed);
+    if (zero)
+        *zero = extra;
     c.place = reinterpret_cast<int2 *>(take(8 * (size_t)n));
     c.x = reinterpret_cast<float *>(take(4 * np));
     c.y = reinterpret_cast<float *>(take(4 * np));
     c.z = reinterpret_cast<float *>(take(4 * np));
     c.meta = reinterpret_cast<int4 *>(take(16 * np));
     c.bounds = reinterpret_cast<float4 *>(take(48 * (size_t)c.nb));
+    c.atoms4 = reinterpret_cast<float4 *>(take(16 * (size_t)n));
+    c.mol = reinterpret_cast<int *>(take(4 * (size_t)n));
+    if (!coords) {  // packed already; read only
+        c.atoms4 = const_cast<float4 *>(atoms4);
+        c.mol = const_cast<int *>(mol);
+    }
     h.nb = c.nb;
     h.x = c.x;
     h.y = c.y;
@@ -542,7 +586,8 @@ int sort_cells(int sms, const float *coords, const float4 *atoms4, const int *el
     while ((h.segw < 32 && all > 16 * warps * h.segw) || all > 256 * warps * h.segw) h.segw *= 2;
     h.nseg = (half + h.segw - 1) / h.segw;
 
-    FRMC_CUDA(cudaMemsetAsync(scratch, 0, 256 + 4 * (size_t)kCellCap, st));  // scalars and cell counts
+    // scalars, cell counts and what the caller wants zero
+    FRMC_CUDA(cudaMemsetAsync(scratch, 0, 256 + 4 * (size_t)kCellCap + zeroed, st));
     k_cell_bounds<<<std::min((n + 255) / 256, sms), 256, 0, st>>>(c);
     k_cell_count<<<(n + 255) / 256, 256, 0, st>>>(c);
     k_cell_scan<<<1, 1024, 0, st>>>(c.cells, c.sc, 0);
@@ -580,7 +625,7 @@ int launch_cell_hist(int sms, int max_smem_optin, const float *coords, const flo
                      unsigned *intra, unsigned *inter, void *scratch, cudaStream_t st)
 {
     CellHist h{};
-    FRMC_TRY(sort_cells(sms, coords, atoms4, el, mol, n, bm, B, maxD, ne, hs, scratch, &h.walk, st));
+    FRMC_TRY(sort_cells(sms, coords, atoms4, el, mol, n, bm, B, maxD, ne, hs, scratch, &h.walk, st, 0, nullptr));
     sq_limits(minD, maxD, &h.s_lo, &h.s_hi);
     h.minD = minD;
     h.binw = binw;

@@ -40,11 +40,14 @@ struct CellWalk {
 
 // Whether the walk can find the pairs of n atoms within `reach`.
 bool cell_walk_applies(long long n, int bm, const Basis &B, float reach);
-// Sorts the atoms on `st` into `scratch` (cell_hist_scratch(n) bytes, its
-// first 256 the CellScalars) and fills the walk over their pairs within
-// `reach`.  An atom's meta is (el * ne * hs, el * hs, molecule, index).
+// Sorts the atoms on `st` into `scratch` (cell_hist_scratch(n, zeroed) bytes,
+// its first 256 the CellScalars) and fills the walk over their pairs within
+// `reach`.  The atoms come as three arrays (device memory, or host memory that
+// the device reads) or packed with their molecules.  An atom's meta is
+// (el * ne * hs, el * hs, molecule, index).  `zeroed` bytes at *zero start as 0.
 int sort_cells(int sms, const float *coords, const float4 *atoms4, const int *el, const int *mol, int n, int bm,
-               const Basis &B, float reach, int ne, int hs, void *scratch, CellWalk *walk, cudaStream_t st);
+               const Basis &B, float reach, int ne, int hs, void *scratch, CellWalk *walk, cudaStream_t st,
+               size_t zeroed, void **zero);
 // CTAs of kCellThreads for a walk.
 int walk_grid(int sms, const CellWalk &w);
 // Exclusive scan in place of n counts, zero up to the next multiple of 4,096.

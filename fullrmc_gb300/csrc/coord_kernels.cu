@@ -247,8 +247,8 @@ int coordination_walk(Context *c, const float *coords, const int *row_mask, cons
     float s_lo;
     sq_limits(0.0f, reach, &s_lo, &p.s_hi);
     FRMC_TRY(c->buf[BUF_CELLS].ensure(cell_hist_scratch(n)));
-    FRMC_TRY(c->buf[BUF_ATOMIC_LIMITS].ensure(16 * kCoordSlots));
-    p.totals = c->buf[BUF_ATOMIC_LIMITS].as<unsigned long long>();
+    FRMC_TRY(c->buf[BUF_ATOMIC_ACC].ensure(16 * kCoordSlots));
+    p.totals = c->buf[BUF_ATOMIC_ACC].as<unsigned long long>();
     float *limits = reinterpret_cast<float *>(p.totals + kCoordSlots);
     p.lower = limits;
     p.upper = limits + kCoordSlots;
@@ -257,7 +257,7 @@ int coordination_walk(Context *c, const float *coords, const int *row_mask, cons
     memcpy(block + 12 * kCoordSlots, up, sizeof(up));
     FRMC_CUDA(cudaMemcpyAsync(p.totals, block, sizeof(block), cudaMemcpyHostToDevice, st));
     FRMC_TRY(sort_cells(c->sms, coords, nullptr, row_mask, member_mask, n, bm, B, reach, 1, 1, c->buf[BUF_CELLS].p,
-                        &p.walk, st));
+                        &p.walk, st, 0, nullptr));
     const int grid = walk_grid(c->sms, p.walk);
     switch (bm) {
     case BM_IBC: k_coord_walk<BM_IBC><<<grid, kCellThreads, 0, st>>>(p); break;

@@ -6,6 +6,7 @@
 
 #include <cstdint>
 #include <mutex>
+#include <vector>
 
 #include "frmc_gpu.h"
 #include "frmc_math.cuh"
@@ -65,7 +66,6 @@ enum BufRole {
     BUF_ATOMIC_LIST_B,
     BUF_ATOMIC_LIST_V,
     BUF_ATOMIC_ACC,
-    BUF_ATOMIC_LIMITS,
     BUF_COORD_LISTS,
     BUF_COORD_META,
     BUF_CELLS,
@@ -136,15 +136,16 @@ double accept_fraction(const float *basis, int isPBC, float minD, float maxD);
 long long full_hist_items(int n, const FullTune *tune);
 
 // The same histogram over spatially sorted atoms (cell_pairs.cu): block pairs
-// out of range are skipped.  Atoms as AoS coordinates with element indexes or
-// packed (atoms4); `scratch` holds cell_hist_scratch(n) bytes of device memory
+// out of range are skipped.  Atoms as AoS coordinates with element indexes (in
+// device memory, or host memory that the device reads) or packed (atoms4); `scratch` holds cell_hist_scratch(n) bytes of device memory
 // that nothing else uses until the work on `st` is done.  From kMinPairsCells
-// pairs the sort pays for itself: whole calls of 3,000 / 4,000 / 6,000 atoms
-// took 100 / 102 / 111 us sorted (r 8 A) against 89 / 103 us with the row
-// kernel and 279 us tiled; at 20 A 105 / 115 / 135 us against 135 / 199 / 558.
-constexpr double kMinPairsCells = 8.0e6;
+// pairs (2,450 atoms) the sort pays for itself: whole calls of 2,000 / 3,000 /
+// 3,990 atoms by the row kernel took 40 / 49 / 59 us at r 8 A, 64 / 93 / 110 us
+// at 15 A and 83 / 120 / 166 us at 20 A; sorted, 2,460 / 3,000 / 4,100 atoms take
+// 54 / 55 / 58, 55 / 61 / 65 and 78 / 80 / 84 us.
+constexpr double kMinPairsCells = 3.0e6;
 bool cell_hist_applies(long long n, int bm, const Basis &B, float minD, float maxD, float binw, int ne, int hs);
-size_t cell_hist_scratch(int n);
+size_t cell_hist_scratch(int n, size_t zeroed = 0);
 int launch_cell_hist(int sms, int max_smem_optin, const float *coords, const float4 *atoms4, const int *el,
                      const int *mol, int n, int bm, const Basis &B, float minD, float maxD, float binw, int ne, int hs,
                      unsigned *intra, unsigned *inter, void *scratch, cudaStream_t st);
@@ -182,20 +183,48 @@ int atomic_distances_run(Context *c, const float *coords, const float *dists, co
                          int allAtoms, int flags, int ne, const float *basis_host, int isPBC, const int *mol,
                          const int *el, const float *lower, const float *upper, float *dsum, int *nsum,
                          cudaStream_t st);
+// One call's accumulators in a block of device memory: the sums ([2][ne][ne]
+// floats), the numbers of pairs (ints), the list's length (int64), whether the
+// walk found atoms that it leaves to the other passes (uint32, padded to 8),
+// and the lower and upper limits.
+struct AtomicBlock {
+    size_t m = 0;  // ne * ne
+    unsigned char *p = nullptr;
+    std::vector<unsigned char> host;  // what was copied there (alive until the call's end)
+    float *dsum() const { return reinterpret_cast<float *>(p); }
+    int *nsum() const { return reinterpret_cast<int *>(p + 8 * m); }
+    long long *length() const { return reinterpret_cast<long long *>(p + 16 * m); }
+    unsigned *strange() const { return reinterpret_cast<unsigned *>(p + 16 * m + 8); }
+    float *lower() const { return reinterpret_cast<float *>(p + 16 * m + 16); }
+    float *upper() const { return lower() + m; }
+    size_t results() const { return 16 * m + 16; }  // bytes up to the limits
+    size_t bytes() const { return results() + 8 * m; }
+};
 // The same for all pairs i < j (rows 0 .. n - 1, allAtoms off) with limits
-// that bound the distance, by the walk over sorted atoms; *done is 0 where it
-// does not apply.  Synchronises `st`.  From kMinPairsContacts pairs: whole
-// calls of 260 / 520 / 1,040 atoms took 180 / 191 / 192 us by the walk and 179 /
-// 233 / 331 us by two passes over all pairs.
+// that bound the distance, by the walk over sorted atoms, from the caller's
+// arrays.  The results come back in `results` (AtomicBlock::results() bytes);
+// *done is 0, and the block's sums are as they were, where it does not apply.
+// Synchronises `st`.  From kMinPairsContacts pairs (1,800 atoms): whole calls of
+// 1,040 / 2,080 / 5,200 atoms took 142 / 143 / 157 us by the walk and 128 / 151 /
+// 276 us by two passes over all pairs.
 int atomic_contacts_run(Context *c, const float *coords, int n, int flags, int ne, const float *basis_host, int isPBC,
                         const int *mol, const int *el, const float *lower_host, const float *upper_host,
-                        const float *lower, const float *upper, float *dsum, int *nsum, int *done, cudaStream_t st);
-constexpr double kMinPairsContacts = 6.0e4;
+                        const AtomicBlock &block, unsigned char *results, int *done, cudaStream_t st);
+// A few rows' sums (K <= kFewRows) in one pass and one ordering, from the
+// caller's arrays; *done is 0 where they have more contacts than it orders.
+constexpr int kFewRows = 64;
+int atomic_few_run(Context *c, const float *coords, const int *rows, int K, int n, int allAtoms, int flags, int ne,
+                   const float *basis_host, int isPBC, const int *mol, const int *el, const AtomicBlock &block,
+                   unsigned char *results, int *done, cudaStream_t st);
+constexpr double kMinPairsContacts = 1.6e6;
 // pair_elements_stats counts ([2][ne][ne] int, zeroed by the caller).
 int launch_pair_stats(const int *el, const int *mol, int n, int ne, int *nintra, int *ninter, cudaStream_t st);
 
 // Pack AoS coordinates and element indexes into float4 (x, y, z, el bits).
 int launch_pack_atoms(const float *coords, const int *el, int n, float4 *out, cudaStream_t st);
+// AoS atoms from host memory that the device reads (5 n below 2^31).
+int launch_gather_atoms(const float *coords, const int *el, const int *mol, int n, float *dcoords, int *del, int *dmol,
+                        cudaStream_t st);
 // The inverse: float4 (x, y, z, el bits) -> AoS coordinates and elements.
 int launch_unpack_atoms(const float4 *atoms, int n, float *coords, int *el, cudaStream_t st);
 

@@ -605,6 +605,21 @@ __global__ void k_pack_atoms(const float *__restrict__ coords, const int *__rest
                              __int_as_float(el[i]));
 }
 
+// Three arrays of host memory that the device reads to device memory, in one
+// launch instead of three copies.
+__global__ void __launch_bounds__(256) k_gather_atoms(const float *__restrict__ coords, const int *__restrict__ el,
+                                                      const int *__restrict__ mol, int n, float *__restrict__ dcoords,
+                                                      int *__restrict__ del, int *__restrict__ dmol)
+{
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i < 3 * n)
+        dcoords[i] = coords[i];
+    else if (i < 4 * n)
+        del[i - 3 * n] = el[i - 3 * n];
+    else if (i < 5 * n)
+        dmol[i - 4 * n] = mol[i - 4 * n];
+}
+
 __global__ void k_unpack_atoms(const float4 *__restrict__ atoms, int n, float *__restrict__ coords,
                                int *__restrict__ el)
 {
@@ -811,6 +826,16 @@ int launch_counts_to_f32(const unsigned *counts, const float *h0, float *out, in
     if (blocks > 4096)
         blocks = 4096;
     k_counts_to_f32<<<(int)blocks, 256, 0, st>>>(counts, h0, out, total);
+    FRMC_CUDA(cudaGetLastError());
+    return FRMC_OK;
+}
+
+int launch_gather_atoms(const float *coords, const int *el, const int *mol, int n, float *dcoords, int *del, int *dmol,
+                        cudaStream_t st)
+{
+    if (n <= 0)
+        return FRMC_OK;
+    k_gather_atoms<<<(5 * n + 255) / 256, 256, 0, st>>>(coords, el, mol, n, dcoords, del, dmol);
     FRMC_CUDA(cudaGetLastError());
     return FRMC_OK;
 }
