@@ -24,6 +24,13 @@ int launch_transform(const float *M, const float *coords, int n, float *out, cud
 int launch_sine(int kind, const float *xs, int nx, const float *ys, const float *f, int ny, double rho, double *out,
                 double *scratch, cudaStream_t st);
 
+bool sine_fixed_scale(const float *xs, int64_t nx, const float *ys, const float *f, int64_t ny, int *scale);
+size_t sine_fixed_scratch(int64_t nx, int64_t ny);
+size_t sine_table_bytes();
+int sine_table_upload(void *table, cudaStream_t st);
+int launch_sine_fixed(int sms, int kind, const float *xs, int nx, const float *ys, const float *f, int ny, double rho,
+                      int scale, double *out, const void *table, void *scratch, cudaStream_t st);
+
 static FullTune g_full_tune;
 static std::mutex g_tune_mu;
 
@@ -751,9 +758,33 @@ static int sine_common(int kind, const float *xs, int64_t nx, const float *ys, c
     float *dxs = c->buf[BUF_AUX0].as<float>();
     float *dys = c->buf[BUF_AUX1].as<float>();
     float *df = dys + ny;
-    TRY(h2d(dxs, xs, nx * 4, c->stream));
-    TRY(h2d(dys, ys, ny * 4, c->stream));
-    TRY(h2d(df, f, ny * 4, c->stream));
+    int scale = 0;
+    const bool fixed = sine_fixed_scale(xs, nx, ys, f, ny, &scale);
+    if (!(fixed && c->pageable)) {
+        TRY(h2d(dxs, xs, nx * 4, c->stream));
+        TRY(h2d(dys, ys, ny * 4, c->stream));
+        TRY(h2d(df, f, ny * 4, c->stream));
+    }
+    if (fixed) {
+        if (!c->buf[BUF_SINE_TABLE].p) {
+            TRY(c->buf[BUF_SINE_TABLE].ensure(sine_table_bytes()));
+            TRY(sine_table_upload(c->buf[BUF_SINE_TABLE].p, c->stream));
+        }
+        TRY(c->buf[BUF_AUX2].ensure(sine_fixed_scratch(nx, ny)));
+        // outputs of up to 64 KiB go straight to the caller (larger ones may
+        // be pages that nothing has touched, which a kernel is slow to write)
+        const bool direct = c->pageable && nx * 8 <= kDirectBytes;
+        double *dout = direct ? out : c->buf[BUF_OUT].as<double>();
+        if (c->pageable)
+            TRY(launch_sine_fixed(c->sms, kind, xs, (int)nx, ys, f, (int)ny, rho, scale, dout,
+                                  c->buf[BUF_SINE_TABLE].p, c->buf[BUF_AUX2].p, c->stream));
+        else
+            TRY(launch_sine_fixed(c->sms, kind, dxs, (int)nx, dys, df, (int)ny, rho, scale, dout,
+                                  c->buf[BUF_SINE_TABLE].p, c->buf[BUF_AUX2].p, c->stream));
+        if (!direct)
+            TRY(d2h(out, dout, nx * 8, c->stream));
+        return finish(c);
+    }
     TRY(c->buf[BUF_AUX2].ensure(8 * (size_t)(nx + 2 * ny) + 16));
     TRY(launch_sine(kind, dxs, (int)nx, dys, df, (int)ny, rho, c->buf[BUF_OUT].as<double>(),
                     c->buf[BUF_AUX2].as<double>(), c->stream));

@@ -10,9 +10,18 @@
 //
 // The float32 inputs are promoted exactly, so every sine argument q*r is the
 // exact double product; only the summation order differs from a float64
-// numpy evaluation.  One CTA per output point (k_sine_rows), so a grid of a
-// few thousand points fills every SM.
+// numpy evaluation.
+//
+// Bound: GB300's narrow FP64 pipe (2 lanes a clock and SM: 16 cycles for a
+// warp's instruction).  sin() costs about 30 FP64 instructions a term; the
+// grids of the transforms let four do (k_sine_fixed).  k_sine_rows, one CTA per
+// output point with sin(), takes the grids that do not.  Whole calls, r 0-20 A
+// by 0.01 to Q 0.5-30 by 0.01 (5.9e6 terms): 281 -> 93 us, the kernel 243 -> 60
+// us.  Against 128-bit sums over six grids of the declared range both are off by
+// the same 8.8e-17 to 1.2e-16 of the result (ratio 0.96 to 1.02, mean 0.99).
+#include <algorithm>
 #include <cmath>
+#include <cstring>
 
 #include "frmc_runtime.h"
 
@@ -106,6 +115,284 @@ __global__ void k_sine_prep(int kind, const float *__restrict__ xs, int nx, cons
         yd[i] = y;
         w[i] = kind == SK_BIGGR_TO_SQ ? dy * v : dy * y * (v - 1.0);
     }
+}
+
+// ------------------------------------------------- sines in fixed point
+// Both grids are float32, so on a common scale the summation grid is integers,
+// y = Y 2^-e with Y < 2^37, and each output point is the fraction of a turn
+// X = x 2^-e / (2 pi) modulo 1, to 96 bits (Payne and Hanek's reduction: the
+// product of a float's integer with as many bits of 1 / (2 pi) as it needs).
+// The phase X Y modulo 1 is then a few integer multiply-adds, exact to 2^-59 of
+// a turn, and the integer pipes are thirty times as wide as the FP64 pipe.  Its
+// top 11 bits name one of 2,048 arcs, the others the place r in [-1/2, 1/2) of
+// its arc, and with h = 2 pi / 2048
+//   sin = T0 + T1 r + T2 r^2  (FP64: sin, h cos, -h^2/2 sin of the arc's centre)
+//       + (T0's rounding - h^3/6 cos r^3 + h^4/24 sin r^4)   (float32),
+// the last line below 1e-9 and so good to 1e-16 in float32, the next term of
+// the series below 7e-17.  Four FP64 instructions a term: r, two for the
+// polynomial, one for the weighted sum.
+constexpr int kArcs = 2048;
+constexpr int kSineThreads = 512;
+constexpr int kSineWarps = kSineThreads / 32;
+constexpr int kSineParts = 4;    // parts of an output point's sum, a warp each
+constexpr int kSineBatch = 64;   // output points of a CTA between two barriers
+
+struct __align__(16) SineArc {
+    double t0, t1, t2;
+    float low, t3;  // T0's rounding, -h^3/6 cos
+};
+struct SineTable {
+    SineArc arc[kArcs];
+    float t4[kArcs];  // h^4/24 sin
+};
+struct SineTerm {
+    unsigned y0, y1;
+    double w;
+};
+struct SinePoint {
+    unsigned x0, x1, x2;  // X, low word first
+    int zero;             // x is 0: every sine is
+    double x;
+};
+
+// Fixed-point fractions of 112 bits: a b.
+static unsigned __int128 fixed_mul(unsigned __int128 a, unsigned __int128 b)
+{
+    const unsigned long long al = (unsigned long long)a, ah = (unsigned long long)(a >> 64);
+    const unsigned long long bl = (unsigned long long)b, bh = (unsigned long long)(b >> 64);
+    return ((unsigned __int128)ah * bh << 16) + (((unsigned __int128)ah * bl + (unsigned __int128)al * bh) >> 48);
+}
+
+// The nearest double of a fraction, and what is left of it.
+static void fixed_split(unsigned __int128 v, double *hi, double *lo)
+{
+    *hi = std::ldexp((double)(unsigned long long)(v >> 48), -64);
+    const __int128 rest = (__int128)v - ((__int128)(unsigned long long)std::ldexp(*hi, 64) << 48);
+    *lo = std::ldexp((double)(long long)(rest >> 16), -96);
+}
+
+// The arcs' table from the Taylor series in fixed point (pi to 112 bits).
+static void sine_table(SineTable *t)
+{
+    const unsigned __int128 pi = (unsigned __int128)0x3243f6a8885a3ull << 64 | 0x08d313198a2e0370ull;
+    const double h = 2.0 * M_PI / kArcs;
+    for (int k = 0; k < kArcs / 4; ++k) {
+        const unsigned __int128 x = pi * (2 * k + 1) >> 11;  // the centre's angle in the first quadrant
+        const unsigned __int128 x2 = fixed_mul(x, x);
+        // cos above 1/2 and below: 1 - x^2/2 + ...; the terms fall below 2^-112
+        unsigned __int128 one = (unsigned __int128)1 << 112, sn = x, cs = one, ts = x, tc = one;
+        for (int i = 1; i < 20; ++i) {
+            tc = fixed_mul(tc, x2) / (unsigned)((2 * i - 1) * (2 * i));
+            ts = fixed_mul(ts, x2) / (unsigned)((2 * i) * (2 * i + 1));
+            cs = i & 1 ? cs - tc : cs + tc;
+            sn = i & 1 ? sn - ts : sn + ts;
+        }
+        double s, sl, c, cl;
+        fixed_split(sn, &s, &sl);
+        fixed_split(cs, &c, &cl);
+        for (int q = 0; q < 4; ++q) {
+            const double sv = q == 0 ? s : q == 1 ? c : q == 2 ? -s : -c;
+            const double lv = q == 0 ? sl : q == 1 ? cl : q == 2 ? -sl : -cl;
+            const double cv = q == 0 ? c : q == 1 ? -s : q == 2 ? -c : s;
+            SineArc &a = t->arc[q * (kArcs / 4) + k];
+            a.t0 = sv;
+            a.t1 = cv * h;
+            a.t2 = -sv * (h * h / 2.0);
+            a.low = (float)lv;
+            a.t3 = (float)(-cv * (h * h * h / 6.0));
+            t->t4[q * (kArcs / 4) + k] = (float)(sv * (h * h * h * h / 24.0));
+        }
+    }
+}
+
+// The scale of a summation grid: the smallest e with every y 2^e an integer,
+// below 2^37.  False for grids, values and output grids that the fixed-point
+// sines do not take (host arrays).
+bool sine_fixed_scale(const float *xs, int64_t nx, const float *ys, const float *f, int64_t ny, int *scale)
+{
+    int e = -200, top = -200;
+    float ymax = 0.0f;
+    for (int64_t i = 0; i < ny; ++i) {
+        const float y = ys[i];
+        if (!(y >= 0.0f && y < 1e30f) || !(std::fabs(f[i]) < 1e30f))
+            return false;
+        if (y == 0.0f)
+            continue;
+        uint32_t u;
+        memcpy(&u, &y, 4);
+        int ex = (int)(u >> 23);
+        uint32_t m = u & 0x7fffffu;
+        if (ex)
+            m |= 0x800000u;
+        else
+            ex = 1;
+        int low = ex - 150;  // y = m 2^low
+        while (!(m & 1u)) {
+            m >>= 1;
+            ++low;
+        }
+        e = std::max(e, -low);
+        ymax = std::max(ymax, y);
+    }
+    if (!(ymax > 0.0f))
+        return false;
+    std::frexp(ymax, &top);
+    if (top + e > 37 || e > 64 || e < -32)
+        return false;
+    for (int64_t i = 0; i < nx; ++i) {
+        const float x = xs[i];
+        // a sum over small arguments would feel the sines' absolute error
+        if (x != 0.0f && !(x > 0.0f && x < 1e6f && (double)x * ymax >= 0.02))
+            return false;
+    }
+    *scale = e;
+    return true;
+}
+
+__global__ void __launch_bounds__(256) k_sine_fixed_prep(int kind, const float *__restrict__ xs, int nx,
+                                                         const float *__restrict__ ys, const float *__restrict__ f,
+                                                         int ny, int e, SinePoint *__restrict__ point,
+                                                         SineTerm *__restrict__ term, float *__restrict__ wf)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < nx) {
+        const float x = xs[i];
+        const unsigned u = __float_as_uint(x), ex = max(u >> 23, 1u);
+        const unsigned m = (u & 0x7fffffu) | (u >> 23 ? 0x800000u : 0u);
+        // m times 1 / (2 pi) to 160 bits, then the 96 bits below the point
+        const unsigned inv[5] = {0x36d8a566u, 0x7d4d3770u, 0x7f09d5f4u, 0x9391054au, 0x28be60dbu};
+        unsigned p[7];
+        unsigned long long carry = 0;
+        for (int k = 0; k < 5; ++k) {
+            carry += (unsigned long long)m * inv[k];
+            p[k] = (unsigned)carry;
+            carry >>= 32;
+        }
+        p[5] = (unsigned)carry;
+        p[6] = 0u;
+        const int shift = 64 + e - ((int)ex - 150);  // value = m 2^(ex - 150 - e) / (2 pi)
+        unsigned w[3];
+        for (int k = 0; k < 3; ++k) {
+            const int b = shift + 32 * k, q = b >> 5, r = b & 31;
+            const unsigned lo = q >= 0 && q < 7 ? p[q] : 0u, hi = q + 1 >= 0 && q + 1 < 7 ? p[q + 1] : 0u;
+            w[k] = __funnelshift_r(lo, hi, r);
+        }
+        SinePoint pt;
+        pt.x0 = w[0];
+        pt.x1 = w[1];
+        pt.x2 = w[2];
+        pt.zero = x == 0.0f;
+        pt.x = (double)x;
+        point[i] = pt;
+    }
+    if (i < ny) {
+        const double dy = (double)ys[1] - (double)ys[0];
+        const double y = (double)ys[i], v = (double)f[i];
+        const unsigned long long Y = (unsigned long long)ldexp(y, e);
+        SineTerm t;
+        t.y0 = (unsigned)Y;
+        t.y1 = (unsigned)(Y >> 32);
+        t.w = Y == 0 ? 0.0 : kind == SK_BIGGR_TO_SQ ? dy * v : dy * y * (v - 1.0);
+        term[i] = t;
+        wf[i] = (float)t.w;
+    }
+}
+
+// CTA b takes the output points b, b + gridDim.x, ...; a warp sums a quarter
+// of a point's terms, lane by lane in order, and the parts are added in a fixed
+// tree, so the result depends on nothing but the inputs.
+__global__ void __launch_bounds__(kSineThreads, 1) k_sine_fixed(const SineTable *__restrict__ table,
+                                                                const SinePoint *__restrict__ point, int nx,
+                                                                const SineTerm *__restrict__ term,
+                                                                const float *__restrict__ wf, int ny, double add,
+                                                                double mul, int div, double *__restrict__ out)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    SineTable &t = *reinterpret_cast<SineTable *>(smem);
+    __shared__ double part[kSineBatch * kSineParts];
+    {
+        const uint4 *src = reinterpret_cast<const uint4 *>(table);
+        uint4 *dst = reinterpret_cast<uint4 *>(smem);
+        for (int k = threadIdx.x; k < (int)(sizeof(SineTable) / 16); k += kSineThreads) dst[k] = src[k];
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int mine = (nx - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;  // output points of this CTA
+    for (int o0 = 0; o0 < mine; o0 += kSineBatch) {
+        const int batch = min(kSineBatch, mine - o0);
+        for (int item = warp; item < batch * kSineParts; item += kSineWarps) {
+            const SinePoint pt = point[blockIdx.x + (o0 + item / kSineParts) * gridDim.x];
+            double acc = 0.0;
+            float side = 0.0f;
+#pragma unroll 2
+            for (int l = item % kSineParts * 32 + lane; l < ny; l += 32 * kSineParts) {
+                const SineTerm y = term[l];
+                const float w = wf[l];
+                unsigned long long d = (unsigned long long)pt.x0 * y.y0 >> 32;
+                d += (unsigned long long)pt.x1 * y.y0;
+                d += (unsigned long long)pt.x0 * y.y1;
+                d += (unsigned long long)(pt.x2 * y.y0 + pt.x1 * y.y1) << 32;
+                const int k = (int)(d >> 53);
+                const double r = __longlong_as_double((long long)(d >> 1 & 0xfffffffffffffull | 0x3ff0000000000000ull)) - 1.5;
+                const float rf = (float)(int)((unsigned)(d >> 21) ^ 0x80000000u) * 2.3283064365386963e-10f;  // 2^-32
+                const SineArc a = t.arc[k];
+                const float c = __fmaf_rn(__fmul_rn(__fmaf_rn(t.t4[k], rf, a.t3), rf), __fmul_rn(rf, rf), a.low);
+                acc = fma(y.w, fma(fma(a.t2, r, a.t1), r, a.t0), acc);
+                side = __fmaf_rn(w, c, side);
+            }
+            acc += (double)side;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+            if (lane == 0)
+                part[item] = pt.zero ? 0.0 : acc;
+        }
+        __syncthreads();
+        if ((int)threadIdx.x < batch) {
+            const double *p = part + threadIdx.x * kSineParts;
+            const double s = (p[0] + p[1]) + (p[2] + p[3]);
+            const int m = (int)blockIdx.x + (o0 + (int)threadIdx.x) * (int)gridDim.x;
+            out[m] = add + mul * (div ? s / point[m].x : s);
+        }
+        __syncthreads();
+    }
+}
+
+size_t sine_fixed_scratch(int64_t nx, int64_t ny)
+{
+    return sizeof(SineTable) + sizeof(SinePoint) * (size_t)nx + sizeof(SineTerm) * (size_t)ny + 4 * (size_t)ny + 64;
+}
+
+size_t sine_table_bytes() { return sizeof(SineTable); }
+
+// The arcs' table at the start of `scratch` (once per allocation).
+int sine_table_upload(void *scratch, cudaStream_t st)
+{
+    static const SineTable *table = [] {
+        SineTable *t = new SineTable();
+        sine_table(t);
+        return t;
+    }();
+    FRMC_CUDA(cudaMemcpyAsync(scratch, table, sizeof(SineTable), cudaMemcpyHostToDevice, st));
+    return FRMC_OK;
+}
+
+// The transform on grids that sine_fixed_scale took; the arrays and `out` in
+// device memory or host memory that the device reads and writes.
+int launch_sine_fixed(int sms, int kind, const float *xs, int nx, const float *ys, const float *f, int ny, double rho,
+                      int scale, double *out, const void *table, void *scratch, cudaStream_t st)
+{
+    SinePoint *point = static_cast<SinePoint *>(scratch);
+    SineTerm *term = reinterpret_cast<SineTerm *>(point + nx);
+    float *wf = reinterpret_cast<float *>(term + ny);
+    const int n = nx > ny ? nx : ny;
+    k_sine_fixed_prep<<<(n + 255) / 256, 256, 0, st>>>(kind, xs, nx, ys, f, ny, scale, point, term, wf);
+    FRMC_CUDA(cudaFuncSetAttribute(k_sine_fixed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SineTable)));
+    const double add = kind == SK_SQ_TO_GR ? 0.0 : 1.0;
+    const double mul = kind == SK_GR_TO_SQ ? 4.0 * M_PI * rho : kind == SK_BIGGR_TO_SQ ? 1.0 : 2.0 / M_PI;
+    k_sine_fixed<<<sms < nx ? sms : nx, kSineThreads, sizeof(SineTable), st>>>(
+        static_cast<const SineTable *>(table), point, nx, term, wf, ny, add, mul, kind != SK_SQ_TO_GR, out);
+    FRMC_CUDA(cudaGetLastError());
+    return FRMC_OK;
 }
 
 int launch_sine(int kind, const float *xs, int nx, const float *ys, const float *f, int ny, double rho, double *out,

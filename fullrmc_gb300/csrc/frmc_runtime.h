@@ -69,6 +69,7 @@ enum BufRole {
     BUF_COORD_LISTS,
     BUF_COORD_META,
     BUF_CELLS,
+    BUF_SINE_TABLE,
     BUF_COUNT_
 };
 
