@@ -483,51 +483,66 @@ __device__ __forceinline__ void column_bins(const V &D, float s0, float s1, bool
 
 constexpr int kItemUnroll = 4;
 
-// One item of the split path: the moved atom against atoms
-// [t*tile, (t+1)*tile).  For every column j the pair before and after the
-// move is binned; a changed bin adds -1 / +1 to the engine's global oriented
-// delta and element-pair delta, and its oriented index is appended to the
-// touched list (one list reservation per warp and column).  Coordinates of
-// kItemUnroll columns are loaded before any is used.
-template <int BM>
-__device__ void item_delta(const EDesc &Dg, int tile, const MovedGroup &g, int t)
+// One item of the split path: columns [v0, v1) of the step's sweep -- all
+// atoms, or with a column grid those of the selected cells (cell_select) --
+// against the moved atoms.  A thread takes one (column, moved atom) pair at a
+// time, the columns of a warp in order; the pair before and after the move is
+// binned, and a changed bin adds -1 / +1 to the engine's global oriented delta
+// and element-pair delta.  The additions return nothing, so no thread waits
+// for them: a touched list, which needs its place from a shared counter, cost a
+// warp a round trip to L2 for every moved atom and is kept only for engines
+// with an S(Q) term (LIST), whose kernel commits through it.
+//
+// cols: kSplitCols ints of shared memory (the chunk's columns, -1 for moved
+// atoms).
+constexpr int kSplitCols = 1024;
+constexpr int kSplitTiles = 144;  // items of a split step whose columns are few
+
+__device__ __forceinline__ int cell_column(const int *P, const int *Bse, int nc, int v);
+
+template <int BM, bool LIST>
+__device__ void item_delta(const EDesc &Dg, int v0, int v1, const MovedGroup &g, const int *cP, const int *cB, int *cols)
 {
-    const ColView D = col_view(Dg);
+    ColView D = col_view(Dg);
+    const int nc = Dg.nc;
+    if (nc > 0) {
+        D.box = Dg.cbox;
+        D.mol = Dg.cmol;
+    }
     int *__restrict__ delta = Dg.delta;
     int *__restrict__ dP = Dg.dP;
     unsigned *tcount = &Dg.st->tcount;
-    const int j0 = t * tile;
-    const int j1 = min(D.n, j0 + tile);
     const int G = g.n;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned lt = (1u << lane) - 1u;
-    for (int jb = j0; jb < j1; jb += kItemUnroll * blockDim.x) {
-        float4 c[kItemUnroll];
-        int mj[kItemUnroll];
-        bool valid[kItemUnroll];
-#pragma unroll
-        for (int u = 0; u < kItemUnroll; ++u) {
-            const int j = jb + u * blockDim.x + threadIdx.x;
-            c[u] = j < j1 ? D.box[j] : make_float4(0.f, 0.f, 0.f, 0.f);
-            mj[u] = j < j1 ? D.mol[j] : 0;
-            bool ok = j < j1;
-            for (int q = 0; q < G; ++q) ok &= j != g.atom[q];
-            valid[u] = ok;
+    for (int c0 = v0; c0 < v1; c0 += kSplitCols) {
+        const int m = min(kSplitCols, v1 - c0);
+        for (int k = threadIdx.x; k < m; k += blockDim.x) {
+            int j = nc > 0 ? cell_column(cP, cB, nc, c0 + k) : c0 + k;
+            for (int q = 0; q < G; ++q) j = j == (nc > 0 ? g.slot[q] : g.atom[q]) ? -1 : j;
+            cols[k] = j;
         }
-        for (int gi = 0; gi < G; ++gi) {
-            const float3 o = make_float3(g.o[gi][0], g.o[gi][1], g.o[gi][2]);
-            const float3 nw = make_float3(g.nw[gi][0], g.nw[gi][1], g.nw[gi][2]);
-            const int ela = g.el[gi], mola = g.mol[gi], arow = ela * D.ne;
-            float s0[kItemUnroll], s1[kItemUnroll];
-#pragma unroll
-            for (int u = 0; u < kItemUnroll; ++u) {
-                s0[u] = pair_s<BM>(o.x, o.y, o.z, c[u].x, c[u].y, c[u].z, D.B);
-                s1[u] = pair_s<BM>(nw.x, nw.y, nw.z, c[u].x, c[u].y, c[u].z, D.B);
+        __syncthreads();
+        // (the loop is the same for every thread of a warp: LIST votes)
+        const int tasks = m * G;
+#pragma unroll 2
+        for (int t0 = 0; t0 < tasks; t0 += blockDim.x) {
+            const int t = t0 + threadIdx.x;
+            const int gi = t < tasks ? t / m : 0;
+            const int j = t < tasks ? cols[t - gi * m] : -1;
+            float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+            int mj = 0;
+            if (j >= 0) {
+                c = D.box[j];
+                mj = D.mol[j];
             }
-#pragma unroll
-            for (int u = 0; u < kItemUnroll; ++u) {
-                int f0 = -1, f1 = -1, half = 0, b0 = 0, b1 = 0, elj = 0;
-                column_bins(D, s0[u], s1[u], valid[u], c[u], mj[u], arow, mola, f0, f1, half, b0, b1, elj);
+            const int ela = g.el[gi];
+            const float s0 = pair_s<BM>(g.o[gi][0], g.o[gi][1], g.o[gi][2], c.x, c.y, c.z, D.B);
+            const float s1 = pair_s<BM>(g.nw[gi][0], g.nw[gi][1], g.nw[gi][2], c.x, c.y, c.z, D.B);
+            int f0 = -1, f1 = -1, half = 0, b0 = 0, b1 = 0, elj = 0;
+            column_bins(D, s0, s1, j >= 0, c, mj, ela * D.ne, g.mol[gi], f0, f1, half, b0, b1, elj);
+            unsigned pos = 0;
+            if (LIST) {
                 const unsigned m0 = __ballot_sync(0xffffffffu, f0 >= 0);
                 const unsigned m1 = __ballot_sync(0xffffffffu, f1 >= 0);
                 if ((m0 | m1) == 0u)
@@ -536,25 +551,28 @@ __device__ void item_delta(const EDesc &Dg, int tile, const MovedGroup &g, int t
                 if (lane == 0)
                     base = atomicAdd(tcount, __popc(m0) + __popc(m1));
                 base = __shfl_sync(0xffffffffu, base, 0);
-                unsigned pos = base + __popc(m0 & lt) + __popc(m1 & lt);
-                if (f0 >= 0) {
-                    atomicSub(delta + half + f0, 1);
+                pos = base + __popc(m0 & lt) + __popc(m1 & lt);
+            }
+            if (f0 >= 0) {
+                atomicSub(delta + half + f0, 1);
+                if (LIST)
                     D.tlist[pos++] = half + f0;
-                    int p, b;
-                    pair_of_flat(D, f0, ela, elj, b0, p, b);
-                    if (p >= 0)
-                        atomicSub(dP + p * D.hs + b, 1);
-                }
-                if (f1 >= 0) {
-                    atomicAdd(delta + half + f1, 1);
+                int p, b;
+                pair_of_flat(D, f0, ela, elj, b0, p, b);
+                if (p >= 0)
+                    atomicSub(dP + p * D.hs + b, 1);
+            }
+            if (f1 >= 0) {
+                atomicAdd(delta + half + f1, 1);
+                if (LIST)
                     D.tlist[pos] = half + f1;
-                    int p, b;
-                    pair_of_flat(D, f1, ela, elj, b1, p, b);
-                    if (p >= 0)
-                        atomicAdd(dP + p * D.hs + b, 1);
-                }
+                int p, b;
+                pair_of_flat(D, f1, ela, elj, b1, p, b);
+                if (p >= 0)
+                    atomicAdd(dP + p * D.hs + b, 1);
             }
         }
+        __syncthreads();  // the columns are listed again
     }
 }
 
@@ -1039,10 +1057,11 @@ __device__ void split_group_internal(const EDesc &Dg, const MovedGroup &g)
         const unsigned cnt = (f0 >= 0) + (f1 >= 0);
         if (!cnt)
             continue;
-        unsigned pos = atomicAdd(&Dg.st->tcount, cnt);
+        unsigned pos = Dg.sq ? atomicAdd(&Dg.st->tcount, cnt) : 0u;
         if (f0 >= 0) {
             atomicSub(Dg.delta + half + f0, 1);
-            D.tlist[pos++] = half + f0;
+            if (Dg.sq)
+                D.tlist[pos++] = half + f0;
             int p, bb;
             pair_of_flat(D, f0, ela, elj, b0, p, bb);
             if (p >= 0)
@@ -1050,7 +1069,8 @@ __device__ void split_group_internal(const EDesc &Dg, const MovedGroup &g)
         }
         if (f1 >= 0) {
             atomicAdd(Dg.delta + half + f1, 1);
-            D.tlist[pos] = half + f1;
+            if (Dg.sq)
+                D.tlist[pos] = half + f1;
             int p, bb;
             pair_of_flat(D, f1, ela, elj, b1, p, bb);
             if (p >= 0)
@@ -1108,22 +1128,39 @@ __device__ void finish_engine(const EDesc &D, const MovedGroup &g, double *red, 
     }
     __syncthreads();
     const bool accept = *s_flag != 0;
-    // commit (or drop) the oriented delta through the touched list; duplicates
-    // are harmless: atomicExch hands each bin's delta to exactly one entry
-    const unsigned nt = __ldcg(&D.st->tcount);
-    for (unsigned k0 = threadIdx.x; k0 < nt; k0 += kCommitUnroll * blockDim.x) {
-        int f[kCommitUnroll], d[kCommitUnroll];
+    // commit (or drop) the oriented delta: the whole array once, in order and
+    // with kCommitUnroll quads in flight per thread (a group move of 13 atoms
+    // touches 36,000 entries of its 27,000 bins; through a list each took a
+    // dependent load, an exchange and an addition)
+    {
+        const int quads = (int)((2 * D.total + 3) / 4);  // the array is padded and zero past its end
+        int4 *dq = reinterpret_cast<int4 *>(D.delta);
+        int4 *cq = reinterpret_cast<int4 *>(D.counts);
+        for (int k0 = threadIdx.x; k0 < quads; k0 += kCommitUnroll * blockDim.x) {
+            int4 d[kCommitUnroll];
+            bool any[kCommitUnroll];
 #pragma unroll
-        for (int u = 0; u < kCommitUnroll; ++u) {
-            const unsigned k = k0 + u * blockDim.x;
-            f[u] = k < nt ? __ldcg(D.tlist + k) : -1;
-        }
+            for (int u = 0; u < kCommitUnroll; ++u) {
+                const int k = k0 + u * (int)blockDim.x;
+                d[u] = k < quads ? __ldcg(dq + k) : make_int4(0, 0, 0, 0);
+                any[u] = (d[u].x | d[u].y | d[u].z | d[u].w) != 0;
+            }
+            if (accept) {
+                int4 n[kCommitUnroll];
 #pragma unroll
-        for (int u = 0; u < kCommitUnroll; ++u) d[u] = f[u] >= 0 ? atomicExch(D.delta + f[u], 0) : 0;
-        if (accept) {
+                for (int u = 0; u < kCommitUnroll; ++u)
+                    if (any[u])
+                        n[u] = cq[k0 + u * (int)blockDim.x];
+#pragma unroll
+                for (int u = 0; u < kCommitUnroll; ++u)
+                    if (any[u])
+                        cq[k0 + u * (int)blockDim.x] =
+                            make_int4(n[u].x + d[u].x, n[u].y + d[u].y, n[u].z + d[u].z, n[u].w + d[u].w);
+            }
 #pragma unroll
             for (int u = 0; u < kCommitUnroll; ++u)
-                if (d[u]) D.counts[f[u]] += d[u];
+                if (any[u])
+                    dq[k0 + u * (int)blockDim.x] = make_int4(0, 0, 0, 0);
         }
     }
     // on accept G += R S, hence Bq -= 2 A S on the bins that changed
@@ -1766,7 +1803,7 @@ __global__ void __launch_bounds__(kMaxEngineThreads, 1) k_engine_step(StepParams
     __shared__ unsigned s_tcount;
     __shared__ int s_last, s_flag, s_item;
     __shared__ __align__(8) uint64_t s_bar;
-    // fused items read their descriptor from this copy: the sweep streams the
+    // items read their descriptor from this copy: the sweep streams the
     // engine's columns through L1, which would otherwise evict the descriptor
     // and turn every later field read into an L2 round trip
     __shared__ __align__(16) EDesc s_desc;
@@ -1792,28 +1829,28 @@ __global__ void __launch_bounds__(kMaxEngineThreads, 1) k_engine_step(StepParams
         }
         __syncthreads();
     }
-    // a fused launch with an item per CTA needs no scheduler: CTA b takes
-    // item b and leaves
-    const bool one_each = FUSED && p.nitems <= (int)gridDim.x;
+    // a launch with an item per CTA needs no scheduler: CTA b takes item b and
+    // leaves
+    const bool one_each = p.nitems <= (int)gridDim.x;
+    bool first_item = true;
     for (;;) {
         if (threadIdx.x == 0) {
-            // fused launches: item blockIdx.x first (the list is largest
-            // first), then items gridDim.x, gridDim.x + 1, ... by claim
+            // item blockIdx.x first (fused lists are largest first), then
+            // items gridDim.x, gridDim.x + 1, ... by claim
             unsigned long long k;
-            if (FUSED)
-                k = fused_items == 0 ? blockIdx.x
-                                     : (one_each ? (unsigned long long)p.nitems
-                                                 : gridDim.x + atomicAdd(&p.sched->claimed, 1ull));
-            else
-                k = atomicAdd(&p.sched->claimed, 1ull);
+            k = first_item ? blockIdx.x
+                           : (one_each ? (unsigned long long)p.nitems
+                                       : gridDim.x + atomicAdd(&p.sched->claimed, 1ull));
+            first_item = false;
             s_item = k < (unsigned long long)p.nitems ? (int)k : -1;
         }
         __syncthreads();
         const int it = s_item;
-        if (FUSED && it >= 0) {
+        if (it >= 0) {
             // the previous item's last reads of s_desc came before the
             // barrier that ended it
-            const long long *src = reinterpret_cast<const long long *>(p.fdesc + it);
+            const long long *src =
+                reinterpret_cast<const long long *>(FUSED ? p.fdesc + it : p.desc + p.items[it].x);
             long long *dst = reinterpret_cast<long long *>(&s_desc);
             for (int k = threadIdx.x; k < (int)(sizeof(EDesc) / 8); k += blockDim.x) dst[k] = src[k];
         }
@@ -1821,7 +1858,7 @@ __global__ void __launch_bounds__(kMaxEngineThreads, 1) k_engine_step(StepParams
         if (it < 0)
             break;
         const int2 item = FUSED ? make_int2(0, -1) : p.items[it];
-        const EDesc &D = FUSED ? p.fdesc[it] : p.desc[item.x];
+        const EDesc &D = s_desc;
         if (FUSED && fused_items == 0 && threadIdx.x == 32)
             warm_item(p, (long long)it + gridDim.x);
         if (FUSED) {
@@ -1860,15 +1897,47 @@ __global__ void __launch_bounds__(kMaxEngineThreads, 1) k_engine_step(StepParams
             __syncthreads();
             continue;
         }
+        // the column grid's prefix and bases and the item's columns live in the
+        // evaluation scratch until the evaluation
+        int *cP = reinterpret_cast<int *>(cb), *cB = cP + kMaxCells + 1, *cols = cP + kCellInts;
+        static_assert(FUSED || sizeof(cb_s) >= sizeof(int) * (kCellInts + kSplitCols), "cb too small");
+        const int nc = D.nc;
+        float4 clo = make_float4(0.f, 0.f, 0.f, 0.f), chi = clo, clo1 = clo, chi1 = clo;
+        int cs0 = 0, cs1 = 0, cs01 = 0, cs11 = 0;
+        if ((int)threadIdx.x < nc) {
+            clo = D.clo[threadIdx.x];
+            chi = D.chi[threadIdx.x];
+            cs0 = D.cstart[threadIdx.x];
+            cs1 = D.cstart[threadIdx.x + 1];
+        }
+        if ((int)(threadIdx.x + blockDim.x) < nc) {
+            const int c = threadIdx.x + blockDim.x;
+            clo1 = D.clo[c];
+            chi1 = D.chi[c];
+            cs01 = D.cstart[c];
+            cs11 = D.cstart[c + 1];
+        }
         load_moved_group(D, D.st->step, s_group);
         __syncthreads();
-        switch (D.bm) {
-        case BM_IBC: item_delta<BM_IBC>(D, p.tile, s_group, item.y); break;
-        case BM_DIAG: item_delta<BM_DIAG>(D, p.tile, s_group, item.y); break;
-        case BM_XYTRI: item_delta<BM_XYTRI>(D, p.tile, s_group, item.y); break;
-        case BM_LOWER: item_delta<BM_LOWER>(D, p.tile, s_group, item.y); break;
-        default: item_delta<BM_GENERAL>(D, p.tile, s_group, item.y); break;
+        __shared__ float4 s_cell0[2];
+        const int ncol = nc > 0 ? cell_select(D, s_group, clo, chi, cs0, cs1, cP, cB, cB + kMaxCells, clo1, chi1, cs01,
+                                              cs11, s_cell0)
+                                : D.n;
+        const int v0 = (int)((long long)ncol * item.y / D.ntiles), v1 = (int)((long long)ncol * (item.y + 1) / D.ntiles);
+#define FRMC_ITEM(L_)                                                                                \
+    switch (D.bm) {                                                                                  \
+    case BM_IBC: item_delta<BM_IBC, L_>(D, v0, v1, s_group, cP, cB, cols); break;                    \
+    case BM_DIAG: item_delta<BM_DIAG, L_>(D, v0, v1, s_group, cP, cB, cols); break;                  \
+    case BM_XYTRI: item_delta<BM_XYTRI, L_>(D, v0, v1, s_group, cP, cB, cols); break;                \
+    case BM_LOWER: item_delta<BM_LOWER, L_>(D, v0, v1, s_group, cP, cB, cols); break;                \
+    default: item_delta<BM_GENERAL, L_>(D, v0, v1, s_group, cP, cB, cols); break;                    \
+    }
+        if (D.sq) {
+            FRMC_ITEM(true)
+        } else {
+            FRMC_ITEM(false)
         }
+#undef FRMC_ITEM
         // Release: the barrier orders every thread's delta atomics and
         // touched-list stores before thread 0's gpu-scope fence, which is
         // cumulative, so they are visible to the CTA that sees the count.
@@ -2694,6 +2763,10 @@ struct Slot {
     // atoms, or with a column grid the estimate, counted 4 times: a grid
     // column is gathered and mostly in range), times the atoms a move moves
     long long cost = 0;
+    // what a one-engine step weighs against kSoloFusedWork: the columns in
+    // range at the mean density and a quarter of those swept (0: free
+    // boundaries, whose density is not known)
+    long long work = 0;
     EDesc d;
     void *blob = nullptr;
     size_t bytes = 0;
@@ -2733,7 +2806,12 @@ static long long fused_dyn_bytes(long long dp_ints, int bins, int threads)
 }
 
 constexpr long long kFusedMaxCost = 49152;  // engines of a higher step cost (Slot::cost) are split over several CTAs
-constexpr long long kSoloFusedCost = 16384;  // one-engine steps up to this cost use the fused item
+constexpr long long kSoloFusedCost = 16384;  // one-engine steps up to this cost use the fused item,
+// and up to this work (Slot::work): a step of 3,000 / 5,000 / 8,000 / 14,000 atoms
+// at r 20 A (work 3,750 / 4,600 / 5,350 / 6,850) takes 20.7 / 23.9 / 26.0 / 28.5 us
+// fused and 21.6 / 20.8 / 21.7 / 21.0 us split; of 5,000 atoms at 15 A (2,660) 17.7
+// either way, of 30,000 at 12 A (1,310) 17.1 and 19.7 us
+constexpr long long kSoloFusedWork = 3900;
 
 struct EngineSet {
     std::vector<Slot> slots;
@@ -2803,6 +2881,16 @@ struct EngineSet {
     std::vector<int> place_order;       // engine id per fused item, or empty
     long long place_key = -1;           // the launch shape the order was measured for
 };
+
+static long long solo_work(const Slot &sl)
+{
+    const EDesc &D = sl.d;
+    if (D.bm == BM_IBC)
+        return 0;
+    const double in_range = accept_fraction(D.B.b, 1, D.minD, D.maxD) * (double)D.n * D.group;
+    const double swept = (double)sl.cost / (D.nc > 0 ? 4.0 : 1.0);
+    return (long long)(in_range + swept / 4.0);
+}
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
@@ -3018,6 +3106,19 @@ static long long place_key(const EngineSet *s, int nfused)
            fused_dyn_bytes(s->fused_dp_ints, s->fused_bins, s->threads);
 }
 
+// Items of an engine's split step: `tile` pairs of a swept column and a moved
+// atom each, all columns without a grid and the estimated sweep with one, but
+// for moves of several atoms or few swept columns no more than about one per SM.
+static int split_tiles(const Slot &slot, int tile)
+{
+    const EDesc &D = slot.d;
+    if (D.group == 1 && D.nc == 0)
+        return std::max(1, (D.n + tile - 1) / tile);
+    // cost: columns (4 times the estimate with a grid) times atoms per move
+    const long long pairs = D.nc > 0 ? slot.cost / 4 : (long long)D.n * D.group;
+    return (int)std::max<long long>(1, std::min<long long>((pairs + tile - 1) / tile, kSplitTiles));
+}
+
 static int refresh(EngineSet *s)
 {
     if (!s->dirty)
@@ -3028,7 +3129,7 @@ static int refresh(EngineSet *s)
     s->item_count.assign(nslots, 0);
     for (int id : s->live) {
         EDesc &D = s->slots[id].d;
-        D.ntiles = std::max(1, (D.n + s->tile - 1) / s->tile);
+        D.ntiles = split_tiles(s->slots[id], s->tile);
         s->item_first[id] = (int)items.size();
         s->item_count[id] = D.ntiles;
         for (int t = 0; t < D.ntiles; ++t) items.push_back(make_int2(id, t));
@@ -3886,6 +3987,7 @@ static int add_engine(EngineSet *s, const frmc_engine_spec &sp, int *out_id)
     sl.live = true;
     sl.sq_table = sp.sq_table;
     sl.cost = (cg.nc > 0 ? 4 * (long long)std::ceil(cg.sweep) : (long long)sp.n) * spec_group(sp);
+    sl.work = solo_work(sl);
     s->slots[id] = sl;
     s->live.push_back(id);
     std::sort(s->live.begin(), s->live.end());
@@ -4250,7 +4352,9 @@ int frmc_engines_step(void *handle, int32_t engine, int32_t steps, int use_graph
         if (engine < 0)
             return launch_batched(s, sx);
         const int fi = s->fused_item[engine];
-        if (fi >= 0 && s->slots[engine].cost <= kSoloFusedCost)  // one CTA beats tiles plus a finisher
+        const Slot &solo = s->slots[engine];
+        // one CTA beats tiles plus a finisher
+        if (fi >= 0 && solo.cost <= kSoloFusedCost && (solo.d.sq || solo.work <= kSoloFusedWork))
             // one engine alone: the largest CTA (its layout fits by the fused check)
             FRMC_TRY(launch_items(s, s->items + fi, 1, 0, sx,
                                   (int)fused_dyn_bytes(s->fused_dp_ints, s->fused_bins, kMaxEngineThreads), true,
@@ -4688,6 +4792,7 @@ int frmc_engines_regrid(void *handle, int32_t e)
     D.clam2 = cg.clam2;
     D.cthr2 = cg.cthr2;
     sl.cost = (cg.nc > 0 ? 4 * (long long)std::ceil(cg.sweep) : (long long)D.n) * D.group;
+    sl.work = solo_work(sl);
     // a staged next move holds the moved atom's old cell-order slot and cell
     k_bump_gen<<<1, 1, 0, s->stream>>>(D.st);
     FRMC_CUDA(cudaGetLastError());
