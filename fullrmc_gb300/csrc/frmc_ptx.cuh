@@ -103,6 +103,14 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p)
     return v;
 }
 
+// Programmatic dependent launch: waits until the grids this one depends on have
+// completed and their writes are visible (returns at once in a plain launch).
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Lets the next grid's CTAs be placed once every CTA of this grid has said so
+// or ended.
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // 1-D bulk copy global -> shared (both 16-byte aligned, bytes % 16 == 0).
 // Hint: bring the line holding p into L2 (no register result, never faults
 // on a valid address).

@@ -1,0 +1,58 @@
+"""Steps whose kernels are placed while the kernel ahead of them still runs
+(launch_dependent, csrc/engine.cu): engines in one CTA, split over several and
+with an S(Q) term, as many as CTAs and more (items claimed by the scheduler),
+from graphs and launch by launch, give the chains of one-engine steps that
+start on an idle device, bit for bit."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+STEPS = 9
+
+
+def _systems(count):
+    from fullrmc_gb300 import synthetic
+    rng = np.random.default_rng(61)
+    mk = synthetic.make_system
+    out = [mk(rng, int(rng.integers(60, 400)), [0.6, 0.4], np.diag([16.0, 16.0, 16.0]), 6.0) for _ in range(count)]
+    out.append(mk(rng, 900, [0.5, 0.5], np.diag([20.0, 20.0, 20.0]), 8.0, q=synthetic.q_grid(0.5, 12.0, 0.1)))
+    out.append(synthetic.ring_molecules(seed=62, nmol=3200, rmax=15.0))  # split
+    return out
+
+
+def _chain(systems, how):
+    from fullrmc_gb300.engine import EngineSet, group_moves, translation_moves
+    es = EngineSet(systems, move_cap=16)
+    es.init()
+    for e, s in enumerate(systems):
+        rng = np.random.default_rng([63, e])
+        if s.group_size > 1:
+            es.push_group_moves(e, *group_moves(rng, s.groups, STEPS, 0.5, 30.0), 0)
+        else:
+            es.push_moves(e, *translation_moves(rng, s.box_coords.shape[0], STEPS, 0.8), 0)
+    if how == "idle":
+        for e in range(len(systems)):
+            for _ in range(STEPS):
+                es.step(1, engine=e, graph=False)
+                es.state(e)  # waits
+    elif how == "alone":
+        for e in range(len(systems)):
+            es.step(STEPS, engine=e)
+    else:
+        es.step(STEPS, engine=-1, graph=how == "graph")
+    out = []
+    for e in range(len(systems)):
+        c2, acc, at = es.results(e, 0, STEPS)
+        out += [c2.view(np.int64), acc, at, *es.counts(e), *es.coords(e)]
+    es.close()
+    return out
+
+
+@pytest.mark.parametrize("count", [1, 40, 330])
+def test_same_chain(count):
+    systems = _systems(count)
+    want = _chain(systems, "idle")
+    for how in ("alone", "graph", "launches"):
+        for g, w in zip(_chain(systems, how), want):
+            assert np.array_equal(g, w), how
