@@ -611,10 +611,11 @@ int walk_grid(int sms, const CellWalk &w)
 }
 
 template <int BM>
-static int launch_cell_hist_bm(const CellHist &p, int grid, size_t smem, cudaStream_t st)
+static int launch_cell_hist_bm(const CellHist &p, int grid, size_t smem, int max_smem, cudaStream_t st)
 {
     auto kern = p.s_lo > 0.0f ? k_cell_hist<BM, true> : k_cell_hist<BM, false>;
-    FRMC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // the limit, not this launch's size: another thread's launch may come between
+    FRMC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
     kern<<<grid, kCellThreads, smem, st>>>(p);
     FRMC_CUDA(cudaGetLastError());
     return FRMC_OK;
@@ -647,11 +648,11 @@ int launch_cell_hist(int sms, int max_smem_optin, const float *coords, const flo
     const size_t smem = stage + (h.smem_hist ? hist : 0);
     const int grid = walk_grid(sms, h.walk);
     switch (bm) {
-    case BM_IBC: return launch_cell_hist_bm<BM_IBC>(h, grid, smem, st);
-    case BM_DIAG: return launch_cell_hist_bm<BM_DIAG>(h, grid, smem, st);
-    case BM_XYTRI: return launch_cell_hist_bm<BM_XYTRI>(h, grid, smem, st);
-    case BM_LOWER: return launch_cell_hist_bm<BM_LOWER>(h, grid, smem, st);
-    default: return launch_cell_hist_bm<BM_GENERAL>(h, grid, smem, st);
+    case BM_IBC: return launch_cell_hist_bm<BM_IBC>(h, grid, smem, max_smem_optin, st);
+    case BM_DIAG: return launch_cell_hist_bm<BM_DIAG>(h, grid, smem, max_smem_optin, st);
+    case BM_XYTRI: return launch_cell_hist_bm<BM_XYTRI>(h, grid, smem, max_smem_optin, st);
+    case BM_LOWER: return launch_cell_hist_bm<BM_LOWER>(h, grid, smem, max_smem_optin, st);
+    default: return launch_cell_hist_bm<BM_GENERAL>(h, grid, smem, max_smem_optin, st);
     }
 }
 

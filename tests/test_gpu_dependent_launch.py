@@ -56,3 +56,37 @@ def test_same_chain(count):
     for how in ("alone", "graph", "launches"):
         for g, w in zip(_chain(systems, how), want):
             assert np.array_equal(g, w), how
+
+
+@pytest.mark.parametrize("count", [3, 305, 700])
+def test_host_steps_same_chain(count):
+    """Steps from host arrays, two in flight, each one launch that reads its
+    moves ahead of the step before: fewer and more engines than CTAs."""
+    from fullrmc_gb300 import synthetic
+    from fullrmc_gb300.engine import EngineSet, translation_moves
+    rng = np.random.default_rng(64)
+    systems = [synthetic.make_system(rng, int(rng.integers(60, 300)), [1.0], np.diag([16.0, 16.0, 16.0]), 6.0)
+               for _ in range(count)]
+    mv = [translation_moves(np.random.default_rng([65, e]), s.box_coords.shape[0], STEPS, 0.8)
+          for e, s in enumerate(systems)]
+    want = EngineSet(systems, move_cap=16)
+    want.init()
+    for e, m in enumerate(mv):
+        want.push_moves(e, *m, 0)
+    want.step(STEPS, engine=-1, graph=False)
+    es = EngineSet(systems, move_cap=16)
+    es.init()
+    got = []
+    for k in range(STEPS):
+        es.step_host_submit(*(np.stack([m[j][k] for m in mv]) for j in range(3)), k & 1)
+        if k:
+            got.append(es.step_host_collect((k - 1) & 1))
+    got.append(es.step_host_collect((STEPS - 1) & 1))
+    for e in range(count):
+        c2, acc, _ = want.results(e, 0, STEPS)
+        assert np.array_equal(c2.view(np.int64), np.array([g[0][e] for g in got]).view(np.int64))
+        assert np.array_equal(acc, [g[1][e] for g in got])
+        for g, w in zip((*es.counts(e), *es.coords(e)), (*want.counts(e), *want.coords(e))):
+            assert np.array_equal(g, w)
+    want.close()
+    es.close()
