@@ -8,16 +8,16 @@
 #include <climits>
 #include <cmath>
 #include <cstring>
+#include <unistd.h>
 #include <vector>
 
 #include "frmc_gpu.h"
 #include "frmc_runtime.h"
 
 namespace frmc {
-int launch_distances(const float *coords, int n, const float *pts, long long ps, const int *idx, int K,
-                     int fromIndex, int isPBC, const float *basis, float *out, cudaStream_t st);
-int launch_differences(const float *coords, int n, const float *pts, long long ps, const int *idx, int K,
-                       int fromIndex, int isPBC, const float *basis, float *out, cudaStream_t st);
+int launch_distances(int diff, const float *coords, int n, const float *pts, long long ps, const int *idx,
+                     const InlinePoints *few, int K, int fromIndex, int isPBC, const float *basis, float *out,
+                     cudaStream_t st);
 int launch_from_to(const float *from, const float *to, int n, int isPBC, const float *basis, float *out,
                    cudaStream_t st);
 int launch_transform(const float *M, const float *coords, int n, float *out, cudaStream_t st);
@@ -121,6 +121,27 @@ static int finish(Context *c)
 {
     FRMC_CUDA(cudaStreamSynchronize(c->stream));
     return FRMC_OK;
+}
+
+// Outputs of at most this many bytes are written to the caller's array by the
+// kernel, larger ones copied.  Up to 128 KiB malloc serves an array from its
+// heap, whose pages stay; a larger one may be mapped for itself, and to unmap a
+// page that a kernel has written costs 20 us (2.7 MB of distances, array
+// included: pages in use 43 us written by the kernel, 51 copied; mapped and
+// unmapped by each call 1,170 and 360).
+constexpr int64_t kDirectBytes = 131072;
+
+// Ahead of a kernel's writes to a caller's array: makes its pages present and
+// writable by a write of the CPU that leaves each page's bytes as they are.
+// A page that nothing has touched costs a kernel 20 us and the CPU 3.
+static void touch_pages(void *p, size_t bytes)
+{
+    static const size_t page = (size_t)std::max(4096L, sysconf(_SC_PAGESIZE));
+    if (!bytes)
+        return;
+    char *b = static_cast<char *>(p), *end = b + bytes;
+    for (; b < end; b += page) __atomic_fetch_or(b, (char)0, __ATOMIC_RELAXED);
+    __atomic_fetch_or(end - 1, (char)0, __ATOMIC_RELAXED);
 }
 
 // Upload coordinates, element and molecule indexes of n atoms.
@@ -229,15 +250,12 @@ static int prepare_counts(Context *c, int64_t total)
 static int counts_out_direct(Context *c, int64_t total, float *hintra, float *hinter)
 {
     unsigned *cnt = c->buf[BUF_COUNTS].as<unsigned>();
+    touch_pages(hintra, total * 4);
+    touch_pages(hinter, total * 4);
     TRY(launch_counts_pair_to_f32_zero(cnt, total, hintra, hinter, c->stream));
     c->counts_clean = 2 * (size_t)total * 4;
     return finish(c);
 }
-
-// Histograms of at most this many bytes are written to the caller's arrays by
-// the conversion; larger ones, which may be pages that nothing has touched yet
-// (a kernel's first write to one takes 20 us, a copy's 4), are copied.
-constexpr int64_t kDirectBytes = 65536;
 
 // Convert counts to float32 and bring both histograms back; checks the status
 // of kernels with device waits.
@@ -366,32 +384,61 @@ static int distances_common(int diff, int32_t atomIndex, const int32_t *indexes,
         return FRMC_OK;
     const float *B = isPBC ? basis : kIdentity;
     LOCKED_CTX(c);
-    TRY(upload_atoms(c, coords, nullptr, nullptr, n));
     const int width = diff ? 3 : 1;
     const int64_t out_elems = n * width * K;
+    const int fromIndex = (!points && !allAtoms) ? 1 : 0;
+    const int32_t *idx = single_index ? &atomIndex : indexes;
+    // few points go to the kernel by value
+    InlinePoints few;
+    const bool by_value = K <= kInlinePoints;
+    for (int k = 0; by_value && k < K; ++k) {
+        const float *p = idx ? coords + 3 * (int64_t)idx[k] : points + k;
+        const int64_t step = idx ? 1 : ps;
+        few.atom[k] = idx ? idx[k] : -1;
+        few.x[k] = p[0];
+        few.y[k] = p[step];
+        few.z[k] = p[2 * step];
+    }
+    float *dout = out;
+    // The kernel reads the caller's arrays where the device can, and writes a
+    // small output (a call whose output is one of its inputs needs the copies).
+    const char *o = (const char *)out, *oe = o + out_elems * 4;
+    auto apart = [&](const void *p, int64_t bytes) { return (const char *)p + bytes <= o || oe <= (const char *)p; };
+    if (c->pageable && apart(coords, n * 12) && (by_value || (idx ? apart(idx, K * 4) : apart(points, 3 * ps * 4)))) {
+        if (out_elems * 4 <= kDirectBytes) {
+            touch_pages(out, out_elems * 4);
+        } else {
+            TRY(c->buf[BUF_OUT].ensure(out_elems * 4 + 16));
+            dout = c->buf[BUF_OUT].as<float>();
+            if (fromIndex)
+                TRY(h2d(dout, out, out_elems * 4, c->stream));
+        }
+        TRY(launch_distances(diff, coords, (int)n, by_value ? nullptr : points, ps, by_value ? nullptr : idx,
+                             by_value ? &few : nullptr, (int)K, fromIndex, isPBC, B, dout, c->stream));
+        if (dout != out)
+            TRY(d2h(out, dout, out_elems * 4, c->stream));
+        return finish(c);
+    }
+    TRY(upload_atoms(c, coords, nullptr, nullptr, n));
     TRY(c->buf[BUF_OUT].ensure(out_elems * 4 + 16));
     const int *didx = nullptr;
     const float *dpts = nullptr;
-    if (single_index || indexes) {
+    if (by_value) {
+    } else if (idx) {
         TRY(c->buf[BUF_ROWS].ensure(K * 4 + 16));
-        TRY(h2d(c->buf[BUF_ROWS].p, single_index ? &atomIndex : indexes, K * 4, c->stream));
+        TRY(h2d(c->buf[BUF_ROWS].p, idx, K * 4, c->stream));
         didx = c->buf[BUF_ROWS].as<int>();
     } else {
         TRY(c->buf[BUF_AUX0].ensure(3 * ps * 4 + 16));
         TRY(h2d(c->buf[BUF_AUX0].p, points, 3 * ps * 4, c->stream));
         dpts = c->buf[BUF_AUX0].as<float>();
     }
-    const int fromIndex = (didx && !allAtoms) ? 1 : 0;
-    float *dout = c->buf[BUF_OUT].as<float>();
+    dout = c->buf[BUF_OUT].as<float>();
     // Multi-index rows below their start keep the caller's values.
     if (fromIndex && !single_index)
         TRY(h2d(dout, out, out_elems * 4, c->stream));
-    if (diff)
-        TRY(launch_differences(c->buf[BUF_COORDS].as<float>(), (int)n, dpts, ps, didx, (int)K, fromIndex, isPBC, B,
-                               dout, c->stream));
-    else
-        TRY(launch_distances(c->buf[BUF_COORDS].as<float>(), (int)n, dpts, ps, didx, (int)K, fromIndex, isPBC, B,
-                             dout, c->stream));
+    TRY(launch_distances(diff, c->buf[BUF_COORDS].as<float>(), (int)n, dpts, ps, didx, by_value ? &few : nullptr,
+                         (int)K, fromIndex, isPBC, B, dout, c->stream));
     if (fromIndex && single_index) {
         const int64_t off = (int64_t)atomIndex * width;
         TRY(d2h(out + off, dout + off, (out_elems - off) * 4, c->stream));
@@ -771,10 +818,10 @@ static int sine_common(int kind, const float *xs, int64_t nx, const float *ys, c
             TRY(sine_table_upload(c->buf[BUF_SINE_TABLE].p, c->stream));
         }
         TRY(c->buf[BUF_AUX2].ensure(sine_fixed_scratch(nx, ny)));
-        // outputs of up to 64 KiB go straight to the caller (larger ones may
-        // be pages that nothing has touched, which a kernel is slow to write)
         const bool direct = c->pageable && nx * 8 <= kDirectBytes;
         double *dout = direct ? out : c->buf[BUF_OUT].as<double>();
+        if (direct)
+            touch_pages(out, nx * 8);
         if (c->pageable)
             TRY(launch_sine_fixed(c->sms, kind, xs, (int)nx, ys, f, (int)ny, rho, scale, dout,
                                   c->buf[BUF_SINE_TABLE].p, c->buf[BUF_AUX2].p, c->stream));

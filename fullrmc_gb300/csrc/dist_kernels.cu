@@ -2,72 +2,94 @@
 // (fullrmc Extensions/pairs_distances.pyx and
 //  Extensions/boundary_conditions_collection.pyx:88-110).
 //
-// One thread per (atom i, point k).  Distances use the same squared-distance
-// arithmetic as the histogram kernels followed by an IEEE sqrt; differences
-// keep every basis term so that even signed zeros match the reference.
+// Distances use the same squared-distance arithmetic as the histogram kernels
+// followed by an IEEE sqrt; differences keep every basis term so that even
+// signed zeros match the reference.
+#include <algorithm>
+
 #include "frmc_math.cuh"
 #include "frmc_runtime.h"
 
 namespace frmc {
 
 struct PointSrc {
-    const float *pts;  // explicit points: component c of point k at pts[c*ps + k]
+    const float *pts;   // explicit points: component c of point k at pts[c*ps + k]
     long long ps;
-    const int *idx;    // or atom indexes into coords
+    const int *idx;     // or atom indexes into coords
+    InlinePoints few;   // or (neither given) at most kInlinePoints points by value
 };
 
-__device__ __forceinline__ void point_of(const PointSrc &src, const float *coords, int k, float &px, float &py,
-                                         float &pz, int &atom)
+constexpr int kDistAtoms = 256;  // threads of a block, and its largest tile of atoms
+// Outputs that a block forms: 16 a thread, so that calls of few atoms and many
+// points still fill the SMs (differences of 5,000 atoms to 70 points: tiles of
+// 256 atoms, 40 blocks, 75.7 us a call, of 21 atoms 60.4).
+constexpr int kDistOutputs = 4096;
+
+// W = 1: out[i, k] = |bc(point k - coords[i])|; W = 3: out[i, c, k] = component c
+// of the difference.
+//
+// Bound by the bytes over the host link (coordinates in, rows out; an output is
+// 4 bytes and about 25 instructions), so that each is moved once and in whole
+// lines: a block stages its atoms' coordinates and up to kInlinePoints points in
+// shared memory and writes the block's outputs in the order they are stored.  A
+// difference is formed once per component for that.  13 rows of 52,000 atoms,
+// whole call: one thread per (atom, row) between copies 65.5 us, so 36.
+template <int BM, int W>
+__global__ void __launch_bounds__(kDistAtoms) k_distances(const float *__restrict__ coords, int n,
+                                                          const __grid_constant__ PointSrc src, int tile, int K,
+                                                          int fromIndex, Basis B, float *__restrict__ out)
 {
-    if (src.idx) {
-        atom = src.idx[k];
-        px = coords[3 * (long long)atom];
-        py = coords[3 * (long long)atom + 1];
-        pz = coords[3 * (long long)atom + 2];
-    } else {
-        atom = -1;
-        px = src.pts[k];
-        py = src.pts[src.ps + k];
-        pz = src.pts[2 * src.ps + k];
+    __shared__ float sc[3 * kDistAtoms], sx[kInlinePoints], sy[kInlinePoints], sz[kInlinePoints];
+    __shared__ int sa[kInlinePoints];
+    const int i0 = blockIdx.x * tile, k0 = blockIdx.y * kInlinePoints;
+    const int na = min(tile, n - i0), kt = min(kInlinePoints, K - k0);
+    for (int e = threadIdx.x; e < 3 * na; e += kDistAtoms) sc[e] = coords[3 * (long long)i0 + e];
+    if ((int)threadIdx.x < kt) {
+        const int t = threadIdx.x, k = k0 + t;
+        if (src.idx) {
+            const int a = src.idx[k];
+            sa[t] = a;
+            sx[t] = coords[3 * (long long)a];
+            sy[t] = coords[3 * (long long)a + 1];
+            sz[t] = coords[3 * (long long)a + 2];
+        } else if (src.pts) {
+            sa[t] = -1;
+            sx[t] = src.pts[k];
+            sy[t] = src.pts[src.ps + k];
+            sz[t] = src.pts[2 * src.ps + k];
+        } else {
+            sa[t] = src.few.atom[t];
+            sx[t] = src.few.x[t];
+            sy[t] = src.few.y[t];
+            sz[t] = src.few.z[t];
+        }
     }
-}
-
-template <int BM>
-__global__ void __launch_bounds__(256) k_distances(const float *__restrict__ coords, int n, PointSrc src, int K,
-                                                   int fromIndex, Basis B, float *__restrict__ out)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int k = blockIdx.y;
-    if (i >= n)
-        return;
-    float px, py, pz;
-    int atom;
-    point_of(src, coords, k, px, py, pz, atom);
-    if (fromIndex && i < atom)
-        return;
-    float s = pair_s<BM>(px, py, pz, coords[3 * (long long)i], coords[3 * (long long)i + 1],
-                         coords[3 * (long long)i + 2], B);
-    out[(long long)i * K + k] = __fsqrt_rn(s);
-}
-
-__global__ void __launch_bounds__(256) k_differences(const float *__restrict__ coords, int n, PointSrc src, int K,
-                                                     int fromIndex, Basis B, int isPBC, float *__restrict__ out)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int k = blockIdx.y;
-    if (i >= n)
-        return;
-    float px, py, pz;
-    int atom;
-    point_of(src, coords, k, px, py, pz, atom);
-    if (fromIndex && i < atom)
-        return;
-    float ox, oy, oz;
-    pair_diff(px, py, pz, coords[3 * (long long)i], coords[3 * (long long)i + 1], coords[3 * (long long)i + 2], B,
-              isPBC, ox, oy, oz);
-    out[((long long)i * 3 + 0) * K + k] = ox;
-    out[((long long)i * 3 + 1) * K + k] = oy;
-    out[((long long)i * 3 + 2) * K + k] = oz;
+    __syncthreads();
+    // row r = W * atom + component; consecutive threads take consecutive outputs
+    const int dr = kDistAtoms / kt, dk = kDistAtoms % kt;
+    int r = threadIdx.x / kt, k = threadIdx.x % kt;
+    while (r < W * na) {
+        const int a = W == 1 ? r : r / 3;
+        if (!(fromIndex && i0 + a < sa[k])) {
+            float v;
+            if (W == 1) {
+                v = __fsqrt_rn(pair_s<BM>(sx[k], sy[k], sz[k], sc[3 * a], sc[3 * a + 1], sc[3 * a + 2], B));
+            } else {
+                float d[3];
+                pair_diff(sx[k], sy[k], sz[k], sc[3 * a], sc[3 * a + 1], sc[3 * a + 2], B, BM != BM_IBC, d[0], d[1],
+                          d[2]);
+                const int c = r - 3 * a;
+                v = c == 0 ? d[0] : c == 1 ? d[1] : d[2];
+            }
+            out[((long long)i0 * W + r) * K + k0 + k] = v;
+        }
+        r += dr;
+        k += dk;
+        if (k >= kt) {
+            k -= kt;
+            ++r;
+        }
+    }
 }
 
 // out[i] = bc(to[i] - from[i])  (pairs_distances.pyx:71-93, :113-126)
@@ -100,37 +122,32 @@ __global__ void __launch_bounds__(256) k_transform(Basis M, const float *__restr
             __fadd_rn(__fadd_rn(__fmul_rn(x, M.b[c]), __fmul_rn(y, M.b[3 + c])), __fmul_rn(z, M.b[6 + c]));
 }
 
-int launch_distances(const float *coords, int n, const float *pts, long long ps, const int *idx, int K,
-                     int fromIndex, int isPBC, const float *basis, float *out, cudaStream_t st)
+int launch_distances(int diff, const float *coords, int n, const float *pts, long long ps, const int *idx,
+                     const InlinePoints *few, int K, int fromIndex, int isPBC, const float *basis, float *out,
+                     cudaStream_t st)
 {
     if (n <= 0 || K <= 0)
         return FRMC_OK;
     if (K > 65535)
         return set_error(FRMC_E_ARG, "too many points (%d)", K);
-    PointSrc src{pts, ps, idx};
+    PointSrc src{pts, ps, idx, few ? *few : InlinePoints()};
     Basis B = make_basis(basis);
-    dim3 grid((n + 255) / 256, K);
-    switch (basis_mode(basis, isPBC)) {
-    case BM_IBC: k_distances<BM_IBC><<<grid, 256, 0, st>>>(coords, n, src, K, fromIndex, B, out); break;
-    case BM_DIAG: k_distances<BM_DIAG><<<grid, 256, 0, st>>>(coords, n, src, K, fromIndex, B, out); break;
-    case BM_XYTRI: k_distances<BM_XYTRI><<<grid, 256, 0, st>>>(coords, n, src, K, fromIndex, B, out); break;
-    case BM_LOWER: k_distances<BM_LOWER><<<grid, 256, 0, st>>>(coords, n, src, K, fromIndex, B, out); break;
-    default: k_distances<BM_GENERAL><<<grid, 256, 0, st>>>(coords, n, src, K, fromIndex, B, out); break;
-    }
-    FRMC_CUDA(cudaGetLastError());
-    return FRMC_OK;
-}
-
-int launch_differences(const float *coords, int n, const float *pts, long long ps, const int *idx, int K,
-                       int fromIndex, int isPBC, const float *basis, float *out, cudaStream_t st)
-{
-    if (n <= 0 || K <= 0)
+    const int tile = std::max(16, std::min(kDistAtoms, kDistOutputs / ((diff ? 3 : 1) * std::min(K, kInlinePoints))));
+    dim3 grid((n + tile - 1) / tile, (K + kInlinePoints - 1) / kInlinePoints);
+    if (diff) {
+        // one form for every basis: no term that is zero may be left out
+        auto kern = isPBC ? k_distances<BM_GENERAL, 3> : k_distances<BM_IBC, 3>;
+        kern<<<grid, kDistAtoms, 0, st>>>(coords, n, src, tile, K, fromIndex, B, out);
+        FRMC_CUDA(cudaGetLastError());
         return FRMC_OK;
-    if (K > 65535)
-        return set_error(FRMC_E_ARG, "too many points (%d)", K);
-    PointSrc src{pts, ps, idx};
-    dim3 grid((n + 255) / 256, K);
-    k_differences<<<grid, 256, 0, st>>>(coords, n, src, K, fromIndex, make_basis(basis), isPBC, out);
+    }
+    switch (basis_mode(basis, isPBC)) {
+    case BM_IBC: k_distances<BM_IBC, 1><<<grid, kDistAtoms, 0, st>>>(coords, n, src, tile, K, fromIndex, B, out); break;
+    case BM_DIAG: k_distances<BM_DIAG, 1><<<grid, kDistAtoms, 0, st>>>(coords, n, src, tile, K, fromIndex, B, out); break;
+    case BM_XYTRI: k_distances<BM_XYTRI, 1><<<grid, kDistAtoms, 0, st>>>(coords, n, src, tile, K, fromIndex, B, out); break;
+    case BM_LOWER: k_distances<BM_LOWER, 1><<<grid, kDistAtoms, 0, st>>>(coords, n, src, tile, K, fromIndex, B, out); break;
+    default: k_distances<BM_GENERAL, 1><<<grid, kDistAtoms, 0, st>>>(coords, n, src, tile, K, fromIndex, B, out); break;
+    }
     FRMC_CUDA(cudaGetLastError());
     return FRMC_OK;
 }

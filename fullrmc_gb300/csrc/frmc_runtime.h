@@ -100,6 +100,13 @@ Basis make_basis(const float *B);
 void sq_limits(float minD, float maxD, float *s_lo, float *s_hi);
 
 // ---------------------------------------------------------------- launchers
+// Points that a kernel takes by value (1 KB of its parameters).
+constexpr int kInlinePoints = 64;
+struct InlinePoints {
+    float x[kInlinePoints], y[kInlinePoints], z[kInlinePoints];
+    int atom[kInlinePoints];
+};
+
 struct FullTune {
     int threads = 512;  // CTA size
     int rows = 2;       // row atoms per thread (tile = threads * rows)
