@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(kCellThreads, 1) k_contacts(ContactParams p)
     int fill = 0;
     walk_blocks<BM>(
         p.walk, stage[threadIdx.x >> 5], [](const int4 &m, bool) { return m; },
-        [&](f2 s01, f2 s23, const CellRow &row, const int4 *meta, int) {
+        [&](f2 s01, f2 s23, const CellRow &row, const int4 *meta, int, auto) {
             const float s[4] = {lo2(s01), hi2(s01), lo2(s23), hi2(s23)};
             unsigned in = 0u;
 #pragma unroll

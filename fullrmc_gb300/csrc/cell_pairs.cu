@@ -32,17 +32,22 @@
 // evaluated once, in either order, and counted at [el(i)][el(j)] for the
 // original indexes i < j.
 //
-// Bound: SM issue and the FMA pipe.  Two columns at a time go through
+// Where the boxes' largest distance is below maxD (and their smallest above
+// minD) by the same margin, every pair of the two blocks is in range.
+//
+// Bound: SM issue and the FMA pipe (blocks wholly in range: issue and the
+// shared-memory pipe, 77 % of its wavefronts).  Two columns at a time go through
 // add/fma.rn.f32x2 (one issue slot for two IEEE float32 operations, at the
 // FMA pipe's scalar rate), the bin comes from an approximate quotient that is
 // checked against the distance to the next integer, and one lane in three of
 // an evaluated pair counts; per-lane queues of the counted pairs, as in
 // k_full_tiles, measured slower here (1.10 against 0.90 ms per call: the lanes
 // of a block have unequal numbers of neighbours).  Measured (whole host calls):
-// 100,000 atoms, 103 A box with gamma = 120, r 0-20 A: 6.92 -> 0.73 ms, the
-// kernel 6.81 -> 0.62 ms for 5.1e5 of 4.9e6 block pairs, 34 issue slots per
-// column of 32 rows; 11,303 atoms, r 0-12 A: 335 -> 118 us; a 100,000-atom
-// particle with every pair counted (shape function): 12.5 -> 5.3 ms.
+// 100,000 atoms, 103 A box with gamma = 120, r 0-20 A: 6.92 -> 0.71 ms, the
+// kernel 6.81 -> 0.61 ms for 5.1e5 of 4.9e6 block pairs, 34 issue slots per
+// column of 32 rows; 11,303 atoms, r 0-12 A: 335 -> 100 us; a 100,000-atom
+// particle with every pair counted (shape function): 12.5 -> 4.1 ms, 24 issue
+// slots per column (5.3 ms and 32 with each pair tested).
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -370,19 +375,23 @@ __device__ __noinline__ void bin_exact(const CellHist &p, float s, int i, int j,
 // atom per lane.  A quotient from rsqrt.approx (2^-22.9) differs from the
 // reference's by less than a known bound, so where it is further than that
 // from an integer its floor is the bin; the others (0.2 % of the pairs at
-// 2,000 bins) and pairs of one molecule go through bin_exact.  Offsets in
+// 2,000 bins) and pairs of one molecule go through bin_exact.  IN: every pair
+// is in range (but NaNs), so where all of the warp's bins hold there is nothing
+// to select.  Offsets in
 // `row` and `meta` are in bytes and count from `shaddr` and 2^23's bits.
-template <bool LO>
+template <bool LO, bool IN>
 __device__ __forceinline__ void bin_quad(const CellHist &p, const CellBins &k, f2 s01, f2 s23, const CellRow &row,
                                          const int4 *meta, int j0, unsigned *shist, f2 nz)
 {
     const float s[4] = {lo2(s01), hi2(s01), lo2(s23), hi2(s23)};
     bool in[4];
+    if (!IN) {
 #pragma unroll
-    for (int h = 0; h < 4; ++h) in[h] = (!LO || s[h] >= k.s_lo) && s[h] < k.s_hi;  // s >= 0 or NaN
-    if (!__any_sync(0xffffffffu, in[0] || in[1] || in[2] || in[3]))
-        return;
-    bool fast[4], rare = false;
+        for (int h = 0; h < 4; ++h) in[h] = (!LO || s[h] >= k.s_lo) && s[h] < k.s_hi;  // s >= 0 or NaN
+        if (!__any_sync(0xffffffffu, in[0] || in[1] || in[2] || in[3]))
+            return;
+    }
+    bool sure[4];
     unsigned at[4];
 #pragma unroll
     for (int h = 0; h < 4; h += 2) {
@@ -394,11 +403,25 @@ __device__ __forceinline__ void bin_quad(const CellHist &p, const CellBins &k, f
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
             const int4 col = meta[h + g];
-            at[h + g] = (row.meta.w < col.w ? row.meta.x + col.y : col.x + row.meta.y) +
-                        4u * __float_as_uint(g ? hi2(r) : lo2(r));
-            fast[h + g] = in[h + g] && fabsf(g ? hi2(u) : lo2(u)) < k.slack && row.meta.z != col.z;
-            rare |= in[h + g] && !fast[h + g];
+            at[h + g] = (4u * __float_as_uint(g ? hi2(r) : lo2(r)) + row.meta.y) + col.y +
+                        (row.meta.w < col.w ? row.meta.x : col.x);
+            sure[h + g] = fabsf(g ? hi2(u) : lo2(u)) < k.slack && row.meta.z != col.z;
         }
+    }
+    if (IN) {
+        if (__all_sync(0xffffffffu, sure[0] && sure[1] && sure[2] && sure[3])) {
+#pragma unroll
+            for (int h = 0; h < 4; ++h) asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(at[h]) : "memory");
+            return;
+        }
+#pragma unroll
+        for (int h = 0; h < 4; ++h) in[h] = s[h] < k.s_hi;  // not a NaN
+    }
+    bool fast[4], rare = false;
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+        fast[h] = in[h] && sure[h];
+        rare |= in[h] && !fast[h];
     }
     if (k.limit == 0u) {
         // the other lanes add to a spare counter: a predicated shared-memory
@@ -439,14 +462,15 @@ __global__ void __launch_bounds__(kCellThreads, 1) k_cell_hist(CellHist p)
     const unsigned rowbase = (shist ? smem_addr(shist) : 0u) - 4u * (kMagicBits + 1u);
     const CellBins bins(p, shist ? smem_addr(shist) : 0u);
     const f2 nz = dup2(p.walk.negzero);
-    walk_blocks<BM>(
+    walk_blocks<BM, true>(
         p.walk, reinterpret_cast<CellStage *>(smem)[tid >> 5],
         [&](const int4 &m, bool row) {
-            const unsigned base = row ? rowbase : 0u;
-            return make_int4((int)(4u * m.x + base), (int)(4u * m.y + base), m.z, m.w);
+            // (el (ne - 1) hs, el hs): a pair's offset is the sum of both
+            // second terms and the first of the atom with the smaller index
+            return make_int4(4 * (m.x - m.y), (int)(4u * m.y + (row ? rowbase : 0u)), m.z, m.w);
         },
-        [&](f2 s01, f2 s23, const CellRow &row, const int4 *meta, int j0) {
-            bin_quad<LO>(p, bins, s01, s23, row, meta, j0, shist, nz);
+        [&](f2 s01, f2 s23, const CellRow &row, const int4 *meta, int j0, auto in) {
+            bin_quad<LO, decltype(in)::value>(p, bins, s01, s23, row, meta, j0, shist, nz);
         });
     __syncthreads();
     if (shist)
@@ -646,6 +670,10 @@ int launch_cell_hist(int sms, int max_smem_optin, const float *coords, const flo
     const size_t hist = 4 * ((size_t)h.total + 33);  // + bin hs of the last row, 32 spare counters
     h.smem_hist = stage + hist <= (size_t)max_smem_optin;
     const size_t smem = stage + (h.smem_hist ? hist : 0);
+    // the walk's margins on both limits (reach0 is maxD and its own)
+    const float own = h.walk.reach0 - maxD;
+    h.walk.in0 = h.smem_hist ? maxD - own : -1.0f;
+    h.walk.from0 = h.s_lo > 0.0f ? minD + own : -1.0f;
     const int grid = walk_grid(sms, h.walk);
     switch (bm) {
     case BM_IBC: return launch_cell_hist_bm<BM_IBC>(h, grid, smem, max_smem_optin, st);

@@ -4,6 +4,7 @@
 // time.  cell_pairs.cu sorts the atoms and says what makes the test exact.
 #pragma once
 #include <cstdint>
+#include <type_traits>
 
 #include "frmc_math.cuh"
 #include "frmc_runtime.h"
@@ -35,6 +36,8 @@ struct CellWalk {
     Basis B;
     float w[3];              // perpendicular widths of the box
     float reach0, reach1;    // reach = reach0 + reach1 * max |coordinate|
+    float in0, from0;        // distances of block pairs wholly in range: past from0 + reach1 * max, up to in0 less
+                             // that (in0 < 0: none)
     float negzero;           // -0 (mul2)
 };
 
@@ -183,15 +186,18 @@ enum CellWrap : int {
 // One lane's row atom against the 32 staged columns (sorted indexes from j0).
 // CW_WRAP and CW_FAR take only the columns past `after` (a block against
 // itself: past the lane's own).
-// `quad` gets the squared distances of four columns, two and two.
-template <int BM, int WRAP, class Quad>
+// `quad` gets the squared distances of four columns, two and two, and whether
+// (IN) every pair of the blocks without a NaN is known to be in range.
+template <int BM, int WRAP, bool IN, class Quad>
 __device__ __forceinline__ void block_pairs(const CellWalk &p, const CellStage &c, const CellRow &row, const float *sh,
                                             const Basis2<BM> &B2, int j0, int after, const Quad &quad)
 {
     const f2 magic = dup2(kMagic);
     const f2 rx2 = dup2(row.x), ry2 = dup2(row.y), rz2 = dup2(row.z);
     const f2 kx = dup2(-sh[0]), ky = dup2(-sh[1]), kz = dup2(-sh[2]);
-#pragma unroll 1
+    // the short body of blocks in range pays for its loop (4.54 -> 4.10 ms of
+    // the particle's call; 2: 4.37, 8: 4.09), the longer one does not
+#pragma unroll(IN ? 4 : 1)
     for (int g = 0; g < kCellBlock; g += 4) {
         f2 s[2];
         if (WRAP != CW_FAR) {
@@ -223,7 +229,7 @@ __device__ __forceinline__ void block_pairs(const CellWalk &p, const CellStage &
 #pragma unroll
             for (int h = 0; h < 2; ++h)
                 s[h] = pack2(g + 2 * h > after ? lo2(s[h]) : INFINITY, g + 2 * h + 1 > after ? hi2(s[h]) : INFINITY);
-        quad(s[0], s[1], row, c.meta + g, j0 + g);
+        quad(s[0], s[1], row, c.meta + g, j0 + g, std::integral_constant<bool, IN>());
     }
 }
 
@@ -241,9 +247,11 @@ __device__ __forceinline__ BlockBox block_box(const float4 *bounds, int b)
     return r;
 }
 
+constexpr int kBlockIn = 4;  // or-ed to CW_NONE and CW_SHIFT where every pair is in range
+
 // The CellWrap of two blocks (`pack`: the shift of CW_SHIFT as three int8), or
 // -1 where every pair is out of range.
-template <int BM>
+template <int BM, bool INNER>
 __device__ __forceinline__ int block_test(const CellWalk &p, const BlockBox &a, const BlockBox &b, float reach,
                                           unsigned &pack)
 {
@@ -269,20 +277,30 @@ __device__ __forceinline__ int block_test(const CellWalk &p, const BlockBox &a, 
         if (!same)
             return near ? CW_WRAP : CW_FAR;
     }
-    float gap2 = 0.f;
+    float gap2 = 0.f, far2 = 0.f;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         const float t = BM == BM_IBC ? 0.f : k[0] * p.B.b[d] + k[1] * p.B.b[3 + d] + k[2] * p.B.b[6 + d];
-        const float gap = fmaxf(0.f, fmaxf(a.rlo[d] - b.rhi[d] - t, t - (a.rhi[d] - b.rlo[d])));
+        const float lo = a.rlo[d] - b.rhi[d] - t, hi = a.rhi[d] - b.rlo[d] - t;
+        const float gap = fmaxf(0.f, fmaxf(lo, -hi));
         gap2 += gap * gap;
+        if (INNER) {
+            const float far = fmaxf(-lo, hi);
+            far2 += far * far;
+        }
     }
     if (gap2 > reach * reach)
         return -1;
+    int in = 0;
+    if (INNER) {
+        const float margin = reach - p.reach0, top = p.in0 - margin, from = p.from0 + margin;
+        in = top > 0.f && far2 < top * top && (p.from0 < 0.f || gap2 > from * from) ? kBlockIn : 0;
+    }
     if (BM == BM_IBC)
-        return CW_NONE;
+        return CW_NONE | in;
     const int kx = (int)k[0], ky = (int)k[1], kz = (int)k[2];
     pack = (unsigned)(kx & 255) | (unsigned)(ky & 255) << 8 | (unsigned)(kz & 255) << 16;
-    return pack ? CW_SHIFT : CW_NONE;
+    return (pack ? CW_SHIFT : CW_NONE) | in;
 }
 
 // Column block of offset o from row block I, or -1: each unordered pair of
@@ -297,8 +315,9 @@ __device__ __forceinline__ int column_block(int I, int o, int nb)
 
 // Walks the pairs of blocks that can hold a pair within reach, a warp per
 // item (a row block and a range of offsets).  `prepare` turns an atom's meta
-// into what `quad` expects of a row (true) and of a column.
-template <int BM, class Prepare, class Quad>
+// into what `quad` expects of a row (true) and of a column.  INNER: blocks
+// wholly in range (p.in0) are told apart.
+template <int BM, bool INNER = false, class Prepare, class Quad>
 __device__ __forceinline__ void walk_blocks(const CellWalk &p, CellStage &stage, const Prepare &prepare,
                                             const Quad &quad)
 {
@@ -330,7 +349,7 @@ __device__ __forceinline__ void walk_blocks(const CellWalk &p, CellStage &stage,
             unsigned pack = 0u;
             int what = -1;
             if (mine >= 0)
-                what = block_test<BM>(p, a, block_box(p.bounds, mine), reach, pack);
+                what = block_test<BM, INNER>(p, a, block_box(p.bounds, mine), reach, pack);
             unsigned left = __ballot_sync(0xffffffffu, what >= 0);
             // the next block's columns are loaded while one is evaluated
             float nx = 0.f, ny = 0.f, nz = 0.f;
@@ -365,13 +384,17 @@ __device__ __forceinline__ void walk_blocks(const CellWalk &p, CellStage &stage,
                                      (float)(signed char)(pk >> 16 & 255u)};
                 const int after = diag ? lane : -1;
                 if (kind == CW_FAR)
-                    block_pairs<BM, CW_FAR>(p, stage, row, sh, B2, j0, after, quad);
+                    block_pairs<BM, CW_FAR, false>(p, stage, row, sh, B2, j0, after, quad);
                 else if (diag || kind == CW_WRAP)
-                    block_pairs<BM, CW_WRAP>(p, stage, row, sh, B2, j0, after, quad);
+                    block_pairs<BM, CW_WRAP, false>(p, stage, row, sh, B2, j0, after, quad);
+                else if (INNER && kind == (CW_NONE | kBlockIn))
+                    block_pairs<BM, CW_NONE, INNER>(p, stage, row, sh, B2, j0, -1, quad);
+                else if (INNER && kind == (CW_SHIFT | kBlockIn))
+                    block_pairs<BM, CW_SHIFT, INNER>(p, stage, row, sh, B2, j0, -1, quad);
                 else if (kind == CW_NONE)
-                    block_pairs<BM, CW_NONE>(p, stage, row, sh, B2, j0, -1, quad);
+                    block_pairs<BM, CW_NONE, false>(p, stage, row, sh, B2, j0, -1, quad);
                 else
-                    block_pairs<BM, CW_SHIFT>(p, stage, row, sh, B2, j0, -1, quad);
+                    block_pairs<BM, CW_SHIFT, false>(p, stage, row, sh, B2, j0, -1, quad);
             }
         }
         next = __shfl_sync(0xffffffffu, next, 0);

@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(kCellThreads, 1) k_coord_walk(CoordWalk p)
     const float s_hi = p.s_hi;
     walk_blocks<BM>(
         p.walk, stage[threadIdx.x >> 5], [](const int4 &m, bool) { return m; },
-        [&](f2 s01, f2 s23, const CellRow &row, const int4 *meta, int) {
+        [&](f2 s01, f2 s23, const CellRow &row, const int4 *meta, int, auto) {
             const float s[4] = {lo2(s01), hi2(s01), lo2(s23), hi2(s23)};
             unsigned in = 0u;
 #pragma unroll
