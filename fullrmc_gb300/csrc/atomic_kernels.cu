@@ -19,6 +19,7 @@
 #include <cstring>
 
 #include "cell_walk.cuh"
+#include "frmc_ptx.cuh"
 
 namespace frmc {
 
@@ -559,6 +560,8 @@ __device__ __forceinline__ void contact_flush(const ContactParams &p, ContactQue
 template <int BM>
 __global__ void __launch_bounds__(kCellThreads, 1) k_contacts(ContactParams p)
 {
+    grid_dependency_wait();
+    grid_launch_dependents();
     __shared__ CellStage stage[kCellThreads / 32];
     __shared__ ContactQueue queue[kCellThreads / 32];
     ContactQueue &q = queue[threadIdx.x >> 5];
@@ -604,6 +607,8 @@ __global__ void __launch_bounds__(kCellThreads, 1) k_contacts(ContactParams p)
 
 __global__ void __launch_bounds__(256) k_contact_place(ContactParams p, ListGuard guard, unsigned *strange)
 {
+    grid_dependency_wait();
+    grid_launch_dependents();
     if (blockIdx.x == 0 && threadIdx.x == 0)
         *strange = *guard.strange;  // to the host with the results
     if (guard.closed())
@@ -617,6 +622,8 @@ __global__ void __launch_bounds__(256) k_contact_place(ContactParams p, ListGuar
 
 __global__ void __launch_bounds__(256) k_contact_order(ContactParams p, ListGuard guard)
 {
+    grid_dependency_wait();
+    grid_launch_dependents();
     if (guard.closed())
         return;
     const long long len = *p.count;
@@ -681,18 +688,19 @@ int atomic_contacts_run(Context *c, const float *coords, int n, int flags, int n
         const unsigned *strange = &p.walk.sc->strange;
         const int grid = walk_grid(c->sms, p.walk);
         switch (bm) {
-        case BM_IBC: k_contacts<BM_IBC><<<grid, kCellThreads, 0, st>>>(p); break;
-        case BM_DIAG: k_contacts<BM_DIAG><<<grid, kCellThreads, 0, st>>>(p); break;
-        case BM_XYTRI: k_contacts<BM_XYTRI><<<grid, kCellThreads, 0, st>>>(p); break;
-        case BM_LOWER: k_contacts<BM_LOWER><<<grid, kCellThreads, 0, st>>>(p); break;
-        default: k_contacts<BM_GENERAL><<<grid, kCellThreads, 0, st>>>(p); break;
+        case BM_IBC: FRMC_TRY(launch_after(k_contacts<BM_IBC>, grid, kCellThreads, 0, st, p)); break;
+        case BM_DIAG: FRMC_TRY(launch_after(k_contacts<BM_DIAG>, grid, kCellThreads, 0, st, p)); break;
+        case BM_XYTRI: FRMC_TRY(launch_after(k_contacts<BM_XYTRI>, grid, kCellThreads, 0, st, p)); break;
+        case BM_LOWER: FRMC_TRY(launch_after(k_contacts<BM_LOWER>, grid, kCellThreads, 0, st, p)); break;
+        default: FRMC_TRY(launch_after(k_contacts<BM_GENERAL>, grid, kCellThreads, 0, st, p)); break;
         }
-        FRMC_CUDA(cudaGetLastError());
         FRMC_TRY(launch_cell_scan(p.row, n + 1, st));
         const ListGuard guard{p.count, p.cap, strange};
         const int g = (int)((p.cap + 255) / 256 < 4ll * c->sms ? (p.cap + 255) / 256 : 4ll * c->sms);
-        k_contact_place<<<g, 256, 0, st>>>(p, guard, block.strange());
-        k_contact_order<<<g, 256, 0, st>>>(p, guard);
+        FRMC_TRY(launch_after(k_contact_place, g, 256, 0, st, p, guard, block.strange()));
+        FRMC_TRY(launch_after(k_contact_order, g, 256, 0, st, p, guard));
+        // in full order: its few large CTAs, placed while the one ahead runs, come
+        // two to an SM (the call 229 -> 259 us)
         k_atomic_sum<<<2 * ne * ne, kSumThreads, 0, st>>>(p.list_bucket, p.list_value, p.count, guard, block.dsum(),
                                                           block.nsum());
         FRMC_CUDA(cudaGetLastError());
@@ -732,6 +740,7 @@ struct FewParams {
 template <int BM>
 __global__ void __launch_bounds__(256) k_few_rows(FewParams p)
 {
+    grid_launch_dependents();
     __shared__ float4 row[kFewRows];
     __shared__ int atom[kFewRows], mol[kFewRows];
     const AtomicParams &a = p.a;
@@ -768,6 +777,8 @@ __global__ void __launch_bounds__(256) k_few_rows(FewParams p)
 // after the other.
 __global__ void __launch_bounds__(256) k_few_sum(FewParams p, float *dsum, int *nsum)
 {
+    grid_dependency_wait();
+    grid_launch_dependents();
     __shared__ unsigned long long key[kFewHits];
     __shared__ float value[kFewHits], sorted[kFewHits];
     __shared__ int count;
@@ -832,8 +843,8 @@ int atomic_few_run(Context *c, const float *coords, const int *rows, int K, int 
     case BM_LOWER: k_few_rows<BM_LOWER><<<g, 256, 0, st>>>(p); break;
     default: k_few_rows<BM_GENERAL><<<g, 256, 0, st>>>(p); break;
     }
-    k_few_sum<<<2 * ne * ne, 256, 0, st>>>(p, block.dsum(), block.nsum());
     FRMC_CUDA(cudaGetLastError());
+    FRMC_TRY(launch_after(k_few_sum, 2 * ne * ne, 256, 0, st, p, block.dsum(), block.nsum()));
     FRMC_CUDA(cudaMemcpyAsync(results, block.p, block.results(), cudaMemcpyDeviceToHost, st));
     FRMC_CUDA(cudaStreamSynchronize(st));
     long long len;

@@ -114,6 +114,7 @@ __device__ __forceinline__ float3 cell_real(const CellSort &p, float3 c)
 // kernel went before.
 __global__ void __launch_bounds__(256) k_cell_bounds(CellSort p)
 {
+    grid_launch_dependents();
     __shared__ float tile[3 * 256];
     __shared__ unsigned red[7];
     const int tid = threadIdx.x;
@@ -214,6 +215,8 @@ __device__ __forceinline__ int cell_axis(const CellGeom &g, int k, float v)
 
 __global__ void __launch_bounds__(256) k_cell_count(CellSort p)
 {
+    grid_dependency_wait();
+    grid_launch_dependents();
     __shared__ CellGeom g;
     if (threadIdx.x == 0) {
         g = cell_geom(p);
@@ -237,6 +240,8 @@ __global__ void __launch_bounds__(256) k_cell_count(CellSort p)
 // turn; the array is zero up to the next multiple of 4,096.
 __global__ void __launch_bounds__(1024) k_cell_scan(int *cells, const CellScalars *sc, int n)
 {
+    grid_dependency_wait();
+    grid_launch_dependents();
     __shared__ int warp[2][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int turns = ((n ? n : sc->ncells) + 4095) / 4096;
@@ -280,6 +285,8 @@ __device__ __forceinline__ int cell_offset(int el, long long f)
 
 __global__ void __launch_bounds__(256) k_cell_scatter(CellSort p)
 {
+    grid_dependency_wait();
+    grid_launch_dependents();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= p.nb * kCellBlock)
         return;
@@ -309,6 +316,8 @@ __device__ __forceinline__ float warp_min(float v)
 
 __global__ void __launch_bounds__(256) k_cell_blocks(CellSort p)
 {
+    grid_dependency_wait();
+    grid_launch_dependents();
     const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (b >= p.nb)
         return;
@@ -450,6 +459,8 @@ __device__ __forceinline__ void bin_quad(const CellHist &p, const CellBins &k, f
 template <int BM, bool LO>
 __global__ void __launch_bounds__(kCellThreads, 1) k_cell_hist(CellHist p)
 {
+    grid_dependency_wait();
+    grid_launch_dependents();
     extern __shared__ __align__(128) unsigned char smem[];
     const int tid = threadIdx.x;
     unsigned *shist = nullptr;
@@ -613,19 +624,16 @@ int sort_cells(int sms, const float *coords, const float4 *atoms4, const int *el
     // scalars, cell counts and what the caller wants zero
     FRMC_CUDA(cudaMemsetAsync(scratch, 0, 256 + 4 * (size_t)kCellCap + zeroed, st));
     k_cell_bounds<<<std::min((n + 255) / 256, sms), 256, 0, st>>>(c);
-    k_cell_count<<<(n + 255) / 256, 256, 0, st>>>(c);
-    k_cell_scan<<<1, 1024, 0, st>>>(c.cells, c.sc, 0);
-    k_cell_scatter<<<(int)((np + 255) / 256), 256, 0, st>>>(c);
-    k_cell_blocks<<<(c.nb * 32 + 255) / 256, 256, 0, st>>>(c);
     FRMC_CUDA(cudaGetLastError());
-    return FRMC_OK;
+    FRMC_TRY(launch_after(k_cell_count, (n + 255) / 256, 256, 0, st, c));
+    FRMC_TRY(launch_after(k_cell_scan, 1, 1024, 0, st, c.cells, c.sc, 0));
+    FRMC_TRY(launch_after(k_cell_scatter, (int)((np + 255) / 256), 256, 0, st, c));
+    return launch_after(k_cell_blocks, (c.nb * 32 + 255) / 256, 256, 0, st, c);
 }
 
 int launch_cell_scan(int *counts, int n, cudaStream_t st)
 {
-    k_cell_scan<<<1, 1024, 0, st>>>(counts, nullptr, n);
-    FRMC_CUDA(cudaGetLastError());
-    return FRMC_OK;
+    return launch_after(k_cell_scan, 1, 1024, 0, st, counts, (CellScalars *)nullptr, n);
 }
 
 int walk_grid(int sms, const CellWalk &w)
@@ -640,9 +648,7 @@ static int launch_cell_hist_bm(const CellHist &p, int grid, size_t smem, int max
     auto kern = p.s_lo > 0.0f ? k_cell_hist<BM, true> : k_cell_hist<BM, false>;
     // the limit, not this launch's size: another thread's launch may come between
     FRMC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
-    kern<<<grid, kCellThreads, smem, st>>>(p);
-    FRMC_CUDA(cudaGetLastError());
-    return FRMC_OK;
+    return launch_after(kern, grid, kCellThreads, smem, st, p);
 }
 
 int launch_cell_hist(int sms, int max_smem_optin, const float *coords, const float4 *atoms4, const int *el,

@@ -19,6 +19,7 @@
 #include <cstring>
 
 #include "cell_walk.cuh"
+#include "frmc_ptx.cuh"
 
 namespace frmc {
 
@@ -183,6 +184,8 @@ struct CoordWalk {
 template <int BM>
 __global__ void __launch_bounds__(kCellThreads, 1) k_coord_walk(CoordWalk p)
 {
+    grid_dependency_wait();
+    grid_launch_dependents();
     __shared__ CellStage stage[kCellThreads / 32];
     __shared__ unsigned count[kCoordSlots];
     __shared__ float lower[kCoordSlots], upper[kCoordSlots];
@@ -260,11 +263,11 @@ int coordination_walk(Context *c, const float *coords, const int *row_mask, cons
                         &p.walk, st, 0, nullptr));
     const int grid = walk_grid(c->sms, p.walk);
     switch (bm) {
-    case BM_IBC: k_coord_walk<BM_IBC><<<grid, kCellThreads, 0, st>>>(p); break;
-    case BM_DIAG: k_coord_walk<BM_DIAG><<<grid, kCellThreads, 0, st>>>(p); break;
-    case BM_XYTRI: k_coord_walk<BM_XYTRI><<<grid, kCellThreads, 0, st>>>(p); break;
-    case BM_LOWER: k_coord_walk<BM_LOWER><<<grid, kCellThreads, 0, st>>>(p); break;
-    default: k_coord_walk<BM_GENERAL><<<grid, kCellThreads, 0, st>>>(p); break;
+    case BM_IBC: FRMC_TRY(launch_after(k_coord_walk<BM_IBC>, grid, kCellThreads, 0, st, p)); break;
+    case BM_DIAG: FRMC_TRY(launch_after(k_coord_walk<BM_DIAG>, grid, kCellThreads, 0, st, p)); break;
+    case BM_XYTRI: FRMC_TRY(launch_after(k_coord_walk<BM_XYTRI>, grid, kCellThreads, 0, st, p)); break;
+    case BM_LOWER: FRMC_TRY(launch_after(k_coord_walk<BM_LOWER>, grid, kCellThreads, 0, st, p)); break;
+    default: FRMC_TRY(launch_after(k_coord_walk<BM_GENERAL>, grid, kCellThreads, 0, st, p)); break;
     }
     FRMC_CUDA(cudaGetLastError());
     long long got[kCoordSlots];

@@ -3457,32 +3457,12 @@ static int refresh(EngineSet *s)
     return FRMC_OK;
 }
 
-// A launch whose CTAs may be placed before the kernel ahead of it in the stream
-// has completed; the kernel waits for that itself (grid_dependency_wait) before
-// it reads anything a step writes.  What it reads earlier (descriptors, work
-// lists, the element-pair tables) is written by the host alone, with the stream
-// drained.  Every CTA waits before it ends, so a grid ends after all that came
-// before it.  A chain of steps is bound by the gap between its launches as much
-// as by the sweep: us a step without and with the early placement, one engine of
-// 5,000 atoms 17.8 and 16.0, of 100,000 23.9 and 23.1, 24 engines with an S(Q)
-// term (two kernels a step) 52.9 and 48.5, 256 engines 25.3 and 24.3.
-template <class Params>
-static int launch_dependent(void (*kern)(Params), int grid, int threads, size_t smem, cudaStream_t st, const Params &p)
-{
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    FRMC_CUDA(cudaLaunchKernelEx(&cfg, kern, p));
-    return FRMC_OK;
-}
-
+// Successive step kernels are launched with launch_after: what they read before
+// they wait (descriptors, work lists, the element-pair tables) is written by the
+// host alone, with the stream drained.  A chain of steps is bound by the gap
+// between its launches as much as by the sweep: us a step without and with it,
+// one engine of 5,000 atoms 17.8 and 16.0, of 100,000 23.9 and 23.1, 24 engines
+// with an S(Q) term (two kernels a step) 52.9 and 48.5, 256 engines 25.3 and 24.3.
 static int launch_items(EngineSet *s, const int2 *items, int count, int eval_only, cudaStream_t st,
                         int dyn_smem = 0, bool fused = false, const EMove *hmoves = nullptr,
                         EResult *hres = nullptr, int threads = 0)
@@ -3514,9 +3494,9 @@ static int launch_items(EngineSet *s, const int2 *items, int count, int eval_onl
         // all shared memory: two CTAs of 256 threads fit one SM where their layouts do
         FRMC_CUDA(cudaFuncSetAttribute(k_engine_step<true>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                        (int)cudaSharedmemCarveoutMaxShared));
-        return launch_dependent(k_engine_step<true>, grid, threads, (size_t)dyn_smem, st, p);
+        return launch_after(k_engine_step<true>, grid, threads, (size_t)dyn_smem, st, p);
     }
-    return launch_dependent(k_engine_step<false>, grid, threads, 0, st, p);
+    return launch_after(k_engine_step<false>, grid, threads, 0, st, p);
 }
 
 // The S(Q) work list items [first, first + count): tiles, then commits.
@@ -3530,7 +3510,7 @@ static int launch_sq(EngineSet *s, int first, int count, cudaStream_t st)
     FRMC_CUDA(cudaFuncSetAttribute(k_sq_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, kSqSmemBytes));
     // one CTA per SM: it holds the SM's shared-memory ring and all of its TMEM
     const int grid = std::min(count, c->sms);
-    return launch_dependent(k_sq_fused, grid, kSqThreads, (size_t)kSqSmemBytes, st, p);
+    return launch_after(k_sq_fused, grid, kSqThreads, (size_t)kSqSmemBytes, st, p);
 }
 
 // Dynamic shared memory of a fused launch: element-pair deltas, A, Bq, the

@@ -341,6 +341,8 @@ constexpr int kRowChunk = 64;
 template <int BM>
 __global__ void __launch_bounds__(256) k_rows_vs_all(RowsParams p)
 {
+    grid_dependency_wait();
+    grid_launch_dependents();
     __shared__ float sx[kRowChunk], sy[kRowChunk], sz[kRowChunk];
     __shared__ int sa[kRowChunk], smol[kRowChunk];
     __shared__ long long srb[kRowChunk];
@@ -611,6 +613,7 @@ __global__ void __launch_bounds__(256) k_gather_atoms(const float *__restrict__ 
                                                       const int *__restrict__ mol, int n, float *__restrict__ dcoords,
                                                       int *__restrict__ del, int *__restrict__ dmol)
 {
+    grid_launch_dependents();
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i < 3 * n)
         dcoords[i] = coords[i];
@@ -761,14 +764,12 @@ int launch_rows_hist(const float *coords, const int *el, const int *mol, int n, 
     if (grid.y > 65535)
         return set_error(FRMC_E_ARG, "too many rows (%d)", K);
     switch (bm) {
-    case BM_IBC: k_rows_vs_all<BM_IBC><<<grid, 256, 0, st>>>(p); break;
-    case BM_DIAG: k_rows_vs_all<BM_DIAG><<<grid, 256, 0, st>>>(p); break;
-    case BM_XYTRI: k_rows_vs_all<BM_XYTRI><<<grid, 256, 0, st>>>(p); break;
-    case BM_LOWER: k_rows_vs_all<BM_LOWER><<<grid, 256, 0, st>>>(p); break;
-    default: k_rows_vs_all<BM_GENERAL><<<grid, 256, 0, st>>>(p); break;
+    case BM_IBC: return launch_after(k_rows_vs_all<BM_IBC>, grid, 256, 0, st, p);
+    case BM_DIAG: return launch_after(k_rows_vs_all<BM_DIAG>, grid, 256, 0, st, p);
+    case BM_XYTRI: return launch_after(k_rows_vs_all<BM_XYTRI>, grid, 256, 0, st, p);
+    case BM_LOWER: return launch_after(k_rows_vs_all<BM_LOWER>, grid, 256, 0, st, p);
+    default: return launch_after(k_rows_vs_all<BM_GENERAL>, grid, 256, 0, st, p);
     }
-    FRMC_CUDA(cudaGetLastError());
-    return FRMC_OK;
 }
 
 int launch_dists_hist(const float *dists, int n, int K, const int *rows, const int *el, const int *mol,
@@ -793,6 +794,8 @@ int launch_dists_hist(const float *dists, int n, int K, const int *rows, const i
 __global__ void k_counts_pair_to_f32_zero(unsigned *__restrict__ counts, long long total, float *__restrict__ out0,
                                           float *__restrict__ out1)
 {
+    grid_dependency_wait();
+    grid_launch_dependents();
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < 2 * total;
          k += (long long)gridDim.x * blockDim.x) {
         const unsigned c = counts[k];
@@ -813,9 +816,7 @@ int launch_counts_pair_to_f32_zero(unsigned *counts, int64_t total, float *out0,
     long long blocks = (2 * total + 255) / 256;
     if (blocks > 4096)
         blocks = 4096;
-    k_counts_pair_to_f32_zero<<<(int)blocks, 256, 0, st>>>(counts, total, out0, out1);
-    FRMC_CUDA(cudaGetLastError());
-    return FRMC_OK;
+    return launch_after(k_counts_pair_to_f32_zero, (int)blocks, 256, 0, st, counts, total, out0, out1);
 }
 
 int launch_counts_to_f32(const unsigned *counts, const float *h0, float *out, int64_t total, cudaStream_t st)

@@ -1,5 +1,5 @@
 """Steps whose kernels are placed while the kernel ahead of them still runs
-(launch_dependent, csrc/engine.cu): engines in one CTA, split over several and
+(launch_after, csrc/engine.cu): engines in one CTA, split over several and
 with an S(Q) term, as many as CTAs and more (items claimed by the scheduler),
 from graphs and launch by launch, give the chains of one-engine steps that
 start on an idle device, bit for bit."""
@@ -90,3 +90,45 @@ def test_host_steps_same_chain(count):
             assert np.array_equal(g, w)
     want.close()
     es.close()
+
+
+@pytest.mark.parametrize("n", [300, 900, 2600])
+def test_host_calls_repeat(n):
+    """Calls of several kernels, one after the other and from four threads at
+    once, give what each gives on an idle device."""
+    import threading
+    import torch
+    from fullrmc_gb300 import atomic_distances as ad
+    from fullrmc_gb300 import pairs_histograms as ph
+    rng = np.random.default_rng(n)
+    c = rng.random((n, 3)).astype(np.float32)
+    el, mol = rng.integers(0, 3, n).astype(np.int32), (np.arange(n) // 5).astype(np.int32)
+    B = np.diag([24.0, 25.0, 26.0]).astype(np.float32)
+    hist = dict(boxCoords=c, basis=B, isPBC=True, moleculeIndex=mol, elementIndex=el, numberOfElements=3,
+                minDistance=np.float32(0), maxDistance=np.float32(11.0), bin=np.float32(0.02), histSize=550)
+    near = dict(boxCoords=c, basis=B, isPBC=True, moleculeIndex=mol, elementIndex=el, numberOfElements=3,
+                lowerLimit=np.zeros((3, 3, 1), np.float32), upperLimit=np.full((3, 3, 1), 2.5, np.float32),
+                reduceDistance=True)
+    rows = np.arange(0, n, 7, dtype=np.int32)[:13]
+    calls = [lambda: ph.full_pairs_histograms_coords(**hist),
+             lambda: ph.multiple_pairs_histograms_coords(indexes=rows, allAtoms=True, **hist),
+             lambda: ad.full_atomic_distances_coords(**near)]
+    want = []
+    for f in calls:
+        torch.cuda.synchronize()
+        want.append(f())
+    bad = []
+
+    def run():
+        for k in range(30):
+            got = calls[k % 3]()
+            if not all(np.array_equal(g, w) for g, w in zip(got, want[k % 3])):
+                bad.append(k)
+
+    run()
+    threads = [threading.Thread(target=run) for _ in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
