@@ -686,14 +686,15 @@ int atomic_contacts_run(Context *c, const float *coords, int n, int flags, int n
         FRMC_TRY(sort_cells(c->sms, coords, nullptr, el, mol, n, bm, B, reach, ne, 1, c->buf[BUF_CELLS].p, &p.walk, st,
                             rows, reinterpret_cast<void **>(&p.row)));
         const unsigned *strange = &p.walk.sc->strange;
-        const int grid = walk_grid(c->sms, p.walk);
-        switch (bm) {
-        case BM_IBC: FRMC_TRY(launch_after(k_contacts<BM_IBC>, grid, kCellThreads, 0, st, p)); break;
-        case BM_DIAG: FRMC_TRY(launch_after(k_contacts<BM_DIAG>, grid, kCellThreads, 0, st, p)); break;
-        case BM_XYTRI: FRMC_TRY(launch_after(k_contacts<BM_XYTRI>, grid, kCellThreads, 0, st, p)); break;
-        case BM_LOWER: FRMC_TRY(launch_after(k_contacts<BM_LOWER>, grid, kCellThreads, 0, st, p)); break;
-        default: FRMC_TRY(launch_after(k_contacts<BM_GENERAL>, grid, kCellThreads, 0, st, p)); break;
-        }
+        FRMC_TRY(walk_lists(c->sms, p.walk, bm, st, [&](int grid) {
+            switch (bm) {
+            case BM_IBC: return launch_after(k_contacts<BM_IBC>, grid, kCellThreads, 0, st, p);
+            case BM_DIAG: return launch_after(k_contacts<BM_DIAG>, grid, kCellThreads, 0, st, p);
+            case BM_XYTRI: return launch_after(k_contacts<BM_XYTRI>, grid, kCellThreads, 0, st, p);
+            case BM_LOWER: return launch_after(k_contacts<BM_LOWER>, grid, kCellThreads, 0, st, p);
+            default: return launch_after(k_contacts<BM_GENERAL>, grid, kCellThreads, 0, st, p);
+            }
+        }));
         FRMC_TRY(launch_cell_scan(p.row, n + 1, st));
         const ListGuard guard{p.count, p.cap, strange};
         const int g = (int)((p.cap + 255) / 256 < 4ll * c->sms ? (p.cap + 255) / 256 : 4ll * c->sms);

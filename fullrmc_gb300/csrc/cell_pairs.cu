@@ -13,9 +13,9 @@
 //   k_cell_scatter  atoms to their sorted places;
 //   k_cell_blocks   bounding boxes of each block, in box coordinates and in
 //                   real space (one warp per block);
-//   k_cell_hist     block pairs: a warp holds one atom of the row block per
-//                   lane, tests 32 column blocks at once (one per lane) and
-//                   evaluates the surviving ones.
+//   k_cell_list     the pairs of blocks that can hold a pair in range;
+//   k_cell_hist     those pairs of blocks: a warp holds one atom of the row
+//                   block per lane and takes the columns in turn.
 //
 // What makes it exact: the float32 difference a - b and the reference's
 // round() are monotone, so if round() of the smallest and of the largest
@@ -43,9 +43,9 @@
 // an evaluated pair counts; per-lane queues of the counted pairs, as in
 // k_full_tiles, measured slower here (1.10 against 0.90 ms per call: the lanes
 // of a block have unequal numbers of neighbours).  Measured (whole host calls):
-// 100,000 atoms, 103 A box with gamma = 120, r 0-20 A: 6.92 -> 0.71 ms, the
-// kernel 6.81 -> 0.61 ms for 5.1e5 of 4.9e6 block pairs, 34 issue slots per
-// column of 32 rows; 11,303 atoms, r 0-12 A: 335 -> 100 us; a 100,000-atom
+// 100,000 atoms, 103 A box with gamma = 120, r 0-20 A: 6.92 -> 0.63 ms, the
+// kernel 6.81 -> 0.55 ms for 5.2e5 of 4.9e6 block pairs, 34 issue slots per
+// column of 32 rows; 11,303 atoms, r 0-12 A: 335 -> 84 us; a 100,000-atom
 // particle with every pair counted (shape function): 12.5 -> 4.1 ms, 24 issue
 // slots per column (5.3 ms and 32 with each pair tested).
 #include <algorithm>
@@ -58,6 +58,7 @@
 namespace frmc {
 
 constexpr int kCellCap = 1 << 16;     // cells at most (one CTA scans them)
+constexpr long long kCellList = 1 << 23;  // entries of a list of block pairs at most (64 MB)
 constexpr int kCellSub = 8;           // cells per block along a column
 
 struct CellSort {
@@ -339,6 +340,60 @@ __global__ void __launch_bounds__(256) k_cell_blocks(CellSort p)
     }
 }
 
+constexpr int kListThreads = 256, kListPer = 8;  // offsets a thread tests
+
+// A CTA per row block and 2,048 offsets: the pairs of blocks that can hold a
+// pair within reach, appended to the list (their order changes no count).
+// Bound by the bounds it reads (48 bytes a test, from L2): 4.9e6 tests 26 us.
+template <int BM>
+__global__ void __launch_bounds__(kListThreads) k_cell_list(CellWalk p)
+{
+    grid_dependency_wait();
+    grid_launch_dependents();
+    const int I = p.i0 + blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const float reach = p.reach0 + p.reach1 * __uint_as_float(p.sc->amax);
+    const BlockBox a = block_box(p.bounds, I);
+    const int o0 = blockIdx.y * (kListThreads * kListPer) + threadIdx.x;
+    unsigned code[kListPer], found = 0u;
+#pragma unroll
+    for (int k = 0; k < kListPer; ++k) {
+        const int o = o0 + k * kListThreads;
+        const int J = o < p.half ? column_block(I, o, p.nb) : -1;
+        unsigned pack = 0u;
+        int what = -1;
+        if (J >= 0)
+            what = block_test<BM>(p, a, block_box(p.bounds, J), reach, pack);
+        code[k] = what >= 0 ? list_code(what, pack) : ~0u;
+        found += what >= 0;
+    }
+    // places: the threads before this one, and one claim per CTA
+    __shared__ unsigned sums[kListThreads / 32], base;
+    unsigned at = found;
+#pragma unroll
+    for (int d = 1; d < 32; d *= 2) {
+        const unsigned v = __shfl_up_sync(0xffffffffu, at, d);
+        at += lane >= d ? v : 0u;
+    }
+    if (lane == 31)
+        sums[warp] = at;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned all = 0u;
+        for (int w = 0; w < kListThreads / 32; ++w) {
+            const unsigned v = sums[w];
+            sums[w] = all;
+            all += v;
+        }
+        base = all ? atomicAdd(&p.sc->listed, all) : 0u;
+    }
+    __syncthreads();
+    at += base + sums[warp] - found;
+#pragma unroll
+    for (int k = 0; k < kListPer; ++k)
+        if (code[k] != ~0u)
+            p.list[at++] = list_entry(I, o0 + k * kListThreads, code[k]);
+}
+
 __device__ __forceinline__ float rsqrt_approx(float s)
 {
     float r;
@@ -545,8 +600,8 @@ bool cell_hist_applies(long long n, int bm, const Basis &B, float minD, float ma
 
 size_t cell_hist_scratch(int n, size_t zeroed)
 {
-    const size_t np = (size_t)(n + kCellBlock - 1) / kCellBlock * kCellBlock;
-    return 256 + up256(4 * (size_t)kCellCap) + up256(zeroed) + up256(8 * (size_t)n) + 3 * up256(4 * np) +
+    const size_t nb = (size_t)(n + kCellBlock - 1) / kCellBlock, np = nb * kCellBlock, half = nb / 2 + 1;
+    return up256(8 * std::min(nb, (size_t)kCellList / half) * half) + 256 + up256(4 * (size_t)kCellCap) + up256(zeroed) + up256(8 * (size_t)n) + 3 * up256(4 * np) +
            up256(16 * np) + up256(48 * (np / kCellBlock)) + up256(16 * (size_t)n) + up256(4 * (size_t)n);
 }
 
@@ -610,16 +665,9 @@ int sort_cells(int sms, const float *coords, const float4 *atoms4, const int *el
     h.meta = c.meta;
     h.bounds = c.bounds;
     h.sc = c.sc;
-    // the row block's offsets in segments: about eight items per warp, of at
-    // most one test of 32 offsets as long as the claims stay few.  Whole calls
-    // with 2 / 4 / 8 / 14 / 24 items per warp and no such limit: 11,303 atoms
-    // 170 / 150 / 150 / 158 / 159 us, 20,000 168 / 156 / 155 / 183 / 180 us,
-    // 100,000 1,430 / 1,232 / 945 / 818 / 781 us (its 24 items are one test).
-    const int half = c.nb / 2 + 1;
-    const long long warps = (long long)sms * (kCellThreads / 32), all = (long long)c.nb * half;
-    h.segw = 1;
-    while ((h.segw < 32 && all > 16 * warps * h.segw) || all > 256 * warps * h.segw) h.segw *= 2;
-    h.nseg = (half + h.segw - 1) / h.segw;
+    h.half = c.nb / 2 + 1;
+    h.rows = (int)std::min<long long>(c.nb, kCellList / h.half);
+    h.list = reinterpret_cast<unsigned long long *>(take(8 * (size_t)h.rows * h.half));
 
     // scalars, cell counts and what the caller wants zero
     FRMC_CUDA(cudaMemsetAsync(scratch, 0, 256 + 4 * (size_t)kCellCap + zeroed, st));
@@ -636,10 +684,11 @@ int launch_cell_scan(int *counts, int n, cudaStream_t st)
     return launch_after(k_cell_scan, 1, 1024, 0, st, counts, (CellScalars *)nullptr, n);
 }
 
-int walk_grid(int sms, const CellWalk &w)
+int launch_cell_list(const CellWalk &w, int bm, cudaStream_t st)
 {
-    const long long items = (long long)w.nb * w.nseg;
-    return (int)std::min<long long>(sms, (items + kCellThreads / 32 - 1) / (kCellThreads / 32));
+    const dim3 grid(w.rows, (w.half + kListThreads * kListPer - 1) / (kListThreads * kListPer));
+    return bm == BM_IBC ? launch_after(k_cell_list<BM_IBC>, grid, kListThreads, 0, st, w)
+                        : launch_after(k_cell_list<BM_GENERAL>, grid, kListThreads, 0, st, w);
 }
 
 template <int BM>
@@ -680,14 +729,15 @@ int launch_cell_hist(int sms, int max_smem_optin, const float *coords, const flo
     const float own = h.walk.reach0 - maxD;
     h.walk.in0 = h.smem_hist ? maxD - own : -1.0f;
     h.walk.from0 = h.s_lo > 0.0f ? minD + own : -1.0f;
-    const int grid = walk_grid(sms, h.walk);
-    switch (bm) {
-    case BM_IBC: return launch_cell_hist_bm<BM_IBC>(h, grid, smem, max_smem_optin, st);
-    case BM_DIAG: return launch_cell_hist_bm<BM_DIAG>(h, grid, smem, max_smem_optin, st);
-    case BM_XYTRI: return launch_cell_hist_bm<BM_XYTRI>(h, grid, smem, max_smem_optin, st);
-    case BM_LOWER: return launch_cell_hist_bm<BM_LOWER>(h, grid, smem, max_smem_optin, st);
-    default: return launch_cell_hist_bm<BM_GENERAL>(h, grid, smem, max_smem_optin, st);
-    }
+    return walk_lists(sms, h.walk, bm, st, [&](int grid) {
+        switch (bm) {
+        case BM_IBC: return launch_cell_hist_bm<BM_IBC>(h, grid, smem, max_smem_optin, st);
+        case BM_DIAG: return launch_cell_hist_bm<BM_DIAG>(h, grid, smem, max_smem_optin, st);
+        case BM_XYTRI: return launch_cell_hist_bm<BM_XYTRI>(h, grid, smem, max_smem_optin, st);
+        case BM_LOWER: return launch_cell_hist_bm<BM_LOWER>(h, grid, smem, max_smem_optin, st);
+        default: return launch_cell_hist_bm<BM_GENERAL>(h, grid, smem, max_smem_optin, st);
+        }
+    });
 }
 
 }  // namespace frmc

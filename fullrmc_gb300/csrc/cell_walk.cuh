@@ -20,7 +20,8 @@ struct CellScalars {
     unsigned nlo[3];   // ~ordered(lo): an atomicMax from zero
     unsigned hi[3];
     unsigned amax;     // bits of max |coordinate|
-    unsigned next;     // items claimed after each warp's first
+    unsigned next;     // entries of the list claimed after each warp's first
+    unsigned listed;   // entries of the list
     int ncells;        // cells of the sort
     unsigned bad;      // an element index is outside the histogram
     unsigned strange;  // a coordinate is not finite
@@ -28,7 +29,9 @@ struct CellScalars {
 
 // What the walk over block pairs needs (walk_blocks).
 struct CellWalk {
-    int nb, nseg, segw;
+    int nb, half;            // blocks; offsets of a row block's columns: 0 .. half - 1
+    int i0, rows;            // the list holds the pairs of `rows` row blocks from i0 at a time
+    unsigned long long *list;
     const float *x, *y, *z;
     const int4 *meta;
     const float4 *bounds;
@@ -51,8 +54,25 @@ bool cell_walk_applies(long long n, int bm, const Basis &B, float reach);
 int sort_cells(int sms, const float *coords, const float4 *atoms4, const int *el, const int *mol, int n, int bm,
                const Basis &B, float reach, int ne, int hs, void *scratch, CellWalk *walk, cudaStream_t st,
                size_t zeroed, void **zero);
-// CTAs of kCellThreads for a walk.
-int walk_grid(int sms, const CellWalk &w);
+// Lists the block pairs of w.rows row blocks from w.i0 that can hold a pair
+// within reach.
+int launch_cell_list(const CellWalk &w, int bm, cudaStream_t st);
+// Runs launch(CTAs of kCellThreads) after each list of row blocks.
+template <class Launch>
+int walk_lists(int sms, CellWalk &w, int bm, cudaStream_t st, const Launch &launch)
+{
+    const int rows = w.rows;
+    const long long tests = (long long)rows * w.half;
+    const int grid = (int)(tests < sms * (kCellThreads / 32ll) ? (tests + kCellThreads / 32 - 1) / (kCellThreads / 32) : sms);
+    for (w.i0 = 0; w.i0 < w.nb; w.i0 += rows) {
+        w.rows = w.nb - w.i0 < rows ? w.nb - w.i0 : rows;
+        if (w.i0)
+            FRMC_CUDA(cudaMemsetAsync(&w.sc->next, 0, 2 * sizeof(unsigned), st));
+        FRMC_TRY(launch_cell_list(w, bm, st));
+        FRMC_TRY(launch(grid));
+    }
+    return FRMC_OK;
+}
 // Exclusive scan in place of n counts, zero up to the next multiple of 4,096.
 int launch_cell_scan(int *counts, int n, cudaStream_t st);
 
@@ -251,7 +271,7 @@ constexpr int kBlockIn = 4;  // or-ed to CW_NONE and CW_SHIFT where every pair i
 
 // The CellWrap of two blocks (`pack`: the shift of CW_SHIFT as three int8), or
 // -1 where every pair is out of range.
-template <int BM, bool INNER>
+template <int BM>
 __device__ __forceinline__ int block_test(const CellWalk &p, const BlockBox &a, const BlockBox &b, float reach,
                                           unsigned &pack)
 {
@@ -284,18 +304,13 @@ __device__ __forceinline__ int block_test(const CellWalk &p, const BlockBox &a, 
         const float lo = a.rlo[d] - b.rhi[d] - t, hi = a.rhi[d] - b.rlo[d] - t;
         const float gap = fmaxf(0.f, fmaxf(lo, -hi));
         gap2 += gap * gap;
-        if (INNER) {
-            const float far = fmaxf(-lo, hi);
-            far2 += far * far;
-        }
+        const float far = fmaxf(-lo, hi);
+        far2 += far * far;
     }
     if (gap2 > reach * reach)
         return -1;
-    int in = 0;
-    if (INNER) {
-        const float margin = reach - p.reach0, top = p.in0 - margin, from = p.from0 + margin;
-        in = top > 0.f && far2 < top * top && (p.from0 < 0.f || gap2 > from * from) ? kBlockIn : 0;
-    }
+    const float margin = reach - p.reach0, top = p.in0 - margin, from = p.from0 + margin;
+    const int in = top > 0.f && far2 < top * top && (p.from0 < 0.f || gap2 > from * from) ? kBlockIn : 0;
     if (BM == BM_IBC)
         return CW_NONE | in;
     const int kx = (int)k[0], ky = (int)k[1], kz = (int)k[2];
@@ -313,89 +328,101 @@ __device__ __forceinline__ int column_block(int I, int o, int nb)
     return J < nb ? J : J - nb;
 }
 
-// Walks the pairs of blocks that can hold a pair within reach, a warp per
-// item (a row block and a range of offsets).  `prepare` turns an atom's meta
-// into what `quad` expects of a row (true) and of a column.  INNER: blocks
-// wholly in range (p.in0) are told apart.
+// An entry of the list: row block and offset of the column block (19 bits each),
+// shift (24, of CW_SHIFT, never 0 there) and one of these.
+enum ListKind : unsigned { LK_SAME = 0, LK_IN = 1, LK_WRAP = 2, LK_FAR = 3 };
+
+__device__ __forceinline__ unsigned long long list_entry(int I, int o, unsigned code)
+{
+    return (unsigned long long)I << 45 | (unsigned long long)o << 26 | code;
+}
+__device__ __forceinline__ unsigned list_code(int what, unsigned pack)
+{
+    const unsigned kind = what == CW_FAR ? LK_FAR : what == CW_WRAP ? LK_WRAP : what & kBlockIn ? LK_IN : LK_SAME;
+    return pack << 2 | kind;
+}
+
+// Walks the listed pairs of blocks, a warp per run of entries.  `prepare` turns
+// an atom's meta into what `quad` expects of a row (true) and of a column.
+// INNER: blocks wholly in range (p.in0) are told apart.
+//
+// The list is made by a kernel of its own (k_cell_list): with the tests in the
+// walk, 32 offsets of a row block at a time, the last warps to hold a full test
+// ended 65 us after the others (100,000 atoms, 605 us), and shorter items paid
+// more for their tests than they gained (16 offsets 724 us a call, 32 692;
+// with the list 634).
 template <int BM, bool INNER = false, class Prepare, class Quad>
 __device__ __forceinline__ void walk_blocks(const CellWalk &p, CellStage &stage, const Prepare &prepare,
                                             const Quad &quad)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const Basis2<BM> B2(p.B, p.negzero);
-    const float reach = p.reach0 + p.reach1 * __uint_as_float(p.sc->amax);
-    const unsigned nitems = (unsigned)p.nb * (unsigned)p.nseg;
+    const unsigned listed = p.sc->listed;
     const unsigned nwarps = gridDim.x * (kCellThreads / 32);
+    // about 16 runs per warp, so that the last ones end together (8: 642 us a call, 16: 634)
+    const unsigned run = min(max(listed / (nwarps * 16u), 1u), 16u);
 
-    // the next item is claimed while this one is evaluated
-    unsigned next = blockIdx.x * (kCellThreads / 32) + warp;
-    while (next < nitems) {
-        const unsigned item = next;
+    // the next run is claimed while this one is evaluated
+    unsigned next = (blockIdx.x * (kCellThreads / 32) + warp) * run;
+    CellRow row;
+    int I = -1;
+    while (next < listed) {
+        const unsigned first = next, count = min(run, listed - first);
         if (lane == 0)
-            next = nwarps + atomicAdd(&p.sc->next, 1u);
-        // the nearest offsets, which hold the most pairs, first
-        const int I = (int)(item % (unsigned)p.nb), o0 = (int)(item / (unsigned)p.nb) * p.segw;
-        CellRow row;
-        {
-            const int i = row.index = I * kCellBlock + lane;
-            row.x = -p.x[i];
-            row.y = -p.y[i];
-            row.z = -p.z[i];
-            row.meta = prepare(p.meta[i], true);
-        }
-        const BlockBox a = block_box(p.bounds, I);
-        for (int o = o0; o < o0 + p.segw && 2 * o <= p.nb; o += 32) {
-            const int mine = o + lane < o0 + p.segw ? column_block(I, o + lane, p.nb) : -1;
-            unsigned pack = 0u;
-            int what = -1;
-            if (mine >= 0)
-                what = block_test<BM, INNER>(p, a, block_box(p.bounds, mine), reach, pack);
-            unsigned left = __ballot_sync(0xffffffffu, what >= 0);
-            // the next block's columns are loaded while one is evaluated
-            float nx = 0.f, ny = 0.f, nz = 0.f;
-            int4 nm = make_int4(0, 0, 0, 0);
-            int J = 0;
-            auto load = [&](unsigned m) {
-                J = __shfl_sync(0xffffffffu, mine, __ffs(m) - 1);
-                const int c = J * kCellBlock + lane;
-                nx = p.x[c];
-                ny = p.y[c];
-                nz = p.z[c];
-                nm = p.meta[c];
-            };
-            if (left)
-                load(left);
-            while (left) {
-                const int src = __ffs(left) - 1;
-                const int kind = __shfl_sync(0xffffffffu, what, src);
-                const unsigned pk = __shfl_sync(0xffffffffu, pack, src);
-                const int j0 = J * kCellBlock;
-                const bool diag = J == I;
-                __syncwarp();
-                stage.x[lane] = nx;
-                stage.y[lane] = ny;
-                stage.z[lane] = nz;
-                stage.meta[lane] = prepare(nm, false);
-                __syncwarp();
-                left &= left - 1;
-                if (left)
-                    load(left);
-                const float sh[3] = {(float)(signed char)(pk & 255u), (float)(signed char)(pk >> 8 & 255u),
-                                     (float)(signed char)(pk >> 16 & 255u)};
-                const int after = diag ? lane : -1;
-                if (kind == CW_FAR)
-                    block_pairs<BM, CW_FAR, false>(p, stage, row, sh, B2, j0, after, quad);
-                else if (diag || kind == CW_WRAP)
-                    block_pairs<BM, CW_WRAP, false>(p, stage, row, sh, B2, j0, after, quad);
-                else if (INNER && kind == (CW_NONE | kBlockIn))
-                    block_pairs<BM, CW_NONE, INNER>(p, stage, row, sh, B2, j0, -1, quad);
-                else if (INNER && kind == (CW_SHIFT | kBlockIn))
-                    block_pairs<BM, CW_SHIFT, INNER>(p, stage, row, sh, B2, j0, -1, quad);
-                else if (kind == CW_NONE)
-                    block_pairs<BM, CW_NONE, false>(p, stage, row, sh, B2, j0, -1, quad);
-                else
-                    block_pairs<BM, CW_SHIFT, false>(p, stage, row, sh, B2, j0, -1, quad);
+            next = nwarps * run + atomicAdd(&p.sc->next, run);
+        const unsigned long long mine = lane < (int)count ? p.list[first + lane] : 0ull;
+        // the next block's columns are loaded while one is evaluated
+        float nx = 0.f, ny = 0.f, nz = 0.f;
+        int4 nm = make_int4(0, 0, 0, 0);
+        int J = 0;
+        unsigned long long e = 0ull;
+        auto load = [&](unsigned k) {
+            e = __shfl_sync(0xffffffffu, mine, k);
+            J = (int)(e >> 45) + (int)(e >> 26 & 0x7ffffu);
+            J = J < p.nb ? J : J - p.nb;
+            const int c = J * kCellBlock + lane;
+            nx = p.x[c];
+            ny = p.y[c];
+            nz = p.z[c];
+            nm = p.meta[c];
+        };
+        load(0);
+        for (unsigned k = 0; k < count; ++k) {
+            const unsigned kind = (unsigned)e & 3u, pk = (unsigned)e >> 2 & 0xffffffu;
+            const int row_block = (int)(e >> 45);
+            const int j0 = J * kCellBlock;
+            if (row_block != I) {
+                I = row_block;
+                const int i = row.index = I * kCellBlock + lane;
+                row.x = -p.x[i];
+                row.y = -p.y[i];
+                row.z = -p.z[i];
+                row.meta = prepare(p.meta[i], true);
             }
+            const bool diag = J == I;
+            __syncwarp();
+            stage.x[lane] = nx;
+            stage.y[lane] = ny;
+            stage.z[lane] = nz;
+            stage.meta[lane] = prepare(nm, false);
+            __syncwarp();
+            if (k + 1 < count)
+                load(k + 1);
+            const float sh[3] = {(float)(signed char)(pk & 255u), (float)(signed char)(pk >> 8 & 255u),
+                                 (float)(signed char)(pk >> 16 & 255u)};
+            const int after = diag ? lane : -1;
+            if (kind == LK_FAR)
+                block_pairs<BM, CW_FAR, false>(p, stage, row, sh, B2, j0, after, quad);
+            else if (diag || kind == LK_WRAP)
+                block_pairs<BM, CW_WRAP, false>(p, stage, row, sh, B2, j0, after, quad);
+            else if (INNER && kind == LK_IN && !pk)
+                block_pairs<BM, CW_NONE, INNER>(p, stage, row, sh, B2, j0, -1, quad);
+            else if (INNER && kind == LK_IN)
+                block_pairs<BM, CW_SHIFT, INNER>(p, stage, row, sh, B2, j0, -1, quad);
+            else if (!pk)
+                block_pairs<BM, CW_NONE, false>(p, stage, row, sh, B2, j0, -1, quad);
+            else
+                block_pairs<BM, CW_SHIFT, false>(p, stage, row, sh, B2, j0, -1, quad);
         }
         next = __shfl_sync(0xffffffffu, next, 0);
     }

@@ -261,14 +261,15 @@ int coordination_walk(Context *c, const float *coords, const int *row_mask, cons
     FRMC_CUDA(cudaMemcpyAsync(p.totals, block, sizeof(block), cudaMemcpyHostToDevice, st));
     FRMC_TRY(sort_cells(c->sms, coords, nullptr, row_mask, member_mask, n, bm, B, reach, 1, 1, c->buf[BUF_CELLS].p,
                         &p.walk, st, 0, nullptr));
-    const int grid = walk_grid(c->sms, p.walk);
-    switch (bm) {
-    case BM_IBC: FRMC_TRY(launch_after(k_coord_walk<BM_IBC>, grid, kCellThreads, 0, st, p)); break;
-    case BM_DIAG: FRMC_TRY(launch_after(k_coord_walk<BM_DIAG>, grid, kCellThreads, 0, st, p)); break;
-    case BM_XYTRI: FRMC_TRY(launch_after(k_coord_walk<BM_XYTRI>, grid, kCellThreads, 0, st, p)); break;
-    case BM_LOWER: FRMC_TRY(launch_after(k_coord_walk<BM_LOWER>, grid, kCellThreads, 0, st, p)); break;
-    default: FRMC_TRY(launch_after(k_coord_walk<BM_GENERAL>, grid, kCellThreads, 0, st, p)); break;
-    }
+    FRMC_TRY(walk_lists(c->sms, p.walk, bm, st, [&](int grid) {
+        switch (bm) {
+        case BM_IBC: return launch_after(k_coord_walk<BM_IBC>, grid, kCellThreads, 0, st, p);
+        case BM_DIAG: return launch_after(k_coord_walk<BM_DIAG>, grid, kCellThreads, 0, st, p);
+        case BM_XYTRI: return launch_after(k_coord_walk<BM_XYTRI>, grid, kCellThreads, 0, st, p);
+        case BM_LOWER: return launch_after(k_coord_walk<BM_LOWER>, grid, kCellThreads, 0, st, p);
+        default: return launch_after(k_coord_walk<BM_GENERAL>, grid, kCellThreads, 0, st, p);
+        }
+    }));
     FRMC_CUDA(cudaGetLastError());
     long long got[kCoordSlots];
     unsigned odd = 0;
