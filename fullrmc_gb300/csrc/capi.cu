@@ -296,7 +296,7 @@ static int counts_out(Context *c, int64_t total, const float *h0intra, const flo
 // Host-buffer calls with at most this many rows read the caller's arrays
 // directly where the device accesses pageable memory: the row kernel reads
 // every column once per 64 rows, so up to 64 rows read no more than a copy.
-constexpr int64_t kDirectRows = 64;
+constexpr int64_t kDirectRows = kInlineRows;
 
 }  // namespace frmc
 
@@ -661,10 +661,20 @@ int frmc_multiple_pairs_histograms_coords(const int32_t *indexes, int64_t K, con
     unsigned *cnt = c->buf[BUF_COUNTS].as<unsigned>();
     if (direct) {
         // the per-move call (fullrmc's moved atoms, PairDistributionConstraints.py:1016-1026):
-        // the kernels read the caller's arrays and write its histograms in place
-        TRY(launch_rows_hist(boxCoords, elementIndex, moleculeIndex, (int)n, indexes, (int)K, allAtoms,
+        // the kernels take the rows by value, read the caller's arrays and write
+        // its histograms in place
+        InlineRows few;
+        for (int k = 0; k < K; ++k) {
+            const int a = few.atom[k] = indexes[k];
+            few.x[k] = boxCoords[3 * (int64_t)a];
+            few.y[k] = boxCoords[3 * (int64_t)a + 1];
+            few.z[k] = boxCoords[3 * (int64_t)a + 2];
+            few.mol[k] = moleculeIndex[a];
+            few.el[k] = elementIndex[a];
+        }
+        TRY(launch_rows_hist(boxCoords, elementIndex, moleculeIndex, (int)n, nullptr, (int)K, allAtoms,
                              basis_mode(B, isPBC), make_basis(B), minDistance, maxDistance, bin, ne, hs, cnt,
-                             cnt + total, c->stream));
+                             cnt + total, c->stream, &few));
         return counts_out_direct(c, total, hintra, hinter);
     }
     TRY(upload_atoms(c, boxCoords, moleculeIndex, elementIndex, n));

@@ -132,6 +132,13 @@ struct InlinePoints {
     int atom[kInlinePoints];
 };
 
+// Rows (atoms of the system) that a kernel takes by value.
+constexpr int kInlineRows = 64;
+struct InlineRows {
+    float x[kInlineRows], y[kInlineRows], z[kInlineRows];
+    int atom[kInlineRows], mol[kInlineRows], el[kInlineRows];
+};
+
 struct FullTune {
     int threads = 512;  // CTA size
     int rows = 2;       // row atoms per thread (tile = threads * rows)
@@ -183,11 +190,12 @@ int launch_cell_hist(int sms, int max_smem_optin, const float *coords, const flo
                      const int *mol, int n, int bm, const Basis &B, float minD, float maxD, float binw, int ne, int hs,
                      unsigned *intra, unsigned *inter, void *scratch, cudaStream_t st);
 
-// Rows (explicit atom indexes, or explicit coordinates) against every column
-// atom j in [start, n), j != row atom.  Counts are added with global atomics.
+// Rows (atom indexes, null: every atom in order, or at most kInlineRows by value)
+// against every column atom j != row atom, or j > row atom without allAtoms.
+// Counts are added with global atomics.
 int launch_rows_hist(const float *coords, const int *el, const int *mol, int n, const int *rows, int K,
                      int allAtoms, int bm, const Basis &B, float minD, float maxD, float binw, int ne, int hs,
-                     unsigned *intra, unsigned *inter, cudaStream_t st);
+                     unsigned *intra, unsigned *inter, cudaStream_t st, const InlineRows *few = nullptr);
 
 // A group move's change of fullrmc's before/after-move data (M - F after
 // minus M - F before) into signed counts; rows in group order, sorted = the
