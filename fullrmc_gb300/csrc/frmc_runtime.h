@@ -245,9 +245,10 @@ struct AtomicBlock {
 // that bound the distance, by the walk over sorted atoms, from the caller's
 // arrays.  The results come back in `results` (AtomicBlock::results() bytes);
 // *done is 0, and the block's sums are as they were, where it does not apply.
-// Synchronises `st`.  From kMinPairsContacts pairs (1,800 atoms): whole calls of
-// 1,040 / 2,080 / 5,200 atoms took 142 / 143 / 157 us by the walk and 128 / 151 /
-// 276 us by two passes over all pairs.
+// Synchronises `st`.  From kMinPairsContacts pairs (900 atoms): whole calls of
+// 845 / 1,040 / 1,690 / 5,200 atoms take 108 / 108 / 112 / 130 us by the walk and
+// 109 / 122 / 124 / 250 us by two passes over all pairs; fewer atoms are not
+// worth a sort.
 int atomic_contacts_run(Context *c, const float *coords, int n, int flags, int ne, const float *basis_host, int isPBC,
                         const int *mol, const int *el, const float *lower_host, const float *upper_host,
                         const AtomicBlock &block, unsigned char *results, int *done, cudaStream_t st);
@@ -257,7 +258,7 @@ constexpr int kFewRows = 64;
 int atomic_few_run(Context *c, const float *coords, const int *rows, int K, int n, int allAtoms, int flags, int ne,
                    const float *basis_host, int isPBC, const int *mol, const int *el, const AtomicBlock &block,
                    unsigned char *results, int *done, cudaStream_t st);
-constexpr double kMinPairsContacts = 1.6e6;
+constexpr double kMinPairsContacts = 4e5;
 // pair_elements_stats counts ([2][ne][ne] int, zeroed by the caller).
 int launch_pair_stats(const int *el, const int *mol, int n, int ne, int *nintra, int *ninter, cudaStream_t st);
 
