@@ -1,8 +1,8 @@
 // extern "C" entry points (declared in include/frmc_gpu.h).
 //
-// Host-buffer entry points copy their inputs to the current device on the
-// context's stream, run the kernels, copy the results back and synchronise;
-// they keep no host data between calls (fullrmc mutates its coordinate array
+// Host-buffer entry points run on the context's stream from the caller's arrays
+// (read by the kernels where the device can, else copied), bring the results
+// back and synchronise; they keep no host data between calls (fullrmc mutates its coordinate array
 // between calls, PairDistributionConstraints.py:1092-1122).
 #include <algorithm>
 #include <climits>
@@ -189,8 +189,11 @@ static int full_counts(Context *c, const float *coords, const int32_t *mol, cons
     Basis Bs = make_basis(B);
     const double pairs = 0.5 * (double)n * (double)(n - 1);
     FullTune tn = current_tune();
+    // pairs in range per element pair (a free system's are not known)
+    const double hits = isPBC ? pairs * accept_fraction(B, isPBC, minD, maxD) / ((double)ne * ne) : 0.0;
     // a tile configuration set by the caller keeps the tiled kernel
-    if (tn == FullTune() && pairs >= kMinPairsCells && cell_hist_applies(n, bm, Bs, minD, maxD, bin, ne, hs)) {
+    if (tn == FullTune() && (pairs >= kMinPairsCells || hits >= kMinHitsCells) &&
+        cell_hist_applies(n, bm, Bs, minD, maxD, bin, ne, hs)) {
         TRY(c->buf[BUF_CELLS].ensure(cell_hist_scratch((int)n)));
         TRY(device_atoms(c, n, &coords, &mol, &el));
         return launch_cell_hist(c->sms, c->max_smem_optin, coords, nullptr, el, mol, (int)n, bm, Bs, minD, maxD, bin,

@@ -177,13 +177,17 @@ long long full_hist_items(int n, const FullTune *tune);
 
 // The same histogram over spatially sorted atoms (cell_pairs.cu): block pairs
 // out of range are skipped.  Atoms as AoS coordinates with element indexes (in
-// device memory, or host memory that the device reads) or packed (atoms4); `scratch` holds cell_hist_scratch(n) bytes of device memory
-// that nothing else uses until the work on `st` is done.  From kMinPairsCells
-// pairs (2,450 atoms) the sort pays for itself: whole calls of 2,000 / 3,000 /
-// 3,990 atoms by the row kernel took 40 / 49 / 59 us at r 8 A, 64 / 93 / 110 us
-// at 15 A and 83 / 120 / 166 us at 20 A; sorted, 2,460 / 3,000 / 4,100 atoms take
-// 54 / 55 / 58, 55 / 61 / 65 and 78 / 80 / 84 us.
-constexpr double kMinPairsCells = 3.0e6;
+// device memory, or host memory that the device reads) or packed (atoms4);
+// `scratch` holds cell_hist_scratch(n) bytes of device memory that nothing else
+// uses until the work on `st` is done.  The sort and the list make a call of
+// 600 to 2,400 atoms 40 to 47 us whatever is in range.  The row kernel's takes
+// 32 to 36 us up to 1,600 atoms and grows with the pairs (45 to 50 us at 2,400
+// atoms, r 10-12 A, 2 and 4 elements: from kMinPairsCells pairs, 2,240 atoms, the
+// sort pays) and with its atomics on few counters (one element, r 20 A, every
+// pair in range: 40 / 55 / 83 / 122 / 237 us at 600 / 900 / 1,200 / 1,600 / 2,400
+// atoms: so does it from kMinHitsCells pairs in range per element pair).
+constexpr double kMinHitsCells = 1.5e5;
+constexpr double kMinPairsCells = 2.5e6;
 bool cell_hist_applies(long long n, int bm, const Basis &B, float minD, float maxD, float binw, int ne, int hs);
 size_t cell_hist_scratch(int n, size_t zeroed = 0);
 int launch_cell_hist(int sms, int max_smem_optin, const float *coords, const float4 *atoms4, const int *el,
