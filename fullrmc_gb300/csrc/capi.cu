@@ -2,8 +2,8 @@
 //
 // Host-buffer entry points run on the context's stream from the caller's arrays
 // (read by the kernels where the device can, else copied), bring the results
-// back and synchronise; they keep no host data between calls (fullrmc mutates its coordinate array
-// between calls, PairDistributionConstraints.py:1092-1122).
+// back and synchronise; they keep no host data between calls (fullrmc mutates
+// its coordinate array between calls, PairDistributionConstraints.py:1092-1122).
 #include <algorithm>
 #include <climits>
 #include <cmath>

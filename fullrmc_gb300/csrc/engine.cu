@@ -19,12 +19,13 @@
 // moves, a ring of step results and the chain state.  A descriptor array
 // holds each engine's pointers and constants.
 //
-// The step kernel walks a work list of (engine, atom tile) items; persistent
-// CTAs claim items from an atomic counter (the last CTA to leave resets it).
-// Each item adds +-1 to its engine's oriented delta, to its element-pair delta
-// and to a touched list with global atomics; the CTA that completes an
-// engine's last item (threadfence + counter, no waiting) then evaluates,
-// decides and commits that engine while the other CTAs keep claiming items.
+// The step kernel walks a work list of whole engines (one CTA each) or of
+// (engine, share of the swept columns) items; CTAs take an item each, or claim
+// them from an atomic counter (the last CTA to leave resets it).  An item of a
+// split step adds +-1 to its engine's oriented delta and element-pair delta
+// with global atomics; the CTA that completes an engine's last item
+// (threadfence + counter, no waiting) then evaluates, decides and commits that
+// engine while the other CTAs go on.
 // The FP64 evaluation is incremental: G(r) of the current configuration is
 // kept, and only bins whose element-pair counts changed do FP64 work.
 // Nothing spins, so the kernel cannot hang; a chain's arithmetic depends only
