@@ -432,6 +432,43 @@ __device__ void commit_moved_group(const EDesc &D, const MovedGroup &g, const fl
     }
 }
 
+// The same after a split step.  Atoms of a group may share a cell: the
+// thread of the first of them widens it for all, so that the cells' bounds are
+// read side by side (one thread for all atoms took a round trip to L2 for each:
+// 13 atoms among 52,000, about half of the moves accepted, 31.3 us a step, so
+// 30.8; one atom of 14,000 in a split step 20.3, with the state kept from set-up 19.7).
+// (The one-CTA step keeps the form above: 256 engines 424 us for 16 steps with
+// this one, 419 with that.)
+__device__ void commit_split_group(const EDesc &D, const MovedGroup &g)
+{
+    for (int t = threadIdx.x; t < g.n; t += blockDim.x) {
+        const int a = g.atom[t];
+        const float4 nb = make_float4(g.nw[t][0], g.nw[t][1], g.nw[t][2], __int_as_float(g.el[t]));
+        D.box[a] = nb;
+        D.real[a] = make_float4(g.nr[t][0], g.nr[t][1], g.nr[t][2], 0.0f);
+        if (D.nc > 0) {
+            D.cbox[g.slot[t]] = nb;
+            const int c = g.cell[t];
+            bool first = true;
+            for (int q = 0; q < t; ++q) first = first && g.cell[q] != c;
+            if (first) {
+                float4 lo = D.clo[c], hi = D.chi[c];
+                for (int q = t; q < g.n; ++q)
+                    if (g.cell[q] == c) {
+                        lo.x = fminf(lo.x, g.nw[q][0]);
+                        lo.y = fminf(lo.y, g.nw[q][1]);
+                        lo.z = fminf(lo.z, g.nw[q][2]);
+                        hi.x = fmaxf(hi.x, g.nw[q][0]);
+                        hi.y = fmaxf(hi.y, g.nw[q][1]);
+                        hi.z = fmaxf(hi.z, g.nw[q][2]);
+                    }
+                D.clo[c] = lo;
+                D.chi[c] = hi;
+            }
+        }
+    }
+}
+
 // Element-pair index and bin of an oriented flat index.  A count past the
 // last bin lands in bin 0.. of the next oriented row of the C-contiguous
 // array, as with the reference's unchecked index.
@@ -1118,17 +1155,18 @@ __device__ void finish_engine(const EDesc &D, const MovedGroup &g, double *red, 
         }
         return;
     }
-    const EState &S0 = *D.st;
+    // the state and the move's uniform number were read at set-up
     double sd_new = 0.0, chi2_new = 0.0;  // thread 0's
     if (threadIdx.x == 0) {
-        sd_new = D.dense ? sd_dense : S0.sd + dsd;
+        sd_new = D.dense ? sd_dense : g.sd + dsd;
         chi2_new = sd_new / D.var2;
-        const EMove &m = D.moves[S0.step % D.move_cap];
-        const bool reject = (chi2_new > S0.chi2) && (m.u > D.tol);
+        const bool reject = (chi2_new > g.chi2) && (g.u > D.tol);
         *s_flag = reject ? 0 : 1;
     }
     __syncthreads();
     const bool accept = *s_flag != 0;
+    if (accept)
+        commit_split_group(D, g);  // its loads go beside the counts'
     // commit (or drop) the oriented delta: the whole array once, in order and
     // with kCommitUnroll quads in flight per thread (a group move of 13 atoms
     // touches 36,000 entries of its 27,000 bins; through a list each took a
@@ -1180,26 +1218,23 @@ __device__ void finish_engine(const EDesc &D, const MovedGroup &g, double *red, 
             }
         }
     }
-    if (accept) {
-        commit_moved_group(D, g);
-        if (D.dense)
-            dense_commit(D);
-    }
+    if (accept && D.dense)
+        dense_commit(D);
     __syncthreads();
     if (threadIdx.x == 0) {
         EState &S = *D.st;
-        EResult &r = D.results[S.step % D.move_cap];
+        EResult &r = D.results[g.step % D.move_cap];
         r.chi2_new = chi2_new;
         r.accepted = accept ? 1 : 0;
         r.atom = g.atom[0];
         if (accept) {
             S.chi2 = chi2_new;
             S.sd = sd_new;
-            S.accepted += 1;
+            S.accepted = g.accepted + 1;
             if (D.dense)
                 S.sf = s_sf;
         }
-        S.step += 1;
+        S.step = g.step + 1;
         S.done = 0u;
         S.tcount = 0u;
     }
