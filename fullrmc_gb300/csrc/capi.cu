@@ -24,7 +24,7 @@ int launch_transform(const float *M, const float *coords, int n, float *out, cud
 int launch_sine(int kind, const float *xs, int nx, const float *ys, const float *f, int ny, double rho, double *out,
                 double *scratch, cudaStream_t st);
 
-bool sine_fixed_scale(const float *xs, int64_t nx, const float *ys, const float *f, int64_t ny, int *scale);
+bool sine_fixed_scale(int kind, const float *xs, int64_t nx, const float *ys, const float *f, int64_t ny, int *scale);
 size_t sine_fixed_scratch(int64_t nx, int64_t ny);
 size_t sine_table_bytes();
 int sine_table_upload(void *table, cudaStream_t st);
@@ -819,7 +819,7 @@ static int sine_common(int kind, const float *xs, int64_t nx, const float *ys, c
     float *dys = c->buf[BUF_AUX1].as<float>();
     float *df = dys + ny;
     int scale = 0;
-    const bool fixed = sine_fixed_scale(xs, nx, ys, f, ny, &scale);
+    const bool fixed = sine_fixed_scale(kind, xs, nx, ys, f, ny, &scale);
     if (!(fixed && c->pageable)) {
         TRY(h2d(dxs, xs, nx * 4, c->stream));
         TRY(h2d(dys, ys, ny * 4, c->stream));

@@ -206,15 +206,18 @@ static void sine_table(SineTable *t)
 }
 
 // The scale of a summation grid: the smallest e with every y 2^e an integer,
-// below 2^37.  False for grids, values and output grids that the fixed-point
-// sines do not take (host arrays).
-bool sine_fixed_scale(const float *xs, int64_t nx, const float *ys, const float *f, int64_t ny, int *scale)
+// below 2^37.  False for grids, weights and output grids that the fixed-point
+// sines do not take (host arrays): the sines' last line is summed with float32
+// weights, so a weight and any sum of weights has to be finite there.
+bool sine_fixed_scale(int kind, const float *xs, int64_t nx, const float *ys, const float *f, int64_t ny, int *scale)
 {
     int e = -200, top = -200;
     float ymax = 0.0f;
+    const double dy = (double)ys[1] - (double)ys[0];
     for (int64_t i = 0; i < ny; ++i) {
         const float y = ys[i];
-        if (!(y >= 0.0f && y < 1e30f) || !(std::fabs(f[i]) < 1e30f))
+        const double w = kind == SK_BIGGR_TO_SQ ? dy * f[i] : dy * y * ((double)f[i] - 1.0);
+        if (!(y >= 0.0f && y < 1e30f) || !(std::fabs(f[i]) < 1e30f) || !(std::fabs(w) < 1e28))
             return false;
         if (y == 0.0f)
             continue;
