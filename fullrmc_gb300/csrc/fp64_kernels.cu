@@ -16,9 +16,10 @@
 // warp's instruction).  sin() costs about 30 FP64 instructions a term; the
 // grids of the transforms let four do (k_sine_fixed).  k_sine_rows, one CTA per
 // output point with sin(), takes the grids that do not.  Whole calls, r 0-20 A
-// by 0.01 to Q 0.5-30 by 0.01 (5.9e6 terms): 281 -> 93 us, the kernel 243 -> 60
-// us.  Against 128-bit sums over six grids of the declared range both are off by
-// the same 8.8e-17 to 1.2e-16 of the result (ratio 0.96 to 1.02, mean 0.99).
+// by 0.01 to Q 0.5-30 by 0.01 (5.9e6 terms): 278 -> 93.5 us.  Rms error against
+// 80-bit sums, over 21 grids (500-2,000 r by 0.01, 450-2,950 Q, three transforms):
+// 0.86 to 1.16 of k_sine_rows', mean 0.997; over each call's 20 smallest
+// arguments 0.91.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -124,15 +125,26 @@ __global__ void k_sine_prep(int kind, const float *__restrict__ xs, int nx, cons
 // product of a float's integer with as many bits of 1 / (2 pi) as it needs).
 // The phase X Y modulo 1 is then a few integer multiply-adds, exact to 2^-59 of
 // a turn, and the integer pipes are thirty times as wide as the FP64 pipe.  Its
-// top 11 bits name one of 2,048 arcs, the others the place r in [-1/2, 1/2) of
-// its arc, and with h = 2 pi / 2048
+// top 12 bits name one of 4,096 arcs, the others the place r in [-1/2, 1/2) of
+// its arc, and with h = 2 pi / 4096
 //   sin = T0 + T1 r + T2 r^2  (FP64: sin, h cos, -h^2/2 sin of the arc's centre)
 //       + (T0's rounding - h^3/6 cos r^3 + h^4/24 sin r^4)   (float32),
-// the last line below 1e-9 and so good to 1e-16 in float32, the next term of
-// the series below 7e-17.  Four FP64 instructions a term: r, two for the
-// polynomial, one for the weighted sum.
-constexpr int kArcs = 2048;
-constexpr int kSineThreads = 512;
+// the last line below 1.6e-10 and so good to 5e-18 in float32, the next term of
+// the series below 2.3e-18 (with 2,048 arcs 7e-17, as large as a sine's own
+// rounding).  Four FP64 instructions a term: r, two for the polynomial, one for
+// the weighted sum.
+//
+// The last line's sum over a lane's terms is formed first and the FP64 sum starts
+// from it, so that it costs no rounding of its own: added at the end it made the
+// error 3 to 9 % larger.  (The integer and float32 pipes have the room to form the
+// phases twice; all this, the second half of the table and the check below take
+// 2 to 3 us of a call, 91.0 -> 93.5 us at 5.9e6 terms, 38.5 -> 40.5 at 3.5e5.)  What is left is an absolute error of a sine, where sin() has a
+// relative one, so an output whose sines are small throughout -- sum |w| t below
+// 1/32 sum |w|, with t = 2 / pi asin |sin| -- is summed again with sin(), or
+// where an argument is small its series.
+constexpr int kArcs = 4096;
+constexpr float kSineSmall = 1.0f / 32;  // rms error over sin()'s: above it 0.91 to 1.06, at 1/64 1.2, at 1/150 1.6
+constexpr int kSineThreads = 384;  // 512 and 768: 0.5 and 2 us more a call of 5.9e6 terms
 constexpr int kSineWarps = kSineThreads / 32;
 constexpr int kSineParts = 4;    // parts of an output point's sum, a warp each
 constexpr int kSineBatch = 64;   // output points of a CTA between two barriers
@@ -177,7 +189,7 @@ static void sine_table(SineTable *t)
     const unsigned __int128 pi = (unsigned __int128)0x3243f6a8885a3ull << 64 | 0x08d313198a2e0370ull;
     const double h = 2.0 * M_PI / kArcs;
     for (int k = 0; k < kArcs / 4; ++k) {
-        const unsigned __int128 x = pi * (2 * k + 1) >> 11;  // the centre's angle in the first quadrant
+        const unsigned __int128 x = pi * (2 * k + 1) >> 12;  // the centre's angle in the first quadrant
         const unsigned __int128 x2 = fixed_mul(x, x);
         // cos above 1/2 and below: 1 - x^2/2 + ...; the terms fall below 2^-112
         unsigned __int128 one = (unsigned __int128)1 << 112, sn = x, cs = one, ts = x, tc = one;
@@ -208,17 +220,20 @@ static void sine_table(SineTable *t)
 // The scale of a summation grid: the smallest e with every y 2^e an integer,
 // below 2^37.  False for grids, weights and output grids that the fixed-point
 // sines do not take (host arrays): the sines' last line is summed with float32
-// weights, so a weight and any sum of weights has to be finite there.
+// weights, so a weight and any sum of weights has to be finite there and the
+// largest far from its smallest numbers.
 bool sine_fixed_scale(int kind, const float *xs, int64_t nx, const float *ys, const float *f, int64_t ny, int *scale)
 {
     int e = -200, top = -200;
     float ymax = 0.0f;
+    double wmax = 0.0;
     const double dy = (double)ys[1] - (double)ys[0];
     for (int64_t i = 0; i < ny; ++i) {
         const float y = ys[i];
         const double w = kind == SK_BIGGR_TO_SQ ? dy * f[i] : dy * y * ((double)f[i] - 1.0);
         if (!(y >= 0.0f && y < 1e30f) || !(std::fabs(f[i]) < 1e30f) || !(std::fabs(w) < 1e28))
             return false;
+        wmax = std::max(wmax, std::fabs(w));
         if (y == 0.0f)
             continue;
         uint32_t u;
@@ -229,22 +244,17 @@ bool sine_fixed_scale(int kind, const float *xs, int64_t nx, const float *ys, co
             m |= 0x800000u;
         else
             ex = 1;
-        int low = ex - 150;  // y = m 2^low
-        while (!(m & 1u)) {
-            m >>= 1;
-            ++low;
-        }
-        e = std::max(e, -low);
+        e = std::max(e, 150 - ex - __builtin_ctz(m));  // y = m 2^(ex - 150)
         ymax = std::max(ymax, y);
     }
-    if (!(ymax > 0.0f))
+    if (!(ymax > 0.0f) || (wmax > 0.0 && wmax < 1e-20))
         return false;
     std::frexp(ymax, &top);
     if (top + e > 37 || e > 64 || e < -32)
         return false;
     for (int64_t i = 0; i < nx; ++i) {
         const float x = xs[i];
-        // a sum over small arguments would feel the sines' absolute error
+        // sines that are all small are left to sin() (kSineSmall)
         if (x != 0.0f && !(x > 0.0f && x < 1e6f && (double)x * ymax >= 0.02))
             return false;
     }
@@ -301,18 +311,71 @@ __global__ void __launch_bounds__(256) k_sine_fixed_prep(int kind, const float *
     }
 }
 
+// The phase of one term in 2^-64 of a turn.
+__device__ __forceinline__ unsigned long long sine_phase(const SinePoint &x, unsigned y0, unsigned y1)
+{
+    unsigned long long d = (unsigned long long)x.x0 * y0 >> 32;
+    d += (unsigned long long)x.x1 * y0;
+    d += (unsigned long long)x.x0 * y1;
+    return d + ((unsigned long long)(x.x2 * y0 + x.x1 * y1) << 32);
+}
+
+// A lane's float32 sums over its terms.
+struct SineSide {
+    float low = 0.0f;    // weights times the sines' last line
+    float small = 0.0f;  // |w| times the quarter turns from the sine's next zero
+    float all = 0.0f;    // |w|
+    __device__ __forceinline__ void add(const SineTable &t, unsigned long long d, float w)
+    {
+        const int k = (int)(d >> 52);
+        const float r = (float)(int)((unsigned)(d >> 20) ^ 0x80000000u) * 2.3283064365386963e-10f;  // 2^-32
+        const float2 a = *reinterpret_cast<const float2 *>(&t.arc[k].low);  // low, t3
+        const float c = __fmaf_rn(__fmul_rn(__fmaf_rn(t.t4[k], r, a.y), r), __fmul_rn(r, r), a.x);
+        low = __fmaf_rn(w, c, low);
+        const float q = fabsf((float)(int)((unsigned)(d >> 32) << 1)) * 4.656612873077393e-10f;  // 2^-31
+        small = __fmaf_rn(fabsf(w), q, small);
+        all = __fadd_rn(all, fabsf(w));
+    }
+};
+
+// sin(a) for 0 <= a <= 1/2 by its Taylor series (the next term is below 2^-65 a):
+// a third of sin()'s FP64 instructions.
+__device__ __forceinline__ double sine_series(double a)
+{
+    const double z = a * a;
+    double p = -1.0 / 1307674368000.0;
+    p = fma(p, z, 1.0 / 6227020800.0);
+    p = fma(p, z, -1.0 / 39916800.0);
+    p = fma(p, z, 1.0 / 362880.0);
+    p = fma(p, z, -1.0 / 5040.0);
+    p = fma(p, z, 1.0 / 120.0);
+    p = fma(p, z, -1.0 / 6.0);
+    return fma(a * z, p, a);
+}
+
+__device__ __forceinline__ double lane_sum(double v)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    return v;
+}
+
 // CTA b takes the output points b, b + gridDim.x, ...; a warp sums a quarter
 // of a point's terms, lane by lane in order, and the parts are added in a fixed
 // tree, so the result depends on nothing but the inputs.
 __global__ void __launch_bounds__(kSineThreads, 1) k_sine_fixed(const SineTable *__restrict__ table,
                                                                 const SinePoint *__restrict__ point, int nx,
                                                                 const SineTerm *__restrict__ term,
-                                                                const float *__restrict__ wf, int ny, double add,
-                                                                double mul, int div, double *__restrict__ out)
+                                                                const float *__restrict__ wf, int ny, double unit,
+                                                                double add, double mul, int div,
+                                                                double *__restrict__ out)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     SineTable &t = *reinterpret_cast<SineTable *>(smem);
     __shared__ double part[kSineBatch * kSineParts];
+    __shared__ float2 size[kSineBatch * kSineParts];  // sums of |w| t and |w|
+    __shared__ bool again[kSineBatch];
+    static_assert(kSineWarps % kSineParts == 0, "a warp keeps its part");
     {
         const uint4 *src = reinterpret_cast<const uint4 *>(table);
         uint4 *dst = reinterpret_cast<uint4 *>(smem);
@@ -323,33 +386,69 @@ __global__ void __launch_bounds__(kSineThreads, 1) k_sine_fixed(const SineTable 
     const int mine = (nx - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;  // output points of this CTA
     for (int o0 = 0; o0 < mine; o0 += kSineBatch) {
         const int batch = min(kSineBatch, mine - o0);
-        for (int item = warp; item < batch * kSineParts; item += kSineWarps) {
-            const SinePoint pt = point[blockIdx.x + (o0 + item / kSineParts) * gridDim.x];
-            double acc = 0.0;
-            float side = 0.0f;
+        const int items = batch * kSineParts, l0 = warp % kSineParts * 32 + lane;  // a warp's items are one part
+        auto point_of = [&](int item) { return point[blockIdx.x + (o0 + item / kSineParts) * gridDim.x]; };
+        SineSide next;
+        SinePoint ahead{};
+        if (warp < items) {
+            ahead = point_of(warp);
+            for (int l = l0; l < ny; l += 32 * kSineParts)
+                next.add(t, sine_phase(ahead, term[l].y0, term[l].y1), wf[l]);
+        }
+        for (int item = warp; item < items; item += kSineWarps) {
+            // this item's FP64 sum beside the float32 sums of the one after
+            const SinePoint pt = ahead;
+            const SineSide side = next;
+            next = SineSide();
+            if (item + kSineWarps < items)
+                ahead = point_of(item + kSineWarps);
+            double acc = (double)side.low;
 #pragma unroll 2
-            for (int l = item % kSineParts * 32 + lane; l < ny; l += 32 * kSineParts) {
+            for (int l = l0; l < ny; l += 32 * kSineParts) {
                 const SineTerm y = term[l];
-                const float w = wf[l];
-                unsigned long long d = (unsigned long long)pt.x0 * y.y0 >> 32;
-                d += (unsigned long long)pt.x1 * y.y0;
-                d += (unsigned long long)pt.x0 * y.y1;
-                d += (unsigned long long)(pt.x2 * y.y0 + pt.x1 * y.y1) << 32;
-                const int k = (int)(d >> 53);
-                const double r = __longlong_as_double((long long)(d >> 1 & 0xfffffffffffffull | 0x3ff0000000000000ull)) - 1.5;
-                const float rf = (float)(int)((unsigned)(d >> 21) ^ 0x80000000u) * 2.3283064365386963e-10f;  // 2^-32
-                const SineArc a = t.arc[k];
-                const float c = __fmaf_rn(__fmul_rn(__fmaf_rn(t.t4[k], rf, a.t3), rf), __fmul_rn(rf, rf), a.low);
+                const unsigned long long d = sine_phase(pt, y.y0, y.y1);
+                const double r = __longlong_as_double((long long)(d & 0xfffffffffffffull | 0x3ff0000000000000ull)) - 1.5;
+                const SineArc &a = t.arc[d >> 52];
                 acc = fma(y.w, fma(fma(a.t2, r, a.t1), r, a.t0), acc);
-                side = __fmaf_rn(w, c, side);
+                next.add(t, sine_phase(ahead, y.y0, y.y1), wf[l]);
             }
-            acc += (double)side;
+            acc = lane_sum(acc);
+            float small = side.small, all = side.all;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-            if (lane == 0)
+            for (int o = 16; o > 0; o >>= 1) {
+                small += __shfl_down_sync(0xffffffffu, small, o);
+                all += __shfl_down_sync(0xffffffffu, all, o);
+            }
+            if (lane == 0) {
                 part[item] = pt.zero ? 0.0 : acc;
+                size[item] = make_float2(pt.zero ? all : small, all);
+            }
         }
         __syncthreads();
+        bool low = false;
+        if ((int)threadIdx.x < batch) {
+            const float2 *z = size + threadIdx.x * kSineParts;
+            low = again[threadIdx.x] =
+                (z[0].x + z[1].x) + (z[2].x + z[3].x) < kSineSmall * ((z[0].y + z[1].y) + (z[2].y + z[3].y));
+        }
+        if (__syncthreads_or(low)) {
+            for (int item = warp; item < items; item += kSineWarps) {
+                if (!again[item / kSineParts])
+                    continue;
+                const double x = point_of(item).x * unit;
+                double acc = 0.0;
+                for (int l = l0; l < ny; l += 32 * kSineParts) {
+                    const SineTerm y = term[l];
+                    // the integer y in a double's last place at 2^52
+                    const double a = x * (__hiloint2double(0x43300000 | (int)y.y1, (int)y.y0) - 4503599627370496.0);
+                    acc = fma(y.w, a <= 0.5 ? sine_series(a) : sin(a), acc);
+                }
+                acc = lane_sum(acc);
+                if (lane == 0)
+                    part[item] = acc;
+            }
+            __syncthreads();
+        }
         if ((int)threadIdx.x < batch) {
             const double *p = part + threadIdx.x * kSineParts;
             const double s = (p[0] + p[1]) + (p[2] + p[3]);
@@ -362,20 +461,20 @@ __global__ void __launch_bounds__(kSineThreads, 1) k_sine_fixed(const SineTable 
 
 size_t sine_fixed_scratch(int64_t nx, int64_t ny)
 {
-    return sizeof(SineTable) + sizeof(SinePoint) * (size_t)nx + sizeof(SineTerm) * (size_t)ny + 4 * (size_t)ny + 64;
+    return sizeof(SinePoint) * (size_t)nx + sizeof(SineTerm) * (size_t)ny + 4 * (size_t)ny + 64;
 }
 
 size_t sine_table_bytes() { return sizeof(SineTable); }
 
-// The arcs' table at the start of `scratch` (once per allocation).
-int sine_table_upload(void *scratch, cudaStream_t st)
+// The arcs' table to `dst` (once per allocation).
+int sine_table_upload(void *dst, cudaStream_t st)
 {
     static const SineTable *table = [] {
         SineTable *t = new SineTable();
         sine_table(t);
         return t;
     }();
-    FRMC_CUDA(cudaMemcpyAsync(scratch, table, sizeof(SineTable), cudaMemcpyHostToDevice, st));
+    FRMC_CUDA(cudaMemcpyAsync(dst, table, sizeof(SineTable), cudaMemcpyHostToDevice, st));
     return FRMC_OK;
 }
 
@@ -393,7 +492,8 @@ int launch_sine_fixed(int sms, int kind, const float *xs, int nx, const float *y
     const double add = kind == SK_SQ_TO_GR ? 0.0 : 1.0;
     const double mul = kind == SK_GR_TO_SQ ? 4.0 * M_PI * rho : kind == SK_BIGGR_TO_SQ ? 1.0 : 2.0 / M_PI;
     k_sine_fixed<<<sms < nx ? sms : nx, kSineThreads, sizeof(SineTable), st>>>(
-        static_cast<const SineTable *>(table), point, nx, term, wf, ny, add, mul, kind != SK_SQ_TO_GR, out);
+        static_cast<const SineTable *>(table), point, nx, term, wf, ny, std::ldexp(1.0, -scale), add, mul,
+        kind != SK_SQ_TO_GR, out);
     FRMC_CUDA(cudaGetLastError());
     return FRMC_OK;
 }
