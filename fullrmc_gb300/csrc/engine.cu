@@ -154,6 +154,7 @@ struct EDesc {
     // Dense engines (scale factor != 1, a fitted scale factor or a window):
     // every step evaluates window * (s G') over all bins, G' = Gc + R S.
     int dense, wlen, fit_freq;
+    int list;     // split steps: changed bins go to tlist, and the commit through it (touch_list)
     double sf0, fit_min, fit_max;
     double *Gc;   // [hs] G of the current configuration (before scale factor and window)
     double *fnum; // [hs] fit numerator weights times the fit target
@@ -527,9 +528,10 @@ constexpr int kItemUnroll = 4;
 // time, the columns of a warp in order; the pair before and after the move is
 // binned, and a changed bin adds -1 / +1 to the engine's global oriented delta
 // and element-pair delta.  The additions return nothing, so no thread waits
-// for them: a touched list, which needs its place from a shared counter, cost a
-// warp a round trip to L2 for every moved atom and is kept only for engines
-// with an S(Q) term (LIST), whose kernel commits through it.
+// for them: a touched list, which needs its place from a shared counter, costs a
+// warp a round trip to L2 for every moved atom and is kept only (LIST) for engines
+// with an S(Q) term, whose kernel commits through it, and where it saves a pass
+// over many counts (touch_list).
 //
 // cols: kSplitCols ints of shared memory (the chunk's columns, -1 for moved
 // atoms).
@@ -1095,10 +1097,10 @@ __device__ void split_group_internal(const EDesc &Dg, const MovedGroup &g)
         const unsigned cnt = (f0 >= 0) + (f1 >= 0);
         if (!cnt)
             continue;
-        unsigned pos = Dg.sq ? atomicAdd(&Dg.st->tcount, cnt) : 0u;
+        unsigned pos = Dg.list ? atomicAdd(&Dg.st->tcount, cnt) : 0u;
         if (f0 >= 0) {
             atomicSub(Dg.delta + half + f0, 1);
-            if (Dg.sq)
+            if (Dg.list)
                 D.tlist[pos++] = half + f0;
             int p, bb;
             pair_of_flat(D, f0, ela, elj, b0, p, bb);
@@ -1107,7 +1109,7 @@ __device__ void split_group_internal(const EDesc &Dg, const MovedGroup &g)
         }
         if (f1 >= 0) {
             atomicAdd(Dg.delta + half + f1, 1);
-            if (Dg.sq)
+            if (Dg.list)
                 D.tlist[pos] = half + f1;
             int p, bb;
             pair_of_flat(D, f1, ela, elj, b1, p, bb);
@@ -1167,11 +1169,30 @@ __device__ void finish_engine(const EDesc &D, const MovedGroup &g, double *red, 
     const bool accept = *s_flag != 0;
     if (accept)
         commit_split_group(D, g);  // its loads go beside the counts'
-    // commit (or drop) the oriented delta: the whole array once, in order and
-    // with kCommitUnroll quads in flight per thread (a group move of 13 atoms
-    // touches 36,000 entries of its 27,000 bins; through a list each took a
-    // dependent load, an exchange and an addition)
-    {
+    // commit (or drop) the oriented delta.  Where a move touches much of the array
+    // (touch_list): the whole of it once, in order and with kCommitUnroll quads in
+    // flight per thread (a group move of 13 atoms touches 36,000 entries of its
+    // 27,000 bins; through a list each took a dependent load, an exchange and an
+    // addition).  Else through the touched list; duplicates are harmless:
+    // atomicExch hands each bin's delta to exactly one entry
+    if (D.list) {
+        const unsigned nt = __ldcg(&D.st->tcount);
+        for (unsigned k0 = threadIdx.x; k0 < nt; k0 += kCommitUnroll * blockDim.x) {
+            int f[kCommitUnroll], d[kCommitUnroll];
+#pragma unroll
+            for (int u = 0; u < kCommitUnroll; ++u) {
+                const unsigned k = k0 + u * blockDim.x;
+                f[u] = k < nt ? __ldcg(D.tlist + k) : -1;
+            }
+#pragma unroll
+            for (int u = 0; u < kCommitUnroll; ++u) d[u] = f[u] >= 0 ? atomicExch(D.delta + f[u], 0) : 0;
+            if (accept) {
+#pragma unroll
+                for (int u = 0; u < kCommitUnroll; ++u)
+                    if (d[u]) D.counts[f[u]] += d[u];
+            }
+        }
+    } else {
         const int quads = (int)((2 * D.total + 3) / 4);  // the array is padded and zero past its end
         int4 *dq = reinterpret_cast<int4 *>(D.delta);
         int4 *cq = reinterpret_cast<int4 *>(D.counts);
@@ -1988,7 +2009,7 @@ __global__ void __launch_bounds__(kMaxEngineThreads, 1) k_engine_step(StepParams
     case BM_LOWER: item_delta<BM_LOWER, L_>(D, v0, v1, s_group, cP, cB, cols); break;                \
     default: item_delta<BM_GENERAL, L_>(D, v0, v1, s_group, cP, cB, cols); break;                    \
     }
-        if (D.sq) {
+        if (D.list) {
             FRMC_ITEM(true)
         } else {
             FRMC_ITEM(false)
@@ -2871,6 +2892,13 @@ constexpr long long kSoloFusedCost = 16384;  // one-engine steps up to this cost
 // either way, of 30,000 at 12 A (1,310) 17.1 and 19.7 us
 constexpr long long kSoloFusedWork = 3900;
 
+// Lines of touch_list.  us a step with the list and with the pass, one atom of
+// 14,000 at r 20 A in 2 / 4 / 6 / 10 elements (16,000 / 64,000 / 144,000 / 400,000
+// counts, 3,350 pairs): 25.2 / 31.1 / 42.3 / 72.1 and 19.3 / 27.1 / 41.9 / 80.4; of
+// 5,000 at 15 A in 10 elements (300,000, 1,410) 51.9 and 59.2; 13 atoms of 52,000
+// at 15 A in 3 (27,000, 18,400) 52.5 and 30.3.
+constexpr double kStreamBins = 65536.0, kStreamPerPair = 25.0;
+
 struct EngineSet {
     std::vector<Slot> slots;
     int fused = 1;         // batched steps use one CTA per engine where it fits
@@ -2948,6 +2976,21 @@ static long long solo_work(const Slot &sl)
     const double in_range = accept_fraction(D.B.b, 1, D.minD, D.maxD) * (double)D.n * D.group;
     const double swept = (double)sl.cost / (D.nc > 0 ? 4.0 : 1.0);
     return (long long)(in_range + swept / 4.0);
+}
+
+// Whether an engine's split steps keep a touched list (EDesc::list): with an
+// S(Q) term, and where the oriented counts outnumber what a step changes by so
+// much that one CTA's pass over them all takes longer.  The pass costs 1 us for
+// 25,000 counts, the list 2.5 us and 1 us for 900 pairs in range.
+static int touch_list(const Slot &sl)
+{
+    const EDesc &D = sl.d;
+    double pairs = (double)D.n * D.group;
+    if (D.nc > 0)
+        pairs = sl.cost / 4.0;  // the estimated sweep
+    else if (D.bm != BM_IBC)
+        pairs *= accept_fraction(D.B.b, 1, D.minD, D.maxD);
+    return D.sq || 2.0 * (double)D.total > kStreamBins + kStreamPerPair * pairs;
 }
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -4049,6 +4092,7 @@ static int add_engine(EngineSet *s, const frmc_engine_spec &sp, int *out_id)
     sl.sq_table = sp.sq_table;
     sl.cost = (cg.nc > 0 ? 4 * (long long)std::ceil(cg.sweep) : (long long)sp.n) * spec_group(sp);
     sl.work = solo_work(sl);
+    sl.d.list = touch_list(sl);
     s->slots[id] = sl;
     s->live.push_back(id);
     std::sort(s->live.begin(), s->live.end());
@@ -4861,6 +4905,7 @@ int frmc_engines_regrid(void *handle, int32_t e)
     D.cthr2 = cg.cthr2;
     sl.cost = (cg.nc > 0 ? 4 * (long long)std::ceil(cg.sweep) : (long long)D.n) * D.group;
     sl.work = solo_work(sl);
+    D.list = touch_list(sl);
     // a staged next move holds the moved atom's old cell-order slot and cell
     k_bump_gen<<<1, 1, 0, s->stream>>>(D.st);
     FRMC_CUDA(cudaGetLastError());
