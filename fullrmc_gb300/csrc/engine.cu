@@ -2886,10 +2886,14 @@ static long long fused_dyn_bytes(long long dp_ints, int bins, int threads)
 
 constexpr long long kFusedMaxCost = 49152;  // engines of a higher step cost (Slot::cost) are split over several CTAs
 constexpr long long kSoloFusedCost = 16384;  // one-engine steps up to this cost use the fused item,
-// and up to this work (Slot::work): a step of 3,000 / 5,000 / 8,000 / 14,000 atoms
-// at r 20 A (work 3,750 / 4,600 / 5,350 / 6,850) takes 20.7 / 23.9 / 26.0 / 28.5 us
-// fused and 21.6 / 20.8 / 21.7 / 21.0 us split; of 5,000 atoms at 15 A (2,660) 17.7
-// either way, of 30,000 at 12 A (1,310) 17.1 and 19.7 us
+// and up to this work (Slot::work) or, with many element-pair bins, a quarter of
+// them and 1,625 (solo_fused): a one-CTA step keeps the pairs' deltas in shared
+// memory, a split one's last CTA reads them from L2.  us a step in 1 / 2 / 3 / 4 / 5
+// / 6 elements (2,001 bins a pair), split and fused: 3,000 atoms at r 20 A (work
+// 3,750) 16.9 / 19.8 / 23.6 / 27.5 / 34.6 / 41.2 and 17.6 / 19.4 / 20.1 / 20.7 / 23.2 /
+// 25.7, 5,000 (4,600) 17.0 / 19.5 / 23.3 / 27.3 / 35.1 / 43.0 and 21.5 / 22.8 / 23.2 /
+// 23.9 / 26.4 / 28.9, 14,000 (6,850) 17.4 / 19.3 / 23.3 / 27.4 / 34.9 / 42.4 and 26.2 /
+// 26.6 / 27.3 / 28.2 / 30.7 / 33.0.
 constexpr long long kSoloFusedWork = 3900;
 
 // Lines of touch_list.  us a step with the list and with the pass, one atom of
@@ -2991,6 +2995,13 @@ static int touch_list(const Slot &sl)
     else if (D.bm != BM_IBC)
         pairs *= accept_fraction(D.B.b, 1, D.minD, D.maxD);
     return D.sq || 2.0 * (double)D.total > kStreamBins + kStreamPerPair * pairs;
+}
+
+// Whether a one-engine step of an engine that one CTA can take is left to one.
+static bool solo_fused(const Slot &sl)
+{
+    const long long bins = (long long)sl.d.npairs * sl.d.hs;
+    return sl.cost <= kSoloFusedCost && (sl.d.sq || sl.work <= std::max(kSoloFusedWork, bins / 4 + 1625));
 }
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -4457,9 +4468,7 @@ int frmc_engines_step(void *handle, int32_t engine, int32_t steps, int use_graph
         if (engine < 0)
             return launch_batched(s, sx);
         const int fi = s->fused_item[engine];
-        const Slot &solo = s->slots[engine];
-        // one CTA beats tiles plus a finisher
-        if (fi >= 0 && solo.cost <= kSoloFusedCost && (solo.d.sq || solo.work <= kSoloFusedWork))
+        if (fi >= 0 && solo_fused(s->slots[engine]))
             // one engine alone: the largest CTA (its layout fits by the fused check)
             FRMC_TRY(launch_items(s, s->items + fi, 1, 0, sx,
                                   (int)fused_dyn_bytes(s->fused_dp_ints, s->fused_bins, kMaxEngineThreads), true,
