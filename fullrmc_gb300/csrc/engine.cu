@@ -2957,6 +2957,13 @@ struct EngineSet {
     int sq_engs_cap = 0;
     cudaStream_t stream = nullptr;
     std::map<std::pair<int, int>, cudaGraphExec_t> graphs;
+    // the end of the last steps launched on each caller's stream (drain)
+    struct Foreign {
+        cudaStream_t stream;
+        cudaEvent_t ev;
+    };
+    std::vector<Foreign> foreign;
+    size_t foreign_next = 0;       // the entry that another stream takes when there are kForeignStreams
     cudaGraphExec_t host_graph[2] = {nullptr, nullptr};  // step_host per slot: copy in, scatter,
     int host_graph_E[2] = {0, 0};                        // step, gather, copy out
     bool dirty = true;
@@ -3218,6 +3225,43 @@ static long long place_key(const EngineSet *s, int nfused)
            fused_dyn_bytes(s->fused_dp_ints, s->fused_bins, s->threads);
 }
 
+// Marks the end of steps launched on a caller's stream.  Steps that the caller
+// captures run when the caller's graph does, which only the caller knows.
+constexpr size_t kForeignStreams = 64;
+static int mark_foreign(EngineSet *s, cudaStream_t st)
+{
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    FRMC_CUDA(cudaStreamIsCapturing(st, &cap));
+    if (cap != cudaStreamCaptureStatusNone)
+        return FRMC_OK;
+    auto it = std::find_if(s->foreign.begin(), s->foreign.end(),
+                           [st](const EngineSet::Foreign &f) { return f.stream == st; });
+    if (it == s->foreign.end() && s->foreign.size() < kForeignStreams) {
+        EngineSet::Foreign f{st, nullptr};
+        FRMC_CUDA(cudaEventCreateWithFlags(&f.ev, cudaEventDisableTiming));
+        it = s->foreign.insert(it, f);
+    } else {
+        if (it == s->foreign.end())
+            it = s->foreign.begin() + s->foreign_next++ % kForeignStreams;
+        // the mark stands for what it stood for before, too (another stream's
+        // steps, or those of a destroyed stream whose handle came back)
+        FRMC_CUDA(cudaStreamWaitEvent(st, it->ev, 0));
+        it->stream = st;
+    }
+    FRMC_CUDA(cudaEventRecord(it->ev, st));
+    return FRMC_OK;
+}
+
+// Waits for every step launched so far, on the set's stream or a caller's:
+// step kernels read descriptors, work lists and grids, before their wait for the
+// kernel ahead and after it, that the callers of this are about to change.
+static int drain(EngineSet *s)
+{
+    FRMC_CUDA(cudaStreamSynchronize(s->stream));
+    for (const EngineSet::Foreign &f : s->foreign) FRMC_CUDA(cudaEventSynchronize(f.ev));
+    return FRMC_OK;
+}
+
 // Items of an engine's split step: `tile` pairs of a swept column and a moved
 // atom each, all columns without a grid and the estimated sweep with one, but
 // for moves of several atoms or few swept columns no more than about one per SM.
@@ -3235,6 +3279,7 @@ static int refresh(EngineSet *s)
 {
     if (!s->dirty)
         return FRMC_OK;
+    FRMC_TRY(drain(s));
     const int nslots = (int)s->slots.size();
     std::vector<int2> items;
     s->item_first.assign(nslots, -1);
@@ -3344,7 +3389,6 @@ static int refresh(EngineSet *s)
         s->sq_xcol[id] = t.ncols;
         t.ncols += sl.d.npairs;
     }
-    FRMC_CUDA(cudaStreamSynchronize(s->stream));
     for (auto &t : s->tables) {
         if (t.ncols <= t.cap)
             continue;
@@ -3520,7 +3564,6 @@ static int refresh(EngineSet *s)
                              cudaMemcpyHostToDevice));
     std::vector<EDesc> hd(nslots);
     for (int k = 0; k < nslots; ++k) hd[k] = s->slots[k].d;
-    FRMC_CUDA(cudaStreamSynchronize(s->stream));
     if (nslots)
         FRMC_CUDA(cudaMemcpy(s->ddesc, hd.data(), sizeof(EDesc) * nslots, cudaMemcpyHostToDevice));
     if (!fused_ids.empty()) {
@@ -3549,7 +3592,7 @@ static int refresh(EngineSet *s)
 
 // Successive step kernels are launched with launch_after: what they read before
 // they wait (descriptors, work lists, the element-pair tables) is written by the
-// host alone, with the stream drained.  A chain of steps is bound by the gap
+// host alone, with every stream that steps were launched on drained.  A chain of steps is bound by the gap
 // between its launches as much as by the sweep: us a step without and with it,
 // one engine of 5,000 atoms 17.8 and 16.0, of 100,000 23.9 and 23.1, 24 engines
 // with an S(Q) term (two kernels a step) 52.9 and 48.5, 256 engines 25.3 and 24.3.
@@ -4115,7 +4158,8 @@ static int add_engine(EngineSet *s, const frmc_engine_spec &sp, int *out_id)
 static void free_set(EngineSet *s)
 {
     if (s->stream)
-        cudaStreamSynchronize(s->stream);
+        drain(s);
+    for (const EngineSet::Foreign &f : s->foreign) cudaEventDestroy(f.ev);
     drop_graphs(s);
     for (auto &sl : s->slots)
         if (sl.blob) cudaFree(sl.blob);
@@ -4269,7 +4313,7 @@ int frmc_engines_set_tune(void *handle, int tile, int threads, int ctas_per_sm)
         ctas_per_sm > 32)
         return set_error(FRMC_E_ARG, "engines_set_tune: threads must be a multiple of 32 in [32, %d]",
                          kMaxEngineThreads);
-    FRMC_CUDA(cudaStreamSynchronize(s->stream));
+    FRMC_TRY(drain(s));
     s->tile = tile;
     s->threads = threads;
     s->ctas_per_sm = ctas_per_sm;
@@ -4328,7 +4372,7 @@ int frmc_engines_set_mode(void *handle, int fused)
     EngineSet *s = as_set(handle);
     if (!s)
         return set_error(FRMC_E_ARG, "null handle");
-    FRMC_CUDA(cudaStreamSynchronize(s->stream));
+    FRMC_TRY(drain(s));
     s->fused = fused ? 1 : 0;
     s->dirty = true;
     return refresh(s);
@@ -4480,7 +4524,7 @@ int frmc_engines_step(void *handle, int32_t engine, int32_t steps, int use_graph
     };
     if (!use_graph) {
         for (int k = 0; k < steps; ++k) FRMC_TRY(one(st));
-        return FRMC_OK;
+        return st == s->stream ? FRMC_OK : mark_foreign(s, st);
     }
     auto key = std::make_pair(engine, steps);
     auto it = s->graphs.find(key);
@@ -4507,7 +4551,7 @@ int frmc_engines_step(void *handle, int32_t engine, int32_t steps, int use_graph
         it = s->graphs.emplace(key, ex).first;
     }
     FRMC_CUDA(cudaGraphLaunch(it->second, st));
-    return FRMC_OK;
+    return st == s->stream ? FRMC_OK : mark_foreign(s, st);
 }
 
 // One batched step from host arrays into staging slot `slot` (0 or 1): the
@@ -4540,7 +4584,7 @@ static int step_host_submit(EngineSet *s, const int32_t *atoms, const float *vec
     if (E > s->stage_cap) {
         if (other_busy)
             return set_error(FRMC_E_STATE, "step_host: the staging must grow while a step is in flight");
-        FRMC_CUDA(cudaStreamSynchronize(s->stream));
+        FRMC_TRY(drain(s));
         drop_graphs(s);  // the captured copies name the staging buffers
         const int cap = std::max(E, 2 * s->stage_cap);
         for (int k = 0; k < 2; ++k) {
@@ -4872,7 +4916,7 @@ int frmc_engines_regrid(void *handle, int32_t e)
     EDesc &D = sl.d;
     if (!s->cells)
         return FRMC_OK;
-    FRMC_CUDA(cudaStreamSynchronize(s->stream));
+    FRMC_TRY(drain(s));
     std::vector<float4> b(D.n);
     std::vector<int> mol(D.n), el(D.n);
     std::vector<float> box(3 * (size_t)D.n);
