@@ -407,19 +407,22 @@ static int distances_common(int diff, int32_t atomIndex, const int32_t *indexes,
     // small output (a call whose output is one of its inputs needs the copies).
     const char *o = (const char *)out, *oe = o + out_elems * 4;
     auto apart = [&](const void *p, int64_t bytes) { return (const char *)p + bytes <= o || oe <= (const char *)p; };
-    if (c->pageable && apart(coords, n * 12) && (by_value || (idx ? apart(idx, K * 4) : apart(points, 3 * ps * 4)))) {
+    // A single row is written from its own atom on.
+    const int64_t first = fromIndex && single_index ? (int64_t)atomIndex * width : 0;
+    if (c->pageable && apart(coords, n * 12) &&
+        (by_value || (idx ? apart(idx, K * 4) : apart(points, 3 * ps * 4)))) {
         if (out_elems * 4 <= kDirectBytes) {
             touch_pages(out, out_elems * 4);
         } else {
             TRY(c->buf[BUF_OUT].ensure(out_elems * 4 + 16));
             dout = c->buf[BUF_OUT].as<float>();
-            if (fromIndex)
+            if (fromIndex && !single_index)
                 TRY(h2d(dout, out, out_elems * 4, c->stream));
         }
         TRY(launch_distances(diff, coords, (int)n, by_value ? nullptr : points, ps, by_value ? nullptr : idx,
                              by_value ? &few : nullptr, (int)K, fromIndex, isPBC, B, dout, c->stream));
         if (dout != out)
-            TRY(d2h(out, dout, out_elems * 4, c->stream));
+            TRY(d2h(out + first, dout + first, (out_elems - first) * 4, c->stream));
         return finish(c);
     }
     TRY(upload_atoms(c, coords, nullptr, nullptr, n));
@@ -442,12 +445,7 @@ static int distances_common(int diff, int32_t atomIndex, const int32_t *indexes,
         TRY(h2d(dout, out, out_elems * 4, c->stream));
     TRY(launch_distances(diff, c->buf[BUF_COORDS].as<float>(), (int)n, dpts, ps, didx, by_value ? &few : nullptr,
                          (int)K, fromIndex, isPBC, B, dout, c->stream));
-    if (fromIndex && single_index) {
-        const int64_t off = (int64_t)atomIndex * width;
-        TRY(d2h(out + off, dout + off, (out_elems - off) * 4, c->stream));
-    } else {
-        TRY(d2h(out, dout, out_elems * 4, c->stream));
-    }
+    TRY(d2h(out + first, dout + first, (out_elems - first) * 4, c->stream));
     return finish(c);
 }
 
