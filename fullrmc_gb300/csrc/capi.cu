@@ -130,6 +130,12 @@ static int finish(Context *c)
 // included: pages in use 43 us written by the kernel, 51 copied; mapped and
 // unmapped by each call 1,170 and 360).
 constexpr int64_t kDirectBytes = 131072;
+// Points that do not go by value are copied, and the atoms with them, next to an
+// output that is copied, where the atoms take at most this many bytes: the
+// kernel's trips over the host link, indexes and then the points' atoms, take
+// longer (differences of 100 and 500 atoms to 200 points: read 37 and 38.5 us a
+// call, copied 30.5 and 32; distances of 3,000 atoms to 65: 40 and 43).
+constexpr int64_t kCopiedBytes = 16384;
 
 // Ahead of a kernel's writes to a caller's array: makes its pages present and
 // writable by a write of the CPU that leaves each page's bytes as they are.
@@ -409,7 +415,7 @@ static int distances_common(int diff, int32_t atomIndex, const int32_t *indexes,
     auto apart = [&](const void *p, int64_t bytes) { return (const char *)p + bytes <= o || oe <= (const char *)p; };
     // A single row is written from its own atom on.
     const int64_t first = fromIndex && single_index ? (int64_t)atomIndex * width : 0;
-    if (c->pageable && apart(coords, n * 12) &&
+    if (c->pageable && (out_elems * 4 <= kDirectBytes || by_value || n * 12 > kCopiedBytes) && apart(coords, n * 12) &&
         (by_value || (idx ? apart(idx, K * 4) : apart(points, 3 * ps * 4)))) {
         if (out_elems * 4 <= kDirectBytes) {
             touch_pages(out, out_elems * 4);

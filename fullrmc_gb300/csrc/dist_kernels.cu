@@ -20,10 +20,13 @@ struct PointSrc {
 };
 
 constexpr int kDistAtoms = 256;  // threads of a block, and its largest tile of atoms
-// Outputs that a block forms: 16 a thread, so that calls of few atoms and many
-// points still fill the SMs (differences of 5,000 atoms to 70 points: tiles of
-// 256 atoms, 40 blocks, 75.7 us a call, of 21 atoms 60.4).
+// Outputs that a block forms at most: 16 a thread, and fewer where that leaves
+// less than two blocks an SM (differences of 5,000 atoms to 70 points: tiles of
+// 256 atoms, 40 blocks, 75.7 us a call, of 21 atoms 60.4; 13 distances of 3,000
+// atoms: 12 blocks 37, 188 blocks 28).
 constexpr int kDistOutputs = 4096;
+constexpr int kDistBlocks = 304;
+constexpr int kDistLeast = 4;  // atoms of a tile
 
 // W = 1: out[i, k] = |bc(point k - coords[i])|; W = 3: out[i, c, k] = component c
 // of the difference.
@@ -33,16 +36,16 @@ constexpr int kDistOutputs = 4096;
 // lines: a block stages its atoms' coordinates and up to kInlinePoints points in
 // shared memory and writes the block's outputs in the order they are stored.  A
 // difference is formed once per component for that.  13 rows of 52,000 atoms,
-// whole call: one thread per (atom, row) between copies 65.5 us, so 36.
+// whole call: one thread per (atom, row) between copies 65.5 us, so 50.
 template <int BM, int W>
 __global__ void __launch_bounds__(kDistAtoms) k_distances(const float *__restrict__ coords, int n,
-                                                          const __grid_constant__ PointSrc src, int tile, int K,
+                                                          const __grid_constant__ PointSrc src, int tile, int points, int K,
                                                           int fromIndex, Basis B, float *__restrict__ out)
 {
     __shared__ float sc[3 * kDistAtoms], sx[kInlinePoints], sy[kInlinePoints], sz[kInlinePoints];
     __shared__ int sa[kInlinePoints];
-    const int i0 = blockIdx.x * tile, k0 = blockIdx.y * kInlinePoints;
-    const int na = min(tile, n - i0), kt = min(kInlinePoints, K - k0);
+    const int i0 = blockIdx.x * tile, k0 = blockIdx.y * points;
+    const int na = min(tile, n - i0), kt = min(points, K - k0);
     for (int e = threadIdx.x; e < 3 * na; e += kDistAtoms) sc[e] = coords[3 * (long long)i0 + e];
     if ((int)threadIdx.x < kt) {
         const int t = threadIdx.x, k = k0 + t;
@@ -132,21 +135,24 @@ int launch_distances(int diff, const float *coords, int n, const float *pts, lon
         return set_error(FRMC_E_ARG, "too many points (%d)", K);
     PointSrc src{pts, ps, idx, few ? *few : InlinePoints()};
     Basis B = make_basis(basis);
-    const int tile = std::max(16, std::min(kDistAtoms, kDistOutputs / ((diff ? 3 : 1) * std::min(K, kInlinePoints))));
-    dim3 grid((n + tile - 1) / tile, (K + kInlinePoints - 1) / kInlinePoints);
+    // as many points for each block of a row of blocks (65: 33 and 32)
+    const int turns = (K + kInlinePoints - 1) / kInlinePoints, points = (K + turns - 1) / turns;
+    int tile = std::min(kDistAtoms, kDistOutputs / ((diff ? 3 : 1) * points));
+    tile = std::max(kDistLeast, std::min(tile, (n + kDistBlocks - 1) / kDistBlocks * turns));
+    dim3 grid((n + tile - 1) / tile, turns);
     if (diff) {
         // one form for every basis: no term that is zero may be left out
         auto kern = isPBC ? k_distances<BM_GENERAL, 3> : k_distances<BM_IBC, 3>;
-        kern<<<grid, kDistAtoms, 0, st>>>(coords, n, src, tile, K, fromIndex, B, out);
+        kern<<<grid, kDistAtoms, 0, st>>>(coords, n, src, tile, points, K, fromIndex, B, out);
         FRMC_CUDA(cudaGetLastError());
         return FRMC_OK;
     }
     switch (basis_mode(basis, isPBC)) {
-    case BM_IBC: k_distances<BM_IBC, 1><<<grid, kDistAtoms, 0, st>>>(coords, n, src, tile, K, fromIndex, B, out); break;
-    case BM_DIAG: k_distances<BM_DIAG, 1><<<grid, kDistAtoms, 0, st>>>(coords, n, src, tile, K, fromIndex, B, out); break;
-    case BM_XYTRI: k_distances<BM_XYTRI, 1><<<grid, kDistAtoms, 0, st>>>(coords, n, src, tile, K, fromIndex, B, out); break;
-    case BM_LOWER: k_distances<BM_LOWER, 1><<<grid, kDistAtoms, 0, st>>>(coords, n, src, tile, K, fromIndex, B, out); break;
-    default: k_distances<BM_GENERAL, 1><<<grid, kDistAtoms, 0, st>>>(coords, n, src, tile, K, fromIndex, B, out); break;
+    case BM_IBC: k_distances<BM_IBC, 1><<<grid, kDistAtoms, 0, st>>>(coords, n, src, tile, points, K, fromIndex, B, out); break;
+    case BM_DIAG: k_distances<BM_DIAG, 1><<<grid, kDistAtoms, 0, st>>>(coords, n, src, tile, points, K, fromIndex, B, out); break;
+    case BM_XYTRI: k_distances<BM_XYTRI, 1><<<grid, kDistAtoms, 0, st>>>(coords, n, src, tile, points, K, fromIndex, B, out); break;
+    case BM_LOWER: k_distances<BM_LOWER, 1><<<grid, kDistAtoms, 0, st>>>(coords, n, src, tile, points, K, fromIndex, B, out); break;
+    default: k_distances<BM_GENERAL, 1><<<grid, kDistAtoms, 0, st>>>(coords, n, src, tile, points, K, fromIndex, B, out); break;
     }
     FRMC_CUDA(cudaGetLastError());
     return FRMC_OK;
