@@ -4557,11 +4557,13 @@ int frmc_engines_step(void *handle, int32_t engine, int32_t steps, int use_graph
 // One batched step from host arrays into staging slot `slot` (0 or 1): the
 // moves are written to the slot's pinned buffer; the slot's event marks the
 // step's completion.  Where every engine steps in one CTA the step is one launch
-// that reads the moves from that buffer and writes the results to the other:
-// launched by itself it overlaps the end of the step before, which a graph of it
-// cannot (256 engines, two slots in flight: 26.8 us a step, from graphs 30.3).
-// Else one CUDA graph copies the moves in, scatters them into the rings, steps,
-// gathers the results and copies them back.
+// that reads the moves from that buffer and writes the results to the other.
+// Behind a step in flight it is launched by itself, so that it overlaps that
+// step's end, which a graph of it cannot (256 engines, two slots in flight: 25.7
+// us a step, from graphs 29.5); alone from its graph, which the host launches
+// sooner (one engine of 60 to 1,000 atoms, a step that is waited for: 26.7 us, by
+// itself 29.5).  Else one CUDA graph copies the moves in, scatters them into the
+// rings, steps, gathers the results and copies them back.
 static int step_host_submit(EngineSet *s, const int32_t *atoms, const float *vecs, const float *u, int slot)
 {
     if (slot < 0 || slot > 1)
@@ -4619,18 +4621,24 @@ static int step_host_submit(EngineSet *s, const int32_t *atoms, const float *vec
     cudaStream_t st = s->stream;
     // every live engine fused and none with an S(Q) term: one kernel reads
     // the moves from the mapped staging buffer and writes the results there
-    if (s->nfused == s->nbatch && s->sq_host.empty() && s->nfused == E) {
+    const bool direct = s->nfused == s->nbatch && s->sq_host.empty() && s->nfused == E;
+    auto step = [&](cudaStream_t sx) -> int {
         EMove *dm = nullptr;
         EResult *dr = nullptr;
         FRMC_CUDA(cudaHostGetDevicePointer((void **)&dm, s->hstage_m[slot], 0));
         FRMC_CUDA(cudaHostGetDevicePointer((void **)&dr, s->hstage_r[slot], 0));
-        FRMC_TRY(launch_items(s, s->items + s->nsolo, s->nfused, 0, st, fused_dyn_smem(s), true, dm, dr));
+        return launch_items(s, s->items + s->nsolo, s->nfused, 0, sx, fused_dyn_smem(s), true, dm, dr);
+    };
+    if (direct && other_busy) {
+        FRMC_TRY(step(st));
         FRMC_CUDA(cudaEventRecord(s->stage_ev[slot], st));
         s->stage_busy[slot] = true;
         s->stage_E[slot] = E;
         return FRMC_OK;
     }
     auto body = [&](cudaStream_t sx) -> int {
+        if (direct)
+            return step(sx);
         FRMC_CUDA(cudaMemcpyAsync(s->dstage_m[slot], hm, sizeof(EMove) * E, cudaMemcpyHostToDevice, sx));
         k_scatter_moves<<<(E + 127) / 128, 128, 0, sx>>>(s->ddesc, s->dlive, s->dstage_m[slot], E);
         FRMC_CUDA(cudaGetLastError());
