@@ -2937,6 +2937,7 @@ struct EngineSet {
     cudaEvent_t stage_ev[2] = {nullptr, nullptr};
     bool stage_busy[2] = {false, false};
     int stage_E[2] = {0, 0};       // engines of the step each busy slot holds
+    bool step_alone = false;       // the last host step was submitted with none in flight
     int stage_cap = 0;
     Sched *sched = nullptr;        // [0]: histogram step kernels, [1]: S(Q) kernel
     std::vector<SqTable> tables;
@@ -4560,9 +4561,9 @@ int frmc_engines_step(void *handle, int32_t engine, int32_t steps, int use_graph
 // that reads the moves from that buffer and writes the results to the other.
 // Behind a step in flight it is launched by itself, so that it overlaps that
 // step's end, which a graph of it cannot (256 engines, two slots in flight: 25.7
-// us a step, from graphs 29.5); alone from its graph, which the host launches
-// sooner (one engine of 60 to 1,000 atoms, a step that is waited for: 26.7 us, by
-// itself 29.5).  Else one CUDA graph copies the moves in, scatters them into the
+// us a step, from graphs 29.5); with none ahead, from the second such step on,
+// from its graph, which the host launches sooner (one engine of 60 to 1,000 atoms,
+// each step waited for: 26.7 us, by itself 29.5).  Else one CUDA graph copies the moves in, scatters them into the
 // rings, steps, gathers the results and copies them back.
 static int step_host_submit(EngineSet *s, const int32_t *atoms, const float *vecs, const float *u, int slot)
 {
@@ -4629,7 +4630,9 @@ static int step_host_submit(EngineSet *s, const int32_t *atoms, const float *vec
         FRMC_CUDA(cudaHostGetDevicePointer((void **)&dr, s->hstage_r[slot], 0));
         return launch_items(s, s->items + s->nsolo, s->nfused, 0, sx, fused_dyn_smem(s), true, dm, dr);
     };
-    if (direct && other_busy) {
+    const bool alone = s->step_alone && !other_busy;
+    s->step_alone = !other_busy;
+    if (direct && !alone) {
         FRMC_TRY(step(st));
         FRMC_CUDA(cudaEventRecord(s->stage_ev[slot], st));
         s->stage_busy[slot] = true;
