@@ -185,9 +185,10 @@ int frmc_engines_push_group_moves(void *handle, int32_t e, const int32_t *atoms,
  * captures the launches in a CUDA graph (cached per engine/steps).  Returns
  * without synchronising; stream NULL = the set's own stream.  Calls that
  * change the set (tuning, mode, regrid, and the first step after engines were
- * added or removed) wait for the steps launched on every stream.  Steps that
- * the caller captures name the set's present work lists: the caller waits for
- * its graph before such a call and captures again after it. */
+ * added or removed) wait for the steps launched before them: for the set's
+ * stream, and once steps went to a caller's stream for the device (so not
+ * while one of its streams is being captured).  Steps that the caller captures
+ * name the set's present work lists: capture again after such a call. */
 int frmc_engines_step(void *handle, int32_t engine, int32_t steps, int use_graph, void *stream);
 /* Measured placement of the batched one-CTA launch (no counterpart in
  * fullrmc).  Runs `steps` batched steps (they advance every chain like

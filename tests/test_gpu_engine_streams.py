@@ -63,7 +63,7 @@ def test_change_while_steps_run(change, graph):
         want = got
 
 
-def test_more_streams_than_marks():
+def test_many_streams():
     """70 streams, each with a few steps, one after the other."""
     import torch
     from fullrmc_gb300.engine import EngineSet, translation_moves
