@@ -124,7 +124,8 @@ static int finish(Context *c)
 }
 
 // Outputs of at most this many bytes are written to the caller's array by the
-// kernel, larger ones copied.  Up to 128 KiB malloc serves an array from its
+// kernel, larger ones copied (but for the moved atoms' histograms, which are
+// written in place at any size).  Up to 128 KiB malloc serves an array from its
 // heap, whose pages stay; a larger one may be mapped for itself, and to unmap a
 // page that a kernel has written costs 20 us (2.7 MB of distances, array
 // included: pages in use 43 us written by the kernel, 51 copied; mapped and

@@ -44,7 +44,7 @@
 // k_full_tiles, measured slower here (1.10 against 0.90 ms per call: the lanes
 // of a block have unequal numbers of neighbours).  Measured (whole host calls):
 // 100,000 atoms, 103 A box with gamma = 120, r 0-20 A: 6.92 -> 0.63 ms, the
-// kernel 6.81 -> 0.55 ms for 5.2e5 of 4.9e6 block pairs, 34 issue slots per
+// kernel 6.81 -> 0.55 ms for 5.2e5 of 4.9e6 block pairs, 31 issue slots per
 // column of 32 rows; 11,303 atoms, r 0-12 A: 335 -> 84 us; a 100,000-atom
 // particle with every pair counted (shape function): 12.5 -> 4.1 ms, 24 issue
 // slots per column (5.3 ms and 32 with each pair tested).
@@ -182,7 +182,9 @@ struct CellGeom {
 };
 
 // Columns (x, y) about as wide as the cube that holds one block at the mean
-// density, cut into cells of an eighth of it along z.
+// density, cut into cells of an eighth of it along z.  A free system without
+// extent on an axis has no density: one cell, in no order (a sheet of 11,000 atoms,
+// all pairs within 20 A: 115 us, and 295 with every pair evaluated).
 __device__ CellGeom cell_geom(const CellSort &p)
 {
     CellGeom g;

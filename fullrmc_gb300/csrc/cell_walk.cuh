@@ -1,7 +1,8 @@
-// The walk over pairs of spatially sorted atoms within a reach: a warp holds
-// one atom of a row block per lane, tests 32 column blocks at once and hands
-// the squared distances of the surviving ones to the caller four columns at a
-// time.  cell_pairs.cu sorts the atoms and says what makes the test exact.
+// The walk over pairs of spatially sorted atoms within a reach: a warp takes runs
+// of a list of block pairs (k_cell_list tests and lists them), holds one atom of
+// the row block per lane and hands the squared distances of the column block's
+// atoms to the caller four columns at a time.  cell_pairs.cu sorts the atoms and
+// says what makes the test exact.
 #pragma once
 #include <cstdint>
 #include <type_traits>

@@ -536,7 +536,7 @@ constexpr int kItemUnroll = 4;
 // cols: kSplitCols ints of shared memory (the chunk's columns, -1 for moved
 // atoms).
 constexpr int kSplitCols = 1024;
-constexpr int kSplitTiles = 144;  // items of a split step whose columns are few
+constexpr int kSplitTiles = 144;  // items of a split step whose columns are few (152 SMs; 72, 100, 220, 300: no faster)
 
 __device__ __forceinline__ int cell_column(const int *P, const int *Bse, int nc, int v);
 
@@ -3566,8 +3566,9 @@ static int refresh(EngineSet *s)
 // they wait (descriptors, work lists, the element-pair tables) is written by the
 // host alone, with every stream that steps were launched on drained.  A chain of steps is bound by the gap
 // between its launches as much as by the sweep: us a step without and with it,
-// one engine of 5,000 atoms 17.8 and 16.0, of 100,000 23.9 and 23.1, 24 engines
-// with an S(Q) term (two kernels a step) 52.9 and 48.5, 256 engines 25.3 and 24.3.
+// one engine of 5,000 atoms 17.8 and 16.0, of 100,000 23.9 and 23.1, 256 engines
+// 25.3 and 24.3 (24 engines with an S(Q) term, two kernels a step, 52.8 and 50.7 to
+// 52.2: within what runs differ by).
 static int launch_items(EngineSet *s, const int2 *items, int count, int eval_only, cudaStream_t st,
                         int dyn_smem = 0, bool fused = false, const EMove *hmoves = nullptr,
                         EResult *hres = nullptr, int threads = 0)

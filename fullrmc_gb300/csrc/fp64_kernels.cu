@@ -137,13 +137,16 @@ __global__ void k_sine_prep(int kind, const float *__restrict__ xs, int nx, cons
 // The last line's sum over a lane's terms is formed first and the FP64 sum starts
 // from it, so that it costs no rounding of its own: added at the end it made the
 // error 3 to 9 % larger.  (The integer and float32 pipes have the room to form the
-// phases twice; all this, the second half of the table and the check below take
-// 2 to 3 us of a call, 91.0 -> 93.5 us at 5.9e6 terms, 38.5 -> 40.5 at 3.5e5.)  What is left is an absolute error of a sine, where sin() has a
-// relative one, so an output whose sines are small throughout -- sum |w| t below
-// 1/32 sum |w|, with t = 2 / pi asin |sin| -- is summed again with sin(), or
-// where an argument is small its series.
+// phases twice; this, the larger table and the check below take 2 to 3 us of a
+// call, 91.0 -> 93.5 us at 5.9e6 terms, 38.5 -> 40.5 at 3.5e5.)  What is left is an
+// absolute error of a sine, where sin() has a relative one, so an output whose
+// sines are small throughout -- sum |w| t below 1/32 sum |w|, with t = 2 / pi asin
+// |sin| -- is summed again with sin(), or where an argument is small its series.
 constexpr int kArcs = 4096;
-constexpr float kSineSmall = 1.0f / 32;  // rms error over sin()'s: above it 0.91 to 1.06, at 1/64 1.2, at 1/150 1.6
+// Rms error of an output over that of correctly rounded sines: 0.91 to 1.06 from
+// t = 1/24 on, 0.97 to 1.24 at 1/32, 1.15 to 1.5 at 1/64 (sin() itself rounds
+// a little worse: against k_sine_rows 0.91 over the 20 smallest arguments).
+constexpr float kSineSmall = 1.0f / 32;
 constexpr int kSineThreads = 384;  // 512 and 768: 0.5 and 2 us more a call of 5.9e6 terms
 constexpr int kSineWarps = kSineThreads / 32;
 constexpr int kSineParts = 4;    // parts of an output point's sum, a warp each
